@@ -31,6 +31,15 @@ struct BpLaunch {
 void launch_bp_layered(const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape,
                        cudaStream_t st);
 void launch_bp_flooding(const FloodView& cv, const BpParams& p, const BpIO& io, cudaStream_t st);
+// Register-resident messages (bp_reg.cuh).  reg_plan sets cv.reg_* for a code with layers of
+// `narrowest` to `widest` rows: `group` lanes per codeword if positive, else the smallest power of
+// two covering the widest layer, up to 128; reg_group stays 0 when the code fits no compiled
+// shape.  The flooding launcher takes plain codes only.  The layered one expects
+// io.work_counter reset.
+void reg_plan(LayeredView& cv, int widest, int narrowest, int group);
+void launch_bp_layered_reg(const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape,
+                           bool track_best, cudaStream_t st);
+void launch_bp_flooding_reg(const LayeredView& cv, const BpParams& p, const BpIO& io, cudaStream_t st);
 size_t layered_smem_bytes(const LayeredView& cv, int slots, bool track_best, int* slot_floats_out);
 int layered_default_slots(const LayeredView& cv, bool track_best);
 size_t flooding_smem_bytes(const FloodView& cv, int warps, int* slot_floats_out);

@@ -208,7 +208,20 @@ DeviceCode::DeviceCode(int n, int m, const int* row_ptr, const int* col_ind, int
         if (!systematic_parity(n, m, row_ptr, col_ind, parity_, parity_words_, kk))
             throw InvalidArgument("OSD needs a full-rank code with the information bits first (systematic-front)");
     }
-    if (layered()) build_layered(); else build_flood();
+    if (layered()) {
+        build_layered();
+    } else {
+        build_flood();
+        // flat row layers for the register-resident flooding kernel, where the code's rows fit it
+        std::vector<int> sizes;
+        consecutive_layers(n, m, row_ptr_.data(), col_ind_.data(), sizes);
+        LayeredView probe{};
+        probe.n = n;
+        probe.maxdeg = fv_.maxdeg;
+        probe.num_layers = static_cast<int>(sizes.size());
+        reg_plan(probe, *std::max_element(sizes.begin(), sizes.end()), *std::min_element(sizes.begin(), sizes.end()), 0);
+        if (probe.reg_plain) build_layered();
+    }
     if (need_osd) set_osd(osd);
 }
 
@@ -259,6 +272,7 @@ void DeviceCode::build_layered()
     for (int l = 0; l < L; ++l) starts[l + 1] = starts[l] + sizes[l];
     lv_.m = m_;
     lv_.layer_start = device_upload(starts, owned_);
+    reg_plan(lv_, maxw, *std::min_element(sizes.begin(), sizes.end()), layered_group_ > 0 ? group : 0);
 }
 
 void DeviceCode::build_flood()

@@ -179,6 +179,7 @@ void run_bp_osd(const DeviceCode& code, const BpParams& bp, const BpLaunch& shap
     }
     if (rec) check_cuda(cudaEventRecord(rec->ev[0], st), "cudaEventRecord");
     if (code.layered()) launch_bp_layered(code.layered_view(), p, io, shape, st);
+    else if (code.layered_view().reg_plain) launch_bp_flooding_reg(code.layered_view(), p, io, st);
     else launch_bp_flooding(code.flood_view(), p, io, st);
     if (rec) check_cuda(cudaEventRecord(rec->ev[1], st), "cudaEventRecord");
     if (with_osd) {
@@ -827,6 +828,7 @@ int decode_with_caller_scratch(unsigned long long handle, const float* d_llr, in
         io.osd_count = counters;
     }
     if (d->code->layered()) launch_bp_layered(d->code->layered_view(), p, io, d->shape, st);
+    else if (d->code->layered_view().reg_plain) launch_bp_flooding_reg(d->code->layered_view(), p, io, st);
     else launch_bp_flooding(d->code->flood_view(), p, io, st);
     if (d->osd_enabled) {
         OsdIO oio{};

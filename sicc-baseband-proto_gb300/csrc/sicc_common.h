@@ -57,6 +57,9 @@ struct LayeredView {
     const int* vars;    // [num_layers][maxdeg][width]
     int m;              // rows of the code
     const int* layer_start;  // [num_layers + 1] first row of each layer in layer order (rows packed)
+    int reg_group;      // lanes per codeword of the register-resident kernels (<= 128), 0: not for this code
+    int reg_rpl;        // their rows per lane in a layer
+    int reg_plain;      // 1: every layer has exactly reg_group rows
 };
 
 // Flooding schedule: rows in CSR order plus the column view used for the
