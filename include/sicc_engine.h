@@ -51,7 +51,8 @@ SICC_API int sicc_engine_create(const sicc_engine_config_t* config, unsigned lon
 SICC_API int sicc_engine_destroy(unsigned long long handle);
 /* Registers a code; returns its id (0, 1, ...) used in the batch's code_ids. */
 SICC_API int sicc_engine_add_code(unsigned long long handle, const sicc_engine_code_t* code, int* out_code_id);
-/* Launch shape of the persistent BP kernel: warps per CTA (0 = default) and CTAs (0 = fill the GPU). */
+/* Launch shape of the persistent BP kernel: CTAs (0 = fill the GPU); warps_per_cta (0..8) is checked but
+ * the kernel has one CTA shape, 4 warps. */
 SICC_API int sicc_engine_set_launch_shape(unsigned long long handle, int warps_per_cta, int ctas);
 SICC_API int sicc_engine_decode_device(unsigned long long handle, int codewords, const unsigned char* device_code_ids,
                                        const float* device_llr, const long long* device_llr_offsets,

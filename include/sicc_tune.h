@@ -18,7 +18,7 @@
  *     osd_ctas            grid size;
  *   mixed-code engine (include/sicc_engine.h):
  *     warps per codeword of each registered code (1, 2 or 4: the check-node
- *     layer's rows spread over 32, 64 or 128 lanes) and warps per CTA.
+ *     layer's rows spread over 32, 64 or 128 lanes).
  *
  * Every shape gives bit-identical results: rows of one layer share no
  * variable, and OSD pruning only drops candidates that cannot win.
@@ -73,8 +73,7 @@ SICC_API int sicc_fec_autotune(unsigned long long handle, const float* device_ll
  * over 32 * warps lanes (w must be a multiple of 32 * warps for 2 and 4). */
 SICC_API int sicc_engine_set_code_warps(unsigned long long engine, int code_id, int warps);
 SICC_API int sicc_engine_get_code_warps(unsigned long long engine, int code_id, int* out_warps);
-/* Coordinate search over every code's warps per codeword and the engine's
- * warps per CTA, timing the mixed BP kernel on the caller's batch (the
+/* Coordinate search over every code's warps per codeword, timing the mixed BP kernel on the caller's batch (the
  * arguments of sicc_engine_decode_device; outputs are overwritten).  Applies
  * and caches the fastest; reports the default and the tuned BP time. */
 SICC_API int sicc_engine_autotune(unsigned long long engine, int codewords, const unsigned char* device_code_ids,

@@ -224,7 +224,8 @@ __device__ __forceinline__ unsigned lane_syndrome(const unsigned char* smem, con
 template <int D, int NL>
 constexpr int reg_threads() { return D * NL > 40 ? 128 : 256; }
 
-// The lanes of one codeword: G <= 32 lanes of a warp (W = 1) or W whole warps on a named barrier.
+// The lanes of one codeword: G <= 32 lanes of a warp (W = 1) or W whole warps on a named barrier
+// (1, 2 for groups of four warps, 3 .. 6 for groups of two: at most 256 threads).
 template <int W>
 struct Group {
     int G, gl, slot, lane, leader;
@@ -252,7 +253,7 @@ struct Group {
     __device__ __forceinline__ void sync() const
     {
         if constexpr (W == 1) __syncwarp(gmask);
-        else asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(W * 32) : "memory");
+        else asm volatile("bar.sync %0, %1;" ::"r"((W == 2 ? 3 : 1) + slot), "n"(W * 32) : "memory");
     }
     // Sum over the group, in every lane.  W > 1: two sums of a group need a sync() between them.
     __device__ __forceinline__ int sum(unsigned v) const

@@ -3,21 +3,27 @@
 // One batch holds codewords of several codes.  prepare_kernel groups them by
 // code (a counting sort in the queue order: widest layers, then largest cost
 // first) and sizes the work units; bp_mixed_kernel then runs persistently in
-// three phases, each unit decoded with its code's layered schedule (the same
-// arithmetic as bp_layered_kernel, so results are bit-exact with the
-// single-code decoders):
+// three phases, each unit decoded with its code's layered schedule (results are
+// bit-exact with the single-code decoders):
 //   1. groups of 4 warps take codewords of codes whose layers are >= 128 rows
 //      wide (one codeword per group, synchronised by a named barrier);
 //   2. groups of 2 warps take codes with 64-row layers;
 //   3. single warps take units of up to 32/G codewords of the narrower codes,
 //      G lanes each.
-// Wide codewords thus run on up to 128 lanes (a 2048-bit codeword is not
-// serialised on one warp) and every warp's shared-memory slot only has to
-// hold a quarter of the largest code's state.  Codewords whose syndrome fails
-// go to one OSD launch that reads each item's code tables.
+// A quasi-cyclic code with one row per lane and layer runs register-resident
+// (bp_reg.cuh: messages in registers, posteriors in shared memory): the lanes
+// load the code's row offsets once and keep them while the queue hands them the
+// same code.  Other codes (ragged layers, or a warps-per-codeword setting of the
+// caller's) keep compressed messages in shared memory.  Codewords whose syndrome
+// fails go to one OSD launch that reads each item's code tables.
+//
+// Shape: 4 warps per CTA, three CTAs per SM (168 registers).  20,000 codewords of
+// the 15-code mix: 1.47 ms with compressed messages for every code (8 warps per
+// CTA, ALU pipe 81% busy), 0.71 ms register-resident.
 #include "../../include/sicc_engine.h"
 #include "bp_device.cuh"
 #include "bp_kernels.h"
+#include "bp_reg.cuh"
 #include "code_plan.h"
 #include "engine_internal.h"
 #include "tune_internal.h"
@@ -42,6 +48,7 @@ struct CodeDesc {
     float alpha, beta;
     int route_osd;
     int slot_floats;  // shared-memory floats per codeword slot
+    int reg;          // 1: register-resident (one row per lane and layer, group = width)
     const int* vars;  // [num_layers][maxdeg][width]
 };
 
@@ -253,11 +260,11 @@ __device__ __forceinline__ void wide_unit(const MixedIO& io, const CodeDesc& d, 
     group_sync(bar, G);
     auto syndrome = [&]() -> int {
         const unsigned c = __reduce_add_sync(0xffffffffu, static_cast<unsigned>(lane_syndrome<D>(d, app, gl, G)));
-        if (lane == 0) s_red[g * W + (warp % W)] = static_cast<int>(c);
+        if (lane == 0) s_red[warp % W] = static_cast<int>(c);
         group_sync(bar, G);
         int tot = 0;
 #pragma unroll
-        for (int i = 0; i < W; ++i) tot += s_red[g * W + i];
+        for (int i = 0; i < W; ++i) tot += s_red[i];
         return tot;
     };
     int best_w = syndrome();
@@ -300,6 +307,140 @@ __device__ __forceinline__ void wide_unit(const MixedIO& io, const CodeDesc& d, 
     }
 }
 
+// ---- register-resident units (bp_reg.cuh) ----
+
+// A codeword's way through a register-resident decode, by its group's lanes; the slot is
+// [posteriors, dummy][best posteriors].
+template <int D, int NL, int W>
+struct RegUnit {
+    const MixedIO& io;
+    const CodeDesc& d;
+    const reg::Group<W>& g;
+    unsigned char* smem;
+    unsigned base;  // byte offset of the slot
+    float *app, *best;
+    reg::Rows<D, NL> rows;
+    float msg[NL][D];
+    int cw = 0, iter = 0, best_w = 0;
+    bool route = false;
+
+    __device__ __forceinline__ RegUnit(const MixedIO& io_, const CodeDesc& d_, const reg::Group<W>& g_,
+                                       unsigned char* smem_, unsigned base_)
+        : io(io_), d(d_), g(g_), smem(smem_), base(base_)
+    {
+        const int n_pad = (d.n + 3) & ~3;
+        app = reinterpret_cast<float*>(smem + base);
+        best = app + n_pad + 4;
+        rows.load(d.vars, d.num_layers, 1, d.width, d.maxdeg, g.G, g.gl, base, n_pad);
+        if (g.gl == 0) app[n_pad] = __int_as_float(0x7f800000);  // +inf, before start's sync
+    }
+    __device__ __forceinline__ void start(int codeword)
+    {
+        cw = codeword;
+        route = d.route_osd && (io.protect == nullptr || io.protect[cw]);
+        const float* src = io.llr + io.llr_off[cw];
+        if ((d.n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+            for (int i = g.gl; i < (d.n >> 2); i += g.G) {
+                const float4 v = __ldcs(reinterpret_cast<const float4*>(src) + i);
+                reinterpret_cast<float4*>(app)[i] =
+                    make_float4(reg::canonical(v.x), reg::canonical(v.y), reg::canonical(v.z), reg::canonical(v.w));
+                if (route) reinterpret_cast<float4*>(best)[i] = v;
+            }
+        } else {
+            for (int i = g.gl; i < d.n; i += g.G) {
+                const float v = __ldcs(src + i);
+                app[i] = reg::canonical(v);
+                if (route) best[i] = v;
+            }
+        }
+        reg::static_for<NL>([&](auto ti) {
+#pragma unroll
+            for (int j = 0; j < D; ++j) msg[decltype(ti)::value][j] = 0.0f;
+        });
+        g.sync();
+        best_w = g.sum(reg::lane_syndrome<true>(smem, rows, NL));
+        iter = 0;
+    }
+    // One iteration; true when the codeword has stopped (its outputs are written then).
+    __device__ __forceinline__ bool step()
+    {
+        reg::static_for<NL>([&](auto ti) {
+            constexpr int t = decltype(ti)::value;
+            reg::update_row(smem, rows, t, d.alpha, d.beta, msg[t]);
+            g.sync();
+        });
+        const int w = g.sum(reg::lane_syndrome<true>(smem, rows, NL));
+        ++iter;
+        if (route && w < best_w && w != 0) {
+            reg::copy_slot(g, best, app, (d.n + 3) & ~3);
+            g.sync();  // copied before the next layer rewrites the posteriors
+        }
+        best_w = min(best_w, w);
+        if (w != 0 && iter < d.max_iter) return false;
+        if (g.gl == 0) {
+            if (io.success) io.success[cw] = w == 0 ? 1 : 0;
+            if (io.iterations) io.iterations[cw] = static_cast<uint8_t>(iter);
+            if (io.used_osd) io.used_osd[cw] = 0;
+        }
+        uint8_t* dst = io.info + io.info_off[cw];
+        for (int i = g.gl; i < d.k; i += g.G) dst[i] = app[i] < 0.0f ? 1 : 0;
+        if (w != 0 && route) {
+            unsigned long long off = 0ull;
+            if (g.gl == 0) {
+                const int it = atomicAdd(io.osd_count, 1);
+                off = atomicAdd(io.osd_floats, static_cast<unsigned long long>(d.n));
+                io.osd_index[it] = cw;
+                io.osd_rowoff[it] = static_cast<long long>(off);
+            }
+            const unsigned lo = g.from_leader(static_cast<int>(off)), hi = g.from_leader(static_cast<int>(off >> 32));
+            float* o = io.osd_llr + ((static_cast<unsigned long long>(hi) << 32) | lo);
+            for (int i = g.gl; i < d.n; i += g.G) o[i] = best[i];
+        }
+        return true;
+    }
+};
+
+// Units of queue position q from u on, as long as the counter keeps handing out units of q
+// below u_end; returns the first unit that is not one of them.  One codeword per unit (W > 1).
+template <int D, int NL, int W>
+__device__ __noinline__ int reg_wide_run(const MixedIO& io, const CodeDesc& d, int q, int u, int u_end, int* counter,
+                            unsigned char* smem, unsigned base, int* red)
+{
+    const reg::Group<W> g(W * 32, red);
+    RegUnit<D, NL, W> unit(io, d, g, smem, base);
+    const int last = min(u_end, io.q_units[q + 1]), first = io.q_units[q], start = io.q_start[q];
+    do {
+        unit.start(io.order[start + (u - first)]);
+        while (!unit.step()) {}
+        u = g.from_leader(g.gl == 0 ? atomicAdd(counter, 1) : 0);
+    } while (u < last);
+    return u;
+}
+
+// As reg_wide_run for one warp: a unit is up to 32 / G codewords, one per group of G lanes,
+// in step until all have stopped.
+template <int D, int NL>
+__device__ __noinline__ int reg_narrow_run(const MixedIO& io, const CodeDesc& d, int q, int u, int* counter, unsigned char* smem,
+                              unsigned warp_base)
+{
+    const reg::Group<1> g(d.group, nullptr);
+    const int per = 32 / d.group, sub = g.lane / d.group;
+    RegUnit<D, NL, 1> unit(io, d, g, smem, warp_base + static_cast<unsigned>(sub * d.slot_floats) * 4u);
+    const int last = io.q_units[q + 1], first = io.q_units[q], start = io.q_start[q], count = io.q_start[q + 1] - start;
+    do {
+        const int local = (u - first) * per + sub;
+        bool active = local < count;
+        if (active) unit.start(io.order[start + local]);
+        while (__any_sync(0xffffffffu, active))
+            if (active) active = !unit.step();
+        __syncwarp();
+        u = 0;
+        if (g.lane == 0) u = atomicAdd(counter, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+    } while (u < last);
+    return u;
+}
+
 // Phase of groups of W warps (W = 4: named barriers 1-2, W = 2: 3-6), one
 // codeword per group at a time from `counter`, up to unit `u_end`.  The
 // group scalars (s_unit, s_red, s_off) are the phase's own: a group of the
@@ -317,21 +458,32 @@ __device__ void wide_phase(const MixedIO& io, float* smem_f, int warp_floats, in
     float* app = smem_f + static_cast<size_t>(g * W) * warp_floats;
     const int gwarp0 = blockIdx.x * (blockDim.x >> 5) + g * W;
     float* best = io.best + static_cast<size_t>(gwarp0) * io.best_slots * io.n_max;
-    for (;;) {
+    auto next = [&]() -> int {  // the same value for the whole group
         if (gl == 0) s_unit[g] = atomicAdd(counter, 1);
         group_sync(bar, G);
         const int u = s_unit[g];
-        if (u >= u_end) break;  // the same value for the whole group
-        int q = 0;
+        group_sync(bar, G);  // read before it is written again
+        return u;
+    };
+    int* red = s_red + g * (W + 1);  // the group's own, in both kinds of unit (as reg::Group has it)
+    int u = next(), q = 0;
+    while (u < u_end) {
         while (q + 1 < io.K && u >= io.q_units[q + 1]) ++q;
         const CodeDesc d = io.codes[io.q_code[q]];
+        if (d.reg) {
+            unsigned char* smem = reinterpret_cast<unsigned char*>(smem_f);
+            const unsigned base = static_cast<unsigned>(g * W * warp_floats) * 4u;
+            if (d.num_layers == 8) u = reg_wide_run<10, 8, W>(io, d, q, u, u_end, counter, smem, base, s_red);
+            else if (d.num_layers == 5) u = reg_wide_run<14, 5, W>(io, d, q, u, u_end, counter, smem, base, s_red);
+            else u = reg_wide_run<14, 4, W>(io, d, q, u, u_end, counter, smem, base, s_red);
+            continue;
+        }
         const int cw = io.order[io.q_start[q] + (u - io.q_units[q])];
         // row loops unrolled to the closest D above the code's row degree
-        if (d.maxdeg <= 10) wide_unit<10, W>(io, d, cw, app, best, g, gl, bar, s_red, s_off);
-        else if (d.maxdeg <= 12) wide_unit<12, W>(io, d, cw, app, best, g, gl, bar, s_red, s_off);
-        else if (d.maxdeg <= 14) wide_unit<14, W>(io, d, cw, app, best, g, gl, bar, s_red, s_off);
-        else wide_unit<D, W>(io, d, cw, app, best, g, gl, bar, s_red, s_off);
-        group_sync(bar, G);  // the slot and s_unit are rewritten by the next unit
+        if (d.maxdeg <= 10) wide_unit<10, W>(io, d, cw, app, best, g, gl, bar, red, s_off);
+        else wide_unit<D, W>(io, d, cw, app, best, g, gl, bar, red, s_off);
+        group_sync(bar, G);  // the slot is rewritten by the next unit
+        u = next();
     }
 }
 
@@ -414,14 +566,17 @@ __device__ __forceinline__ void narrow_unit(const MixedIO& io, const CodeDesc& d
     __syncwarp();
 }
 
+constexpr int kMixedWarps = 4;  // warps per CTA
+
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kMixedWarps * 32, 3)
 bp_mixed_kernel(MixedIO io, int warp_floats)
 {
     extern __shared__ __align__(16) float smem_f[];
-    __shared__ int s_unit4[2], s_unit2[4];
-    __shared__ int s_red4[8], s_red2[8];
-    __shared__ unsigned long long s_off4[2], s_off2[4];
+    __shared__ int s_unit4[1], s_unit2[2];
+    __shared__ int s_red4[5], s_red2[6];
+    __shared__ unsigned long long s_off4[1], s_off2[2];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(smem_f);
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
 
@@ -431,20 +586,26 @@ bp_mixed_kernel(MixedIO io, int warp_floats)
 
     // phase 3: one warp per unit
     float* wbase = smem_f + static_cast<size_t>(warp) * warp_floats;
-    const int gwarp = blockIdx.x * (blockDim.x >> 5) + warp;
+    const int gwarp = blockIdx.x * kMixedWarps + warp;
     const int total_units = io.q_units[io.K];
-    for (;;) {
-        int u = 0;
-        if (lane == 0) u = atomicAdd(io.work1, 1);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if (u >= total_units) break;
-        int q = 0;
+    int u = 0, q = 0;
+    if (lane == 0) u = atomicAdd(io.work1, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    while (u < total_units) {
         while (q + 1 < io.K && u >= io.q_units[q + 1]) ++q;
         const CodeDesc d = io.codes[io.q_code[q]];
+        if (d.reg) {
+            const unsigned base = static_cast<unsigned>(warp * warp_floats) * 4u;
+            if (d.num_layers == 8) u = reg_narrow_run<10, 8>(io, d, q, u, io.work1, smem, base);
+            else if (d.num_layers == 5) u = reg_narrow_run<14, 5>(io, d, q, u, io.work1, smem, base);
+            else u = reg_narrow_run<14, 4>(io, d, q, u, io.work1, smem, base);
+            continue;
+        }
+        // row loops unrolled to the closest D above the code's row degree
         if (d.maxdeg <= 10) narrow_unit<10>(io, d, q, u, wbase, gwarp);
-        else if (d.maxdeg <= 12) narrow_unit<12>(io, d, q, u, wbase, gwarp);
-        else if (d.maxdeg <= 14) narrow_unit<14>(io, d, q, u, wbase, gwarp);
         else narrow_unit<D>(io, d, q, u, wbase, gwarp);
+        if (lane == 0) u = atomicAdd(io.work1, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
     }
 }
 
@@ -472,8 +633,9 @@ bool code_warps_allowed(int width, int warps)
 }
 
 // Lanes and rows per lane of a code decoded by `warps` warps per codeword, and the
-// shared-memory floats of one codeword slot.
-void set_code_warps(EngineCode& ec, int warps)
+// shared-memory floats of one codeword slot.  A plain code at its default warps is decoded
+// register-resident, if `allow_reg`.
+void set_code_warps(EngineCode& ec, int warps, bool allow_reg = true)
 {
     const LayeredView& lv = ec.code->layered_view();
     CodeDesc& d = ec.desc;
@@ -485,9 +647,11 @@ void set_code_warps(EngineCode& ec, int warps)
         d.group = 32 * warps;
         d.rows_per_lane = lv.width / d.group;
     }
+    d.reg = allow_reg && lv.reg_plain && warps == default_code_warps(lv.width) ? 1 : 0;
     const int n_pad = (d.n + 3) & ~3;
     // posteriors, the dummy edge's +inf (padded to 4 floats), then the row messages
-    int sf = (n_pad + 4 + 3 * d.num_layers * d.width + 3) & ~3;
+    // (register-resident: the best posteriors)
+    int sf = (n_pad + 4 + (d.reg ? n_pad : 3 * d.num_layers * d.width) + 3) & ~3;
     sf = pad_slot_stride(sf, d.group);
     d.slot_floats = sf;
 }
@@ -498,7 +662,7 @@ struct Engine {
     std::vector<EngineCode> codes;
     int n_max = 0, k_max = 0, maxdeg = 0, osd_nmax = 0, osd_kmax = 0;
     OsdHBounds h_cls[kOsdHClasses];  // large-code OSD launch bounds, by class
-    int warps_per_cta = 0, ctas = 0;
+    int ctas = 0;
     // device state
     CodeDesc* d_codes = nullptr;
     OsdView* d_views = nullptr;
@@ -564,10 +728,34 @@ struct Engine {
         return (w + 3) & ~3;
     }
 
+    // Shared memory of a CTA of the mixed kernel.  The register-resident units hold 16-bit byte
+    // offsets into it, so with a larger CTA (a wide ragged code on one warp) no code runs so.
+    size_t mixed_smem()
+    {
+        size_t smem = static_cast<size_t>(kMixedWarps) * warp_floats() * sizeof(float);
+        if (smem > 65536)
+            for (auto& c : codes)
+                if (c.desc.reg) {
+                    set_code_warps(c, c.desc.warps, false);
+                    dirty = true;
+                }
+        return static_cast<size_t>(kMixedWarps) * warp_floats() * sizeof(float);
+    }
+
+    // Codewords a warp holds at once with its best posteriors in the global scratch.
+    int best_slots() const
+    {
+        int slots = 0;
+        for (const auto& c : codes)
+            if (!c.desc.reg) slots = std::max(slots, c.desc.warps == 1 ? 32 / c.desc.group : 1);
+        return slots;
+    }
+
     // Uploads the code descriptors and the queue order after codes change.
     void commit()
     {
         if (!dirty) return;
+        mixed_smem();  // settles which codes run register-resident
         const int K = static_cast<int>(codes.size());
         std::vector<CodeDesc> descs(K);
         std::vector<OsdView> views(K);
@@ -628,40 +816,43 @@ int guarded(F&& f)
     }
 }
 
+// Grid of the mixed kernel, with its shared-memory grant and its best-posterior scratch (for the
+// codes that are not register-resident) in place.
 template <int D>
-void launch_mixed(Engine& e, const MixedIO& io, cudaStream_t st)
+int prepare_mixed(Engine& e)
 {
-    const int wf = e.warp_floats();
-    // whole groups of 4 warps (the wide phases split a CTA into groups of 4 and 2 warps)
-    int warps = e.warps_per_cta == 4 ? 4 : 8;
-    if (static_cast<size_t>(warps) * wf * sizeof(float) > 200 * 1024) warps = 4;
-    const size_t smem = static_cast<size_t>(warps) * wf * sizeof(float);
+    const size_t smem = e.mixed_smem();
     if (smem > 227 * 1024) throw InvalidArgument("a registered code is too large for the mixed kernel");
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(bp_mixed_kernel<D>), smem),
                "cudaFuncSetAttribute(bp_mixed)");
     int ctas = e.ctas;
     if (ctas <= 0) {
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_mixed_kernel<D>, warps * 32, smem) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_mixed_kernel<D>, kMixedWarps * 32, smem) !=
                 cudaSuccess ||
             per_sm <= 0)
             per_sm = 1;
         ctas = per_sm * device_sm_count();
     }
-    // a warp holds one codeword of a wide code, or 32 / group codewords of a narrow one
-    int slots = 1;
-    for (const auto& c : e.codes)
-        if (c.desc.warps == 1) slots = std::max(slots, 32 / c.desc.group);
-    const size_t need = static_cast<size_t>(ctas) * warps * slots * static_cast<size_t>(e.n_max);
+    const size_t need = static_cast<size_t>(ctas) * kMixedWarps * e.best_slots() * static_cast<size_t>(e.n_max);
     if (need > e.best_floats) {
         if (e.d_best) cudaFree(e.d_best);
+        e.d_best = nullptr;
+        e.best_floats = 0;
         check_cuda(cudaMalloc(&e.d_best, need * sizeof(float)), "cudaMalloc(best)");
         e.best_floats = need;
     }
+    return ctas;
+}
+
+template <int D>
+void launch_mixed(Engine& e, const MixedIO& io, cudaStream_t st)
+{
+    const int ctas = prepare_mixed<D>(e), wf = e.warp_floats();
     MixedIO m = io;
     m.best = e.d_best;
-    m.best_slots = slots;
-    bp_mixed_kernel<D><<<ctas, warps * 32, smem, st>>>(m, wf);
+    m.best_slots = e.best_slots();
+    bp_mixed_kernel<D><<<ctas, kMixedWarps * 32, kMixedWarps * wf * sizeof(float), st>>>(m, wf);
     check_cuda(cudaGetLastError(), "bp_mixed_kernel launch");
 }
 
@@ -827,7 +1018,7 @@ int sicc_engine_set_launch_shape(unsigned long long handle, int warps_per_cta, i
         auto e = get(handle);
         std::lock_guard<std::mutex> lock(e->mu);
         if (warps_per_cta < 0 || warps_per_cta > 8 || ctas < 0) throw InvalidArgument("warps_per_cta must be 0..8");
-        e->warps_per_cta = warps_per_cta;
+        // the kernel has one CTA shape (kMixedWarps); the argument is checked and otherwise unused
         e->ctas = ctas;
         return CUDA_OSD_STATUS_OK;
     });
@@ -872,32 +1063,8 @@ int engine_prepare_capture(unsigned long long handle, int max_codewords)
             throw InvalidArgument("codewords must be in 1..max_codewords");
         check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
         e->commit();
-        // the mixed kernel's best-posterior scratch for the grid it will use (no allocation later)
-        const int wf = e->warp_floats();
-        int warps = e->warps_per_cta == 4 ? 4 : 8;
-        if (static_cast<size_t>(warps) * wf * sizeof(float) > 200 * 1024) warps = 4;
-        const size_t smem = static_cast<size_t>(warps) * wf * sizeof(float);
-        check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(bp_mixed_kernel<16>), smem),
-                   "cudaFuncSetAttribute(bp_mixed)");
-        int ctas = e->ctas;
-        if (ctas <= 0) {
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_mixed_kernel<16>, warps * 32, smem) !=
-                    cudaSuccess ||
-                per_sm <= 0)
-                per_sm = 1;
-            ctas = per_sm * device_sm_count();
-        }
-        int slots = 1;
-        for (const auto& c : e->codes)
-            if (c.desc.warps == 1) slots = std::max(slots, 32 / c.desc.group);
-        const size_t need = static_cast<size_t>(ctas) * warps * slots * static_cast<size_t>(e->n_max);
-        if (need > e->best_floats) {
-            if (e->d_best) cudaFree(e->d_best);
-            e->d_best = nullptr;
-            check_cuda(cudaMalloc(&e->d_best, need * sizeof(float)), "cudaMalloc(best)");
-            e->best_floats = need;
-        }
+        // the mixed kernel's grant and best-posterior scratch for the grid it will use (no allocation later)
+        prepare_mixed<16>(*e);
         return CUDA_OSD_STATUS_OK;
     });
 }
@@ -1075,8 +1242,7 @@ int sicc_engine_last_ms(unsigned long long handle, float* out_prepare_ms, float*
 }
 
 // Coordinate search on the caller's batch: codes in decreasing BP cost, each tried at every
-// allowed warps per codeword (kept when the mixed BP kernel gets at least 1% faster), then the
-// engine's warps per CTA.  Trials decode with every codeword's protection at BP only, so OSD
+// allowed warps per codeword (kept when the mixed BP kernel gets at least 1% faster).  Trials decode with every codeword's protection at BP only, so OSD
 // time stays out of the comparison; each trial is one warm-up and `reps` timed decodes.
 int sicc_engine_autotune(unsigned long long handle, int codewords, const unsigned char* device_code_ids,
                          const float* device_llr, const long long* device_llr_offsets, unsigned char* device_info,
@@ -1152,26 +1318,8 @@ int sicc_engine_autotune(unsigned long long handle, int codewords, const unsigne
                 }
             }
         }
-        int wpc_keep = 0;
         {
             std::lock_guard<std::mutex> lock(e->mu);
-            wpc_keep = e->warps_per_cta;
-        }
-        for (int wpc : {4, 8}) {
-            if (wpc == (wpc_keep == 0 ? 8 : wpc_keep)) continue;
-            {
-                std::lock_guard<std::mutex> lock(e->mu);
-                e->warps_per_cta = wpc;
-            }
-            const float t = time_bp();
-            if (t < 0.99f * best) {
-                best = t;
-                wpc_keep = wpc;
-            }
-        }
-        {
-            std::lock_guard<std::mutex> lock(e->mu);
-            e->warps_per_cta = wpc_keep;
             for (const auto& c : e->codes) tune_cache_put(tune_key("engine-code", c.fingerprint), {c.desc.warps});
         }
         if (out_default_ms) *out_default_ms = default_ms;

@@ -82,7 +82,7 @@ class Engine:
         tune.set_code_warps(self.handle, code_id, warps)
 
     def autotune(self, codewords, d_code, d_llr, d_llr_off, d_info, d_info_off, reps: int = 3):
-        """Tunes warps per codeword of each code and warps per CTA on this batch (outputs are
+        """Tunes warps per codeword of each code on this batch (outputs are
         overwritten); returns (default BP ms, tuned BP ms)."""
         from . import tune
         return tune.engine_autotune(self.handle, codewords, d_code, d_llr, d_llr_off, d_info, d_info_off, reps)
