@@ -48,6 +48,8 @@ size_t flooding_smem_bytes(const FloodView& cv, int warps, int* slot_floats_out)
 // codeword, state in an L2-sized global scratch block.  launch_bp_layered /
 // launch_bp_flooding hand such codes to these.
 bool layered_needs_wide(const LayeredView& cv, bool track_best);
+int wide_split(int n);          // posteriors the layered wide kernel keeps in shared memory
+int wide_slots(int maxdeg);     // edge slots of its row table
 bool flooding_needs_wide(const FloodView& cv);
 void launch_bp_layered_wide(const LayeredView& cv, const BpParams& p, const BpIO& io, cudaStream_t st);
 void launch_bp_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO& io, cudaStream_t st);

@@ -42,7 +42,7 @@ __device__ __forceinline__ void static_for(F&& f)
     static_for_(std::make_integer_sequence<int, N>(), f);
 }
 
-// Edges 0 .. D-1 of a row in up to four groups of two to four.
+// Edges 0 .. D-1 of a row (D <= 16) in two to four groups of two to four.
 template <int D>
 struct Split {
     static constexpr int ng = D <= 6 ? 2 : D <= 8 ? 3 : 4;
@@ -64,6 +64,21 @@ __device__ __forceinline__ float minx(float a, float b)
 template <int D>
 __device__ __forceinline__ void exclusive_min(const float (&a)[D], float (&m)[D])
 {
+    if constexpr (D > 16) {  // prefix and suffix minima: three operations per edge, few registers
+        float run = FLT_MAX;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            m[j] = run;
+            run = minx(run, a[j]);
+        }
+        run = FLT_MAX;
+#pragma unroll
+        for (int j = D - 1; j >= 0; --j) {
+            m[j] = minx(m[j], run);
+            run = minx(run, a[j]);
+        }
+        return;
+    }
     using S = Split<D>;
     float g[4], e[4], pr[4][3];
     static_for<S::ng>([&](auto gi) {

@@ -1,30 +1,28 @@
 // Belief propagation for long codes (DVB-S2 N16200 / N64800 class) whose
 // decoder state does not fit one CTA's shared memory.
 //
-// One CTA of 512 threads decodes one codeword at a time and takes the next
-// from a global counter when it stops.  The posteriors live in shared memory
-// when they fit (n <= ~50k); for longer codes the layered kernel keeps the
-// first 56,320 in shared memory and the rest in the CTA's slice of a global
-// scratch block (the flooding kernel keeps them all there); the compressed check messages (alpha*min1, alpha*min2, argmin,
-// signs per row) and, for the flooding schedule, the variable-to-check
-// messages of every edge live in that slice too.  A slice is touched by one
-// CTA only, so it stays in L2 when the grid's slices fit there (the launcher
-// sizes the grid for that).
+// One CTA decodes one codeword at a time and takes the next from a global
+// counter when it stops.  The posteriors live in shared memory when they fit
+// (n <= ~50k); for longer codes the layered kernel keeps the first 56,320 in
+// shared memory and the rest in the CTA's slice of a global scratch block (the
+// flooding kernel keeps them all there); the row messages live in that slice
+// too.  A slice is touched by one CTA only, so it stays in L2 when the grid's
+// slices fit there (the launcher sizes the grid for that).
 //
 //   layered (schedules 2, 3): the rows of a layer touch disjoint variables,
 //     so the CTA's threads update them in parallel, one barrier per layer;
-//     the per-row arithmetic is the shared-memory layered kernel's
-//     (bp_kernels.cu), operation for operation.
+//     the row arithmetic gives the shared-memory layered kernel's values
+//     (bp_kernels.cu).
 //   flooding (schedules 0, 1): check phase over all rows, variable phase
 //     over all columns (the reference CPU decoder, uhd_ldpc_ofdm_link.cpp:
-//     3013-3094, with the MB damping of cpu_bp_osd_decode.m:180-183), the
-//     shared-memory flooding kernel's arithmetic with CTA-wide loops.
+//     3013-3094, with the MB damping of cpu_bp_osd_decode.m:180-183).
 //
 // Results, stopping rule (zero syndrome or the iteration cap), best-syndrome
 // tracking and the OSD hand-off are those of the shared-memory kernels, so
 // both give the same bits for a code that fits either.
 #include "bp_device.cuh"
 #include "bp_kernels.h"
+#include "bp_reg.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -33,10 +31,8 @@ namespace sicc {
 
 namespace {
 
-constexpr int kWideThreads = 512;
-constexpr int kWideWarps = kWideThreads / 32;
-
-// CTA-wide sum; every thread gets the total.  `red` holds kWideWarps ints.
+// CTA-wide sum; every thread gets the total.  `red` holds one int per warp.
+template <int kThreads>
 __device__ __forceinline__ int cta_sum(int v, int* red)
 {
     v = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(v)));
@@ -45,10 +41,11 @@ __device__ __forceinline__ int cta_sum(int v, int* red)
     __syncthreads();
     int t = 0;
 #pragma unroll
-    for (int i = 0; i < kWideWarps; ++i) t += red[i];
+    for (int i = 0; i < kThreads / 32; ++i) t += red[i];
     return t;
 }
 
+template <int kThreads>
 __device__ __forceinline__ unsigned cta_min(unsigned v, int* red)
 {
     v = __reduce_min_sync(0xffffffffu, v);
@@ -57,12 +54,12 @@ __device__ __forceinline__ unsigned cta_min(unsigned v, int* red)
     __syncthreads();
     unsigned t = 0xffffffffu;
 #pragma unroll
-    for (int i = 0; i < kWideWarps; ++i) t = min(t, static_cast<unsigned>(red[i]));
+    for (int i = 0; i < kThreads / 32; ++i) t = min(t, static_cast<unsigned>(red[i]));
     return t;
 }
 
 // Outputs of a finished codeword (the shared-memory kernels' finalize step).
-template <class App>
+template <int kThreads, class App>
 __device__ void wide_finish(const BpParams& p, const BpIO& io, int c, int n, int w, int iter, const App& app,
                             const float* best, bool track_best, int* red, int* s_slot)
 {
@@ -70,8 +67,8 @@ __device__ void wide_finish(const BpParams& p, const BpIO& io, int c, int n, int
     bool accept = (w == 0);
     if (accept && p.min_abs_accept > 0.0f) {
         unsigned mn = 0x7f800000u;
-        for (int i = tid; i < n; i += kWideThreads) mn = min(mn, __float_as_uint(fabsf(app.ld(i))));
-        accept = __uint_as_float(cta_min(mn, red)) >= p.min_abs_accept;
+        for (int i = tid; i < n; i += kThreads) mn = min(mn, __float_as_uint(fabsf(app.ld(i))));
+        accept = __uint_as_float(cta_min<kThreads>(mn, red)) >= p.min_abs_accept;
     }
     const bool route = !accept && p.route_failures_to_osd && io.osd_llr != nullptr;
     if (tid == 0) {
@@ -82,17 +79,17 @@ __device__ void wide_finish(const BpParams& p, const BpIO& io, int c, int n, int
     }
     if (io.out_bits) {
         uint8_t* dst = io.out_bits + static_cast<size_t>(c) * io.out_stride;
-        for (int i = tid; i < io.out_len; i += kWideThreads) dst[i] = app.ld(i) < 0.0f ? 1 : 0;
+        for (int i = tid; i < io.out_len; i += kThreads) dst[i] = app.ld(i) < 0.0f ? 1 : 0;
     }
     if (io.app_out) {
         float* dst = io.app_out + static_cast<size_t>(c) * n;
-        for (int i = tid; i < n; i += kWideThreads) dst[i] = app.ld(i);
+        for (int i = tid; i < n; i += kThreads) dst[i] = app.ld(i);
     }
     __syncthreads();  // s_slot
     if (route) {
         const int s = *s_slot;
         float* dst = io.osd_llr + static_cast<size_t>(s) * n;
-        for (int i = tid; i < n; i += kWideThreads) dst[i] = track_best ? best[i] : app.ld(i);
+        for (int i = tid; i < n; i += kThreads) dst[i] = track_best ? best[i] : app.ld(i);
         if (tid == 0) io.osd_index[s] = c;
     }
 }
@@ -106,153 +103,78 @@ __device__ __forceinline__ int wide_next(const BpIO& io, int* s_next)
     return *s_next;
 }
 
-// Posteriors of the layered wide kernel: those of variables below `split` in shared
-// memory, the rest in the CTA's global slice (L2), so a code a little too long for shared
-// memory keeps most of its posterior gathers on chip.
+// Posteriors of the layered wide kernel by byte offset (4 x variable): those below `split` in
+// shared memory, the rest in the CTA's global slice (L2), so a code a little too long for
+// shared memory keeps most of its posterior gathers on chip.
 struct SplitApp {
-    float* s;   // shared memory, variables [0, split)
-    float* g;   // global slice, indexed by the variable (entries below split unused)
-    int split;
-    __device__ __forceinline__ float ld(int v) const { return v < split ? s[v] : g[v]; }
-    __device__ __forceinline__ void st(int v, float x) const
+    unsigned char* s;
+    unsigned char* g;  // same offsets; the bytes below `split` are unused
+    unsigned split;
+    __device__ __forceinline__ float at(unsigned off) const
     {
-        if (v < split) s[v] = x;
-        else g[v] = x;
+        return off < split ? *reinterpret_cast<const float*>(s + off) : *reinterpret_cast<const float*>(g + off);
+    }
+    __device__ __forceinline__ void put(unsigned off, float x) const
+    {
+        if (off < split) *reinterpret_cast<float*>(s + off) = x;
+        else *reinterpret_cast<float*>(g + off) = x;
+    }
+    __device__ __forceinline__ float ld(int v) const { return at(4u * static_cast<unsigned>(v)); }
+};
+
+// What a row update reads besides posteriors: the row's posterior offsets (16-byte loads) and
+// its compressed messages.
+template <int D>
+struct WideRow {
+    static constexpr int kQuads = (D + 3) / 4;
+    uint4 o[kQuads];
+    float m1, m2;
+    unsigned meta;
+
+    __device__ __forceinline__ unsigned off(int j) const
+    {
+        const uint4& x = o[j >> 2];
+        return (j & 3) == 0 ? x.x : (j & 3) == 1 ? x.y : (j & 3) == 2 ? x.z : x.w;
+    }
+    __device__ __forceinline__ void load_offsets(const uint4* __restrict__ table, int row)
+    {
+#pragma unroll
+        for (int i = 0; i < kQuads; ++i) o[i] = __ldg(table + static_cast<size_t>(row) * kQuads + i);
+    }
+    __device__ __forceinline__ void load(const uint4* __restrict__ table, int row, bool fresh, const float* r1,
+                                         const float* r2, const unsigned* mt)
+    {
+        load_offsets(table, row);
+        m1 = fresh ? 0.0f : r1[row];  // a codeword's first iteration: no messages yet
+        m2 = fresh ? 0.0f : r2[row];
+        meta = fresh ? 0u : mt[row];
     }
 };
 
-// Rows a thread updates together in a layer: their loads are all issued before the
-// first store (the rows of a layer touch disjoint variables), so the latencies overlap.
-// Two for row degrees up to 16; one above, where the registers would spill.
+// Threads: row degrees up to 10 leave room for 1,024 threads (64 registers), which hide the L2
+// latency of tables and messages; wider rows take 512.
 template <int D>
-constexpr int row_batch() { return D <= 16 ? 2 : 1; }
-
-// Empty edge slots of short rows point at a dummy posterior (+inf: never a row's minimum,
-// argmin or sign, never a parity flip, and left at +inf by its update), so the edge loops
-// test only `j < cv.maxdeg`, the same for every thread.  Above D = 8 the slots keep -1 and
-// a per-edge test: the dummy form's registers would spill there.
-template <int D>
-constexpr bool dummy_slots() { return D <= 8; }
-
-// Layered update of rows rs0, rs0 + kWideThreads, ... (kRowBatch of them, those below
-// `rows`) of layer L, whose messages start at row `first` of the layer-ordered message
-// arrays: the shared-memory layered kernel's per-row arithmetic (bp_kernels.cu).
-template <int D, int kRowBatch = row_batch<D>()>
-__device__ __forceinline__ void wide_rows(const LayeredView& cv, const BpParams& p, int L, int rs0, int rows,
-                                          int first, const SplitApp& app, int dummy, float* r1, float* r2,
-                                          unsigned* meta)
-{
-    int v[kRowBatch][D];
-    float o1[kRowBatch], o2[kRowBatch], x[kRowBatch][D];
-    unsigned om[kRowBatch];
-#pragma unroll
-    for (int b = 0; b < kRowBatch; ++b) {
-        const int rs = rs0 + b * kWideThreads;
-        const bool live = rs < rows;
-        const int* vp = cv.vars + (L * cv.maxdeg) * cv.width + rs;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-            const int vj = (live && j < cv.maxdeg) ? __ldg(vp + j * cv.width) : -1;
-            v[b][j] = (vj >= 0 || !dummy_slots<D>()) ? vj : dummy;
-        }
-        const int ridx = first + rs;
-        o1[b] = live ? r1[ridx] : 0.0f;
-        o2[b] = live ? r2[ridx] : 0.0f;
-        om[b] = live ? meta[ridx] : 0u;
-    }
-    auto used = [&](int b, int j) { return dummy_slots<D>() ? j < cv.maxdeg : v[b][j] >= 0; };
-    if constexpr (dummy_slots<D>()) {
-#pragma unroll
-        for (int b = 0; b < kRowBatch; ++b) {
-            if (rs0 + b * kWideThreads < rows) {
-#pragma unroll
-                for (int j = 0; j < D; ++j) x[b][j] = (j < cv.maxdeg) ? app.ld(v[b][j]) : 0.0f;
-            }
-        }
-    } else {
-#pragma unroll
-        for (int b = 0; b < kRowBatch; ++b)
-#pragma unroll
-            for (int j = 0; j < D; ++j) x[b][j] = v[b][j] >= 0 ? app.ld(v[b][j]) : 0.0f;
-    }
-#pragma unroll
-    for (int b = 0; b < kRowBatch; ++b) {
-        if (dummy_slots<D>() ? rs0 + b * kWideThreads >= rows : v[b][0] < 0) continue;  // past the layer
-        float q[D];
-        float m1 = FLT_MAX, m2 = FLT_MAX;
-        int idx = 0;
-        unsigned neg = 0;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-            q[j] = 0.0f;
-            if (used(b, j)) {
-                const float qj = __fsub_rn(x[b][j], rebuild(o1[b], o2[b], om[b], j));
-                q[j] = qj;
-                neg |= (qj < 0.0f) ? (1u << j) : 0u;
-                const float a = fabsf(qj);
-                idx = (a < m1) ? j : idx;
-                m2 = fminf(m2, fmaxf(m1, a));
-                m1 = fminf(m1, a);
-            }
-        }
-        const unsigned tot = static_cast<unsigned>(__popc(neg)) & 1u;
-        const float n1 = nms_mag(p.alpha, p.beta, m1);
-        const float n2 = nms_mag(p.alpha, p.beta, m2);
-        const unsigned nm = ((neg ^ (0u - tot)) & 0x07FFFFFFu) | (static_cast<unsigned>(idx) << 27);
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-            if (used(b, j)) {
-                const unsigned sg = (nm >> j) & 1u;
-                const float mag = (j == idx) ? n2 : n1;
-                app.st(v[b][j], __fadd_rn(q[j], sg ? -mag : mag));
-            }
-        }
-        const int ridx = first + rs0 + b * kWideThreads;
-        r1[ridx] = n1;
-        r2[ridx] = n2;
-        meta[ridx] = nm;
-    }
-}
-
-// Unsatisfied checks among the same rows under hard(app).
-template <int D, int kRowBatch = row_batch<D>()>
-__device__ __forceinline__ int wide_parity(const LayeredView& cv, int L, int rs0, int rows, const SplitApp& app,
-                                           int dummy)
-{
-    int v[kRowBatch][D];
-#pragma unroll
-    for (int b = 0; b < kRowBatch; ++b) {
-        const int rs = rs0 + b * kWideThreads;
-        const bool live = rs < rows;
-        const int* vp = cv.vars + (L * cv.maxdeg) * cv.width + rs;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-            const int vj = (live && j < cv.maxdeg) ? __ldg(vp + j * cv.width) : -1;
-            v[b][j] = (vj >= 0 || !dummy_slots<D>()) ? vj : dummy;
-        }
-    }
-    int cnt = 0;
-#pragma unroll
-    for (int b = 0; b < kRowBatch; ++b) {
-        if (dummy_slots<D>() && rs0 + b * kWideThreads >= rows) continue;  // past the layer
-        unsigned par = 0;
-#pragma unroll
-        for (int j = 0; j < D; ++j)
-            if (dummy_slots<D>() ? j < cv.maxdeg : v[b][j] >= 0) par ^= (app.ld(v[b][j]) < 0.0f) ? 1u : 0u;
-        cnt += static_cast<int>(par);
-    }
-    return cnt;
-}
+constexpr int wide_threads() { return D <= 10 ? 1024 : 512; }
 
 }  // namespace
 
+// The next row's offsets and messages are loaded while the current one is updated, across the
+// layer barriers too: they do not depend on posteriors.  Slots below cv.wide_smem_slots hold
+// shared-memory posteriors in every row (columns ascend within a row, so for the accumulator
+// codes only the parity slots can lie beyond the split): only the others test.  Without
+// best-syndrome tracking only "zero syndrome or not" matters, so the check stops at the first
+// layer with an unsatisfied row.
+//
+// Measured on GB300, 608 codewords of (64800,32400) at 2 dB: 12.1 ms before (512 threads, a
+// branch per posterior access, variable indices slot by slot, (min1, min2, argmin) row
+// arithmetic, full syndrome: 78 instructions per edge and iteration), 6.95 ms now.
 template <int D>
-__global__ void __launch_bounds__(kWideThreads, 1)
-bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long long slice, int split,
-                       int track_best)
+__global__ void __launch_bounds__(wide_threads<D>(), 1)
+bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long long slice, int split, int track_best)
 {
-    extern __shared__ __align__(16) float s_app[];
-    __shared__ int s_red[kWideWarps];
+    constexpr int kThreads = wide_threads<D>();
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ int s_red[kThreads / 32];
     __shared__ int s_next, s_slot;
     const int tid = threadIdx.x;
     const int n = cv.n, n_pad = (n + 3) & ~3;
@@ -262,56 +184,114 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
     // empty edge slots of short rows: with split > n_pad it and every posterior are in shared
     // memory, else the slice starts with n_pad posteriors and the dummy (4 floats).
     const bool all_smem = split > n_pad;
-    const SplitApp app{s_app, g, split};
-    const int dummy = n_pad;
+    const SplitApp app{s_raw, reinterpret_cast<unsigned char*>(g), 4u * static_cast<unsigned>(split)};
     float* best = all_smem ? g : g + n_pad + 4;
     float* r1 = best + (track_best ? n_pad : 0);
     float* r2 = r1 + mp;
     unsigned* meta = reinterpret_cast<unsigned*>(r2 + mp);
+    const uint4* table = reinterpret_cast<const uint4*>(cv.wide_rows);
+    const int js = cv.wide_smem_slots;
 
+    auto value = [&](const WideRow<D>& row, int j) -> float {
+        return j < js ? reg::lds(s_raw, row.off(j)) : app.at(row.off(j));
+    };
+    auto update = [&](const WideRow<D>& in, int row) {
+        float q[D], m[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) q[j] = __fsub_rn(value(in, j), rebuild(in.m1, in.m2, in.meta, j));
+        reg::exclusive_min<D>(q, m);
+        // the compressed row: all magnitudes but at most one equal the smallest input's
+        const float least = fminf(fabsf(m[0]), fabsf(m[1]));
+        float most = least;
+        unsigned signs = 0u;
+        int idx = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) most = fmaxf(most, fabsf(m[j]));
+#pragma unroll
+        for (int j = D - 1; j >= 0; --j) {
+            signs = __funnelshift_l(__float_as_uint(m[j]), signs, 1);
+            idx = fabsf(m[j]) == most ? j : idx;
+        }
+        const float n1 = nms_mag(p.alpha, p.beta, least), n2 = nms_mag(p.alpha, p.beta, most);
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            // the message, signed: the scaled magnitude with the sign of m
+            const float mag = fabsf(m[j]) == most ? n2 : n1;
+            const float x = __fadd_rn(q[j], __uint_as_float(__float_as_uint(mag) ^ (__float_as_uint(m[j]) & 0x80000000u)));
+            if (j < js) reg::sts(s_raw, in.off(j), x);
+            else app.put(in.off(j), x);
+        }
+        r1[row] = n1;
+        r2[row] = n2;
+        meta[row] = signs | (static_cast<unsigned>(idx) << 27);
+    };
+    auto parity_of = [&](int row) -> unsigned {
+        WideRow<D> r;
+        r.load_offsets(table, row);
+        unsigned par = 0u;
+#pragma unroll
+        for (int j = 0; j < D; ++j) par ^= __float_as_uint(value(r, j));
+        return par >> 31;
+    };
+    // Syndrome weight; without tracking, any nonzero value when it is not zero.
     auto syndrome = [&]() -> int {
         int cnt = 0;
-        for (int L = 0; L < cv.num_layers; ++L) {
-            const int first = __ldg(cv.layer_start + L), rows = __ldg(cv.layer_start + L + 1) - first;
-            for (int rs0 = tid; rs0 < rows; rs0 += row_batch<D>() * kWideThreads)
-                cnt += wide_parity<D>(cv, L, rs0, rows, app, dummy);
+        if (track_best) {
+            for (int r = tid; r < mp; r += kThreads) cnt += static_cast<int>(parity_of(r));
+            return cta_sum<kThreads>(cnt, s_red);
         }
-        return cta_sum(cnt, s_red);
+        for (int L = 0; L < cv.num_layers; ++L) {
+            const int end = __ldg(cv.layer_start + L + 1);
+            for (int r = __ldg(cv.layer_start + L) + tid; r < end && cnt == 0; r += kThreads)
+                cnt += static_cast<int>(parity_of(r));
+            if (__syncthreads_or(cnt)) return 1;
+        }
+        return 0;
     };
 
-    if (tid == 0) app.st(dummy, __int_as_float(0x7f800000));  // +inf, before the first __syncthreads
+    if (tid == 0) app.put(4u * static_cast<unsigned>(n_pad), __int_as_float(0x7f800000));  // +inf, before the first __syncthreads
     for (int c = blockIdx.x; c < io.count; c = wide_next(io, &s_next)) {
         const float* src = io.llr + static_cast<size_t>(c) * n;
-        for (int i = tid; i < n; i += kWideThreads) {
+        for (int i = tid; i < n; i += kThreads) {
             const float v = __ldcs(src + i);
-            app.st(i, v);
+            app.put(4u * static_cast<unsigned>(i), reg::canonical(v));
             if (track_best) best[i] = v;
         }
-        for (int r = tid; r < mp; r += kWideThreads) {
-            r1[r] = 0.0f;
-            r2[r] = 0.0f;
-            meta[r] = 0u;
-        }
         __syncthreads();
-        int best_w = syndrome();
+        int best_w = track_best ? syndrome() : 1;
         int iter = 0, w = 0;
+        WideRow<D> next;
+        if (tid < __ldg(cv.layer_start + 1)) next.load(table, tid, true, r1, r2, meta);
         for (;;) {
+            int first = 0, rows = __ldg(cv.layer_start + 1);
             for (int L = 0; L < cv.num_layers; ++L) {
-                const int first = __ldg(cv.layer_start + L), rows = __ldg(cv.layer_start + L + 1) - first;
-                for (int rs0 = tid; rs0 < rows; rs0 += row_batch<D>() * kWideThreads)
-                    wide_rows<D>(cv, p, L, rs0, rows, first, app, dummy, r1, r2, meta);
+                const bool last = L + 1 == cv.num_layers;
+                const int after = last ? 0 : first + rows;  // first row of the layer that comes next
+                const int after_rows = __ldg(cv.layer_start + (last ? 1 : L + 2)) - after;
+                const bool fresh = iter == 0, after_fresh = fresh && !last;
+                for (int rs = tid;; rs += kThreads) {
+                    const WideRow<D> row = next;
+                    if (rs + kThreads < rows) next.load(table, first + rs + kThreads, fresh, r1, r2, meta);
+                    else if (tid < after_rows) next.load(table, after + tid, after_fresh, r1, r2, meta);
+                    if (rs < rows) update(row, first + rs);
+                    if (rs + kThreads >= rows) break;
+                }
                 __syncthreads();
+                // a single layer: its rows' messages have only just been written
+                if (cv.num_layers == 1 && tid < rows) next.load(table, tid, false, r1, r2, meta);
+                first = after;
+                rows = after_rows;
             }
             w = syndrome();
             ++iter;
             if (track_best && (w < best_w || (w == 0 && best_w == 0))) {
-                for (int i = tid; i < n; i += kWideThreads) best[i] = app.ld(i);
+                for (int i = tid; i < n; i += kThreads) best[i] = app.ld(i);
                 __syncthreads();  // copied before the next layer rewrites the posteriors
             }
             if (w < best_w) best_w = w;
             if (w == 0 || iter >= p.max_iter) break;
         }
-        wide_finish(p, io, c, n, w, iter, app, best, track_best != 0, s_red, &s_slot);
+        wide_finish<kThreads>(p, io, c, n, w, iter, app, best, track_best != 0, s_red, &s_slot);
     }
 }
 
@@ -321,108 +301,152 @@ struct PlainApp {
     __device__ __forceinline__ float ld(int v) const { return a[v]; }
 };
 
-__global__ void __launch_bounds__(kWideThreads, 1)
-bp_flooding_wide_kernel(FloodView cv, BpParams p, BpIO io, float* scratch, long long slice, int app_smem,
-                        int track_best)
+// Flooding threads: one row (or column) per thread and pass.
+template <int D>
+constexpr int flood_threads() { return D <= 18 ? 1024 : 512; }
+
+// One float per edge, input and message of the edge in turn: the check phase replaces a row's
+// inputs by its messages, the variable phase a column's messages by its next inputs.  Edge j of
+// row r sits at cv.wide_stride * j + (r with its low 5 bits XORed by the next 5): rows are read
+// conflict-free and the strided rows of a quasi-cyclic column spread over the banks.  The array
+// lives in shared memory when it fits (kSmem: the N16200 codes), else in the CTA's slice.  The
+// syndrome reads the hard decisions packed 32 to a word; without best-syndrome tracking it stops
+// at the first unsatisfied rows.  kDamp: the inputs are kept beside, in the slice.
+//
+// Measured on GB300, 333 codewords of (16200,13320) at 4 dB: 2.8 ms before (per edge of each of
+// two column passes an edge, row and row-pointer lookup and a message rebuild, all from L2),
+// 0.38 ms now.
+template <int D, bool kDamp, bool kSmem>
+__global__ void __launch_bounds__(flood_threads<D>(), 1)
+bp_flooding_wide_kernel(FloodView cv, BpParams p, BpIO io, float* scratch, long long slice, int track_best)
 {
-    extern __shared__ __align__(16) float s_app[];
-    __shared__ int s_red[kWideWarps];
+    constexpr int kThreads = flood_threads<D>();
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ int s_red[kThreads / 32];
     __shared__ int s_next, s_slot;
     const int tid = threadIdx.x;
-    const int n = cv.n, m = cv.m, E = cv.edges;
-    const int n_pad = (n + 3) & ~3, m_pad = (m + 3) & ~3, e_pad = (E + 3) & ~3;
+    const int n = cv.n, m = cv.m, n_pad = (n + 3) & ~3, stride = cv.wide_stride;
+    const int words = (n + 31) / 32 + 1;  // the last one stays 0: missing edges of short rows read it
+    uint32_t* hard = reinterpret_cast<uint32_t*>(s_raw);
     float* g = scratch + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(slice);
-    float* llr = g;
-    float* best = llr + n_pad;
-    float* q = best + n_pad;
-    float* r1 = q + e_pad;
-    float* r2 = r1 + m_pad;
-    unsigned* meta = reinterpret_cast<unsigned*>(r2 + m_pad);
-    float* app = app_smem ? s_app : reinterpret_cast<float*>(meta + m_pad);
+    float* app = g;
+    float* best = app + n_pad;  // only when track_best
+    float* rest = best + (track_best ? n_pad : 0);
+    float* msg = kSmem ? reinterpret_cast<float*>(s_raw + ((static_cast<size_t>(words) * 4 + 15) & ~size_t(15))) : rest;
+    float* old = rest + (kSmem ? 0 : static_cast<size_t>(cv.maxdeg) * stride);  // only when kDamp
     const float keep = __fsub_rn(1.0f, p.damping);
+    const auto slot = [](int r) { return r ^ ((r >> 5) & 31); };
 
-    auto syndrome = [&](const float* x) {
+    auto parity_of = [&](int r) -> unsigned {
+        unsigned par = 0u;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            if (j < cv.maxdeg) {
+                const unsigned v = __ldg(cv.wide_vars + static_cast<size_t>(j) * m + r);
+                par ^= hard[v >> 5] >> (v & 31u);
+            }
+        }
+        return par & 1u;
+    };
+    // Syndrome weight; without tracking, any nonzero value when it is not zero.
+    auto syndrome = [&]() -> int {
         int cnt = 0;
-        for (int r = tid; r < m; r += kWideThreads) {
-            unsigned par = 0;
-            for (int e = __ldg(cv.row_ptr + r); e < __ldg(cv.row_ptr + r + 1); ++e)
-                par ^= (x[__ldg(cv.col_ind + e)] < 0.0f) ? 1u : 0u;
-            cnt += static_cast<int>(par);
+        if (track_best) {
+            for (int r = tid; r < m; r += kThreads) cnt += static_cast<int>(parity_of(r));
+            return cta_sum<kThreads>(cnt, s_red);
         }
-        return cta_sum(cnt, s_red);
-    };
-    auto edge_msg = [&](int e) {
-        const int r = __ldg(cv.edge_row + e);
-        return rebuild(r1[r], r2[r], meta[r], e - __ldg(cv.row_ptr + r));
+        for (int r0 = 0; r0 < m; r0 += kThreads) {
+            if (r0 + tid < m) cnt = static_cast<int>(parity_of(r0 + tid));
+            if (__syncthreads_or(cnt)) return 1;
+        }
+        return 0;
     };
 
+    if (tid == 0) hard[words - 1] = 0u;
     for (int c = blockIdx.x; c < io.count; c = wide_next(io, &s_next)) {
-        const float* src = io.llr + static_cast<size_t>(c) * n;
-        for (int i = tid; i < n; i += kWideThreads) {
-            const float v = __ldcs(src + i);
-            llr[i] = v;
-            app[i] = v;
-            if (track_best) best[i] = v;
+        const float* llr = io.llr + static_cast<size_t>(c) * n;
+        for (int v0 = 0; v0 < n; v0 += kThreads) {
+            const int v = v0 + tid;
+            const float x = v < n ? llr[v] : 0.0f;
+            if (v < n) {
+                if (track_best) best[v] = x;
+                const float q = reg::canonical(x);
+                const int e1 = __ldg(cv.col_ptr + v + 1);
+                for (int e = __ldg(cv.col_ptr + v); e < e1; ++e) {
+                    const int at = __ldg(cv.wide_pos + e);
+                    msg[at] = q;
+                    if constexpr (kDamp) old[at] = q;
+                }
+            }
+            const unsigned b = __ballot_sync(0xffffffffu, x < 0.0f);
+            if ((tid & 31) == 0 && v < n) hard[v >> 5] = b;
         }
         __syncthreads();
-        for (int e = tid; e < E; e += kWideThreads) q[e] = llr[__ldg(cv.col_ind + e)];
-        __syncthreads();
-        int best_w = syndrome(llr);
+        int best_w = track_best ? syndrome() : 1;
         int iter = 0, w = 0;
         for (;;) {
             // check nodes (L:3033-3060)
-            for (int r = tid; r < m; r += kWideThreads) {
-                const int e0 = __ldg(cv.row_ptr + r), e1 = __ldg(cv.row_ptr + r + 1);
-                float m1 = FLT_MAX, m2 = FLT_MAX;
-                int idx = 0;
-                unsigned neg = 0;
-                for (int e = e0; e < e1; ++e) {
-                    const float v = q[e];
-                    neg |= (v < 0.0f) ? (1u << (e - e0)) : 0u;
-                    const float a = fabsf(v);
-                    if (a < m1) {
-                        m2 = m1;
-                        m1 = a;
-                        idx = e - e0;
-                    } else if (a < m2) {
-                        m2 = a;
+            for (int r = tid; r < m; r += kThreads) {
+                const int deg = __ldg(cv.row_ptr + r + 1) - __ldg(cv.row_ptr + r), base = slot(r);
+                float q[D], out[D];
+#pragma unroll
+                for (int j = 0; j < D; ++j) q[j] = j < deg ? msg[j * stride + base] : __int_as_float(0x7f800000);
+                reg::row_messages<D>(q, p.alpha, p.beta, out);
+#pragma unroll
+                for (int j = 0; j < D; ++j)
+                    if (j < deg) msg[j * stride + base] = out[j];
+            }
+            __syncthreads();
+            // variable nodes (L:3062-3069): llr + sum of messages in row order; the next inputs
+            // (L:3076-3081), optional damping
+            for (int v0 = 0; v0 < n; v0 += kThreads) {
+                const int v = v0 + tid;
+                float acc = 0.0f;
+                if (v < n) {
+                    acc = reg::canonical(__ldg(llr + v));
+                    const int e0 = __ldg(cv.col_ptr + v), e1 = __ldg(cv.col_ptr + v + 1);
+                    int at[4];  // the first edges' positions (and most columns' all)
+                    float r[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        at[i] = e0 + i < e1 ? __ldg(cv.wide_pos + e0 + i) : -1;
+                        r[i] = at[i] >= 0 ? msg[at[i]] : 0.0f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (at[i] >= 0) acc = __fadd_rn(acc, r[i]);
+                    for (int e = e0 + 4; e < e1; ++e) acc = __fadd_rn(acc, msg[__ldg(cv.wide_pos + e)]);
+                    app[v] = acc;
+                    auto next = [&](int pos, float message) {
+                        const float fresh = __fsub_rn(acc, message);
+                        if constexpr (kDamp) {
+                            const float q = reg::canonical(__fadd_rn(__fmul_rn(keep, fresh), __fmul_rn(p.damping, old[pos])));
+                            msg[pos] = q;
+                            old[pos] = q;
+                        } else {
+                            msg[pos] = fresh;
+                        }
+                    };
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (at[i] >= 0) next(at[i], r[i]);
+                    for (int e = e0 + 4; e < e1; ++e) {
+                        const int pos = __ldg(cv.wide_pos + e);
+                        next(pos, msg[pos]);
                     }
                 }
-                const unsigned tot = static_cast<unsigned>(__popc(neg)) & 1u;
-                unsigned nm = static_cast<unsigned>(idx) << 27;
-                for (int j = 0; j < e1 - e0; ++j) nm |= (tot ^ ((neg >> j) & 1u)) << j;
-                r1[r] = nms_mag(p.alpha, p.beta, m1);
-                r2[r] = nms_mag(p.alpha, p.beta, m2);
-                meta[r] = nm;
+                const unsigned b = __ballot_sync(0xffffffffu, acc < 0.0f);
+                if ((tid & 31) == 0 && v < n) hard[v >> 5] = b;
             }
             __syncthreads();
-            // variable nodes (L:3062-3069): llr + sum of messages in row order
-            for (int v = tid; v < n; v += kWideThreads) {
-                float acc = llr[v];
-                for (int j = __ldg(cv.col_ptr + v); j < __ldg(cv.col_ptr + v + 1); ++j)
-                    acc = __fadd_rn(acc, edge_msg(__ldg(cv.col_edge + j)));
-                app[v] = acc;
-            }
-            __syncthreads();
-            w = syndrome(app);
+            w = syndrome();
             ++iter;
-            if (track_best && (w < best_w || (w == 0 && best_w == 0))) {
-                for (int i = tid; i < n; i += kWideThreads) best[i] = app[i];
-            }
+            if (track_best && (w < best_w || (w == 0 && best_w == 0)))
+                for (int i = tid; i < n; i += kThreads) best[i] = app[i];
             if (w < best_w) best_w = w;
             if (w == 0 || iter >= p.max_iter) break;
-            // next variable-to-check messages (L:3076-3081), optional damping
-            for (int v = tid; v < n; v += kWideThreads) {
-                for (int j = __ldg(cv.col_ptr + v); j < __ldg(cv.col_ptr + v + 1); ++j) {
-                    const int e = __ldg(cv.col_edge + j);
-                    const float fresh = __fsub_rn(app[v], edge_msg(e));
-                    q[e] = (p.damping == 0.0f) ? fresh
-                                                : __fadd_rn(__fmul_rn(keep, fresh), __fmul_rn(p.damping, q[e]));
-                }
-            }
-            __syncthreads();
         }
-        wide_finish(p, io, c, n, w, iter, PlainApp{app}, best, track_best != 0, s_red, &s_slot);
+        wide_finish<kThreads>(p, io, c, n, w, iter, PlainApp{app}, best, track_best != 0, s_red, &s_slot);
     }
 }
 
@@ -445,24 +469,30 @@ int wide_grid(int count, int per_sm, size_t slice_bytes)
     return std::max(1, std::min(ctas, count));
 }
 
-template <class K, class Launch>
-void launch_wide(K kernel, size_t app_bytes, long long slice_floats, int count, cudaStream_t st, Launch&& go)
+// Shared memory of the flooding kernel: the packed hard decisions, and the messages when they fit.
+size_t flood_hard_bytes(const FloodView& cv) { return (static_cast<size_t>((cv.n + 31) / 32 + 1) * 4 + 15) & ~size_t(15); }
+size_t flood_msg_bytes(const FloodView& cv) { return static_cast<size_t>(cv.maxdeg) * cv.wide_stride * sizeof(float); }
+
+template <int D, bool kDamp, bool kSmem>
+void launch_flooding_wide_t(const FloodView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
 {
-    // posteriors in shared memory when they fit beside the static arrays
-    const bool app_smem = app_bytes <= 200 * 1024;
-    const size_t smem = app_smem ? app_bytes : 0;
+    const auto kernel = bp_flooding_wide_kernel<D, kDamp, kSmem>;
+    const size_t smem = flood_hard_bytes(cv) + (kSmem ? flood_msg_bytes(cv) : 0);
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp wide)");
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWideThreads, smem) != cudaSuccess || per_sm <= 0)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, flood_threads<D>(), smem) != cudaSuccess || per_sm <= 0)
         per_sm = 1;
-    const size_t slice_bytes = static_cast<size_t>(slice_floats) * sizeof(float);
-    const int ctas = wide_grid(count, per_sm, slice_bytes);
+    const long long n_pad = (cv.n + 3) & ~3, edges = static_cast<long long>(cv.maxdeg) * cv.wide_stride;
+    long long slice = n_pad + (track_best ? n_pad : 0) + (kSmem ? 0 : edges) + (kDamp ? edges : 0);
+    slice = (slice + 31) & ~31LL;
+    const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
+    const int ctas = wide_grid(io.count, per_sm, slice_bytes);
     int device = 0;
     check_cuda(cudaGetDevice(&device), "cudaGetDevice");
     void* scratch = nullptr;
     check_cuda(cudaMallocFromPoolAsync(&scratch, std::max<size_t>(slice_bytes * ctas, 16), scratch_pool(device), st),
                "cudaMallocFromPoolAsync(bp wide)");
-    go(ctas, smem, static_cast<float*>(scratch), app_smem ? 1 : 0);
+    kernel<<<ctas, flood_threads<D>(), smem, st>>>(cv, p, io, static_cast<float*>(scratch), slice, track_best ? 1 : 0);
     const cudaError_t err = cudaGetLastError();
     const cudaError_t ferr = cudaFreeAsync(scratch, st);
     check_cuda(err, "bp wide kernel launch");
@@ -470,24 +500,33 @@ void launch_wide(K kernel, size_t app_bytes, long long slice_floats, int count, 
 }
 
 template <int D>
+void launch_flooding_wide_d(const FloodView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
+{
+    // 1 KB of the 227 KB stays for the kernel's static arrays
+    const bool fits = flood_hard_bytes(cv) + flood_msg_bytes(cv) <= 226 * 1024;
+    if (p.damping == 0.0f) {
+        if (fits) launch_flooding_wide_t<D, false, true>(cv, p, io, track_best, st);
+        else launch_flooding_wide_t<D, false, false>(cv, p, io, track_best, st);
+    } else {
+        if (fits) launch_flooding_wide_t<D, true, true>(cv, p, io, track_best, st);
+        else launch_flooding_wide_t<D, true, false>(cv, p, io, track_best, st);
+    }
+}
+
+template <int D>
 void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
 {
     const long long n_pad = (cv.n + 3) & ~3;
     const long long mp = cv.m;
-    // the posteriors and the dummy posterior (index n_pad, padded to 4 floats)
-    const size_t app_bytes = static_cast<size_t>(n_pad + 4) * sizeof(float);
-    // posteriors in shared memory: all of them up to 200 KB, else the first 56,320 (220 KB;
-    // variables beyond and the dummy stay in the slice)
-    constexpr size_t kSmemApp = 200 * 1024, kSplitApp = 220 * 1024;
-    const bool all_smem = app_bytes <= kSmemApp;
-    const int split = all_smem ? static_cast<int>(n_pad + 4) : static_cast<int>(kSplitApp / sizeof(float));
-    const size_t smem = all_smem ? app_bytes : kSplitApp;
+    const int split = wide_split(cv.n);
+    const bool all_smem = split > n_pad;
+    const size_t smem = static_cast<size_t>(split) * sizeof(float);
     long long slice = (all_smem ? 0 : n_pad + 4) + (track_best ? n_pad : 0) + 3 * mp;
     slice = (slice + 31) & ~31LL;  // 128-byte aligned slices
     const auto kernel = bp_layered_wide_kernel<D>;
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp wide)");
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWideThreads, smem) != cudaSuccess || per_sm <= 0)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, wide_threads<D>(), smem) != cudaSuccess || per_sm <= 0)
         per_sm = 1;
     const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
     const int ctas = wide_grid(io.count, per_sm, slice_bytes);
@@ -496,7 +535,7 @@ void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO&
     void* scratch = nullptr;
     check_cuda(cudaMallocFromPoolAsync(&scratch, std::max<size_t>(slice_bytes * ctas, 16), scratch_pool(device), st),
                "cudaMallocFromPoolAsync(bp wide)");
-    kernel<<<ctas, kWideThreads, smem, st>>>(cv, p, io, static_cast<float*>(scratch), slice, split, track_best ? 1 : 0);
+    kernel<<<ctas, wide_threads<D>(), smem, st>>>(cv, p, io, static_cast<float*>(scratch), slice, split, track_best ? 1 : 0);
     const cudaError_t err = cudaGetLastError();
     const cudaError_t ferr = cudaFreeAsync(scratch, st);
     check_cuda(err, "bp wide kernel launch");
@@ -504,6 +543,22 @@ void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO&
 }
 
 }  // namespace
+
+// Posteriors in shared memory (the dummy posterior, padded to 4 floats, after the last): all of
+// them up to 200 KB, else the first 56,320 (220 KB; variables beyond and the dummy in the slice).
+int wide_split(int n)
+{
+    const int n_pad = (n + 3) & ~3;
+    return (n_pad + 4) * sizeof(float) <= 200 * 1024 ? n_pad + 4 : static_cast<int>(220 * 1024 / sizeof(float));
+}
+
+// Edge slots of a row in the wide kernel: the closest compiled degree.
+int wide_slots(int maxdeg)
+{
+    for (int d : {4, 6, 7, 10, 14, 18, 27})
+        if (maxdeg <= d) return d;
+    return 0;
+}
 
 bool layered_needs_wide(const LayeredView& cv, bool track_best)
 {
@@ -518,12 +573,15 @@ void launch_bp_layered_wide(const LayeredView& cv, const BpParams& p, const BpIO
     if (io.count <= 0) return;
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
     check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
-    if (cv.maxdeg <= 6) launch_layered_wide_t<6>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 8) launch_layered_wide_t<8>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 10) launch_layered_wide_t<10>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 12) launch_layered_wide_t<12>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 16) launch_layered_wide_t<16>(cv, p, io, track_best, st);
-    else launch_layered_wide_t<27>(cv, p, io, track_best, st);
+    switch (wide_slots(cv.maxdeg)) {
+        case 4: launch_layered_wide_t<4>(cv, p, io, track_best, st); break;
+        case 6: launch_layered_wide_t<6>(cv, p, io, track_best, st); break;
+        case 7: launch_layered_wide_t<7>(cv, p, io, track_best, st); break;
+        case 10: launch_layered_wide_t<10>(cv, p, io, track_best, st); break;
+        case 14: launch_layered_wide_t<14>(cv, p, io, track_best, st); break;
+        case 18: launch_layered_wide_t<18>(cv, p, io, track_best, st); break;
+        default: launch_layered_wide_t<27>(cv, p, io, track_best, st); break;
+    }
 }
 
 void launch_bp_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO& io, cudaStream_t st)
@@ -532,16 +590,10 @@ void launch_bp_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO&
     if (cv.maxdeg > 27) throw InvalidArgument("flooding schedule supports row degree <= 27");
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
     check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
-    const long long n_pad = (cv.n + 3) & ~3, m_pad = (cv.m + 3) & ~3, e_pad = (cv.edges + 3) & ~3;
-    const size_t app_bytes = static_cast<size_t>(n_pad) * sizeof(float);
-    const bool app_smem = app_bytes <= 200 * 1024;
-    long long slice = 2 * n_pad + e_pad + 3 * m_pad + (app_smem ? 0 : n_pad);
-    slice = (slice + 31) & ~31LL;
-    launch_wide(bp_flooding_wide_kernel, app_bytes, slice, io.count, st,
-                [&](int ctas, size_t smem, float* scratch, int in_smem) {
-                    bp_flooding_wide_kernel<<<ctas, kWideThreads, smem, st>>>(cv, p, io, scratch, slice, in_smem,
-                                                                              track_best ? 1 : 0);
-                });
+    if (cv.maxdeg <= 6) launch_flooding_wide_d<6>(cv, p, io, track_best, st);
+    else if (cv.maxdeg <= 10) launch_flooding_wide_d<10>(cv, p, io, track_best, st);
+    else if (cv.maxdeg <= 18) launch_flooding_wide_d<18>(cv, p, io, track_best, st);
+    else launch_flooding_wide_d<27>(cv, p, io, track_best, st);
 }
 
 }  // namespace sicc

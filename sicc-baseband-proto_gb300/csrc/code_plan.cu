@@ -273,6 +273,21 @@ void DeviceCode::build_layered()
     lv_.m = m_;
     lv_.layer_start = device_upload(starts, owned_);
     reg_plan(lv_, maxw, *std::min_element(sizes.begin(), sizes.end()), layered_group_ > 0 ? group : 0);
+    if (layered_needs_wide(lv_, false) || layered_needs_wide(lv_, true)) {
+        const int slots = wide_slots(maxdeg), entries = (slots + 3) & ~3, split = wide_split(n_);
+        std::vector<uint32_t> off(static_cast<size_t>(m_) * entries, 4u * static_cast<uint32_t>((n_ + 3) & ~3));
+        int below = slots;
+        for (int i = 0; i < m_; ++i) {
+            const int r = row_order_[i], b = row_ptr_[r], deg = row_ptr_[r + 1] - b;
+            for (int j = 0; j < slots; ++j) {
+                uint32_t& o = off[static_cast<size_t>(i) * entries + j];
+                if (j < deg) o = 4u * static_cast<uint32_t>(col_ind_[b + j]);
+                if (o >= 4u * static_cast<uint32_t>(split)) below = std::min(below, j);
+            }
+        }
+        lv_.wide_rows = device_upload(off, owned_);
+        lv_.wide_smem_slots = below;
+    }
 }
 
 void DeviceCode::build_flood()
@@ -299,6 +314,21 @@ void DeviceCode::build_flood()
     fv_.col_ptr = device_upload(col_ptr, owned_);
     fv_.col_edge = device_upload(col_edge, owned_);
     fv_.edge_row = device_upload(edge_row, owned_);
+    if (flooding_needs_wide(fv_)) {
+        const int stride = (m_ + 31) & ~31;
+        std::vector<int> pos(edges_);
+        std::vector<uint32_t> vars(static_cast<size_t>(maxdeg) * m_, static_cast<uint32_t>((n_ + 31) & ~31));
+        for (int i = 0; i < edges_; ++i) {
+            const int e = col_edge[i], r = edge_row[e];
+            pos[i] = stride * (e - row_ptr_[r]) + (r ^ ((r >> 5) & 31));
+        }
+        for (int r = 0; r < m_; ++r)
+            for (int e = row_ptr_[r], j = 0; e < row_ptr_[r + 1]; ++e, ++j)
+                vars[static_cast<size_t>(j) * m_ + r] = static_cast<uint32_t>(col_ind_[e]);
+        fv_.wide_pos = device_upload(pos, owned_);
+        fv_.wide_vars = device_upload(vars, owned_);
+        fv_.wide_stride = stride;
+    }
     row_order_.resize(m_);
     for (int r = 0; r < m_; ++r) row_order_[r] = r;
 }

@@ -60,6 +60,11 @@ struct LayeredView {
     int reg_group;      // lanes per codeword of the register-resident kernels (<= 128), 0: not for this code
     int reg_rpl;        // their rows per lane in a layer
     int reg_plain;      // 1: every layer has exactly reg_group rows
+    // long codes (bp_wide.cu): per row in layer order, the byte offsets (4 x variable) of its
+    // posteriors, padded with the dummy's to a multiple of 4 entries; and the slots that lie below
+    // the shared-memory split in every row
+    const uint32_t* wide_rows;
+    int wide_smem_slots;
 };
 
 // Flooding schedule: rows in CSR order plus the column view used for the
@@ -71,6 +76,12 @@ struct FloodView {
     const int* col_ptr;   // [n+1]
     const int* col_edge;  // [E] edge id
     const int* edge_row;  // [E] row of the edge
+    // long codes (bp_wide.cu): position in the message array of each edge in column order, the
+    // row stride of that array, and the rows' variables slot by slot (missing edges: the first
+    // variable index past the packed hard decisions)
+    const int* wide_pos;        // [E]
+    const uint32_t* wide_vars;  // [maxdeg][m]
+    int wide_stride;
 };
 
 struct BpParams {
