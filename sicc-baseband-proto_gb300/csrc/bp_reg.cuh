@@ -58,6 +58,13 @@ __device__ __forceinline__ float minx(float a, float b)
     return d;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c)  // the largest magnitude
+{
+    float d;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // |m[j]| = min(FLT_MAX, min over i != j of |a[i]|), sign = product of the other
 // signs: the magnitude (min1, min2, argmin) tracking from FLT_MAX gives edge j,
 // whichever of equal minima it names the argmin.

@@ -128,8 +128,7 @@ template <int D>
 struct WideRow {
     static constexpr int kQuads = (D + 3) / 4;
     uint4 o[kQuads];
-    float m1, m2;
-    unsigned meta;
+    uint4 state;  // messages: min1, min2 (scaled), signs and argmin
 
     __device__ __forceinline__ unsigned off(int j) const
     {
@@ -141,20 +140,19 @@ struct WideRow {
 #pragma unroll
         for (int i = 0; i < kQuads; ++i) o[i] = __ldg(table + static_cast<size_t>(row) * kQuads + i);
     }
-    __device__ __forceinline__ void load(const uint4* __restrict__ table, int row, bool fresh, const float* r1,
-                                         const float* r2, const unsigned* mt)
+    __device__ __forceinline__ void load(const uint4* __restrict__ table, int row, bool fresh, const uint4* states)
     {
         load_offsets(table, row);
-        m1 = fresh ? 0.0f : r1[row];  // a codeword's first iteration: no messages yet
-        m2 = fresh ? 0.0f : r2[row];
-        meta = fresh ? 0u : mt[row];
+        state = make_uint4(0u, 0u, 0u, 0u);  // a codeword's first iteration: no messages yet
+        if (!fresh) state = states[row];
     }
 };
 
-// Threads: row degrees up to 10 leave room for 1,024 threads (64 registers), which hide the L2
-// latency of tables and messages; wider rows take 512.
+// Threads: as many as the rows' registers allow without spills in the row loop (they hide the L2
+// latency of tables and messages).  608 codewords of (64800,32400), D = 7: 768 threads 6.41 ms,
+// 1,024 (64 registers, spilling) 6.83; 600 of (16200,3240), D = 4: 2.58 and 2.35.
 template <int D>
-constexpr int wide_threads() { return D <= 10 ? 1024 : 512; }
+constexpr int wide_threads() { return D <= 4 ? 1024 : D <= 10 ? 768 : 512; }
 
 }  // namespace
 
@@ -167,7 +165,7 @@ constexpr int wide_threads() { return D <= 10 ? 1024 : 512; }
 //
 // Measured on GB300, 608 codewords of (64800,32400) at 2 dB: 12.1 ms before (512 threads, a
 // branch per posterior access, variable indices slot by slot, (min1, min2, argmin) row
-// arithmetic, full syndrome: 78 instructions per edge and iteration), 6.95 ms now.
+// arithmetic, full syndrome: 78 instructions per edge and iteration), 6.41 ms now.
 template <int D>
 __global__ void __launch_bounds__(wide_threads<D>(), 1)
 bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long long slice, int split, int track_best)
@@ -186,9 +184,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
     const bool all_smem = split > n_pad;
     const SplitApp app{s_raw, reinterpret_cast<unsigned char*>(g), 4u * static_cast<unsigned>(split)};
     float* best = all_smem ? g : g + n_pad + 4;
-    float* r1 = best + (track_best ? n_pad : 0);
-    float* r2 = r1 + mp;
-    unsigned* meta = reinterpret_cast<unsigned*>(r2 + mp);
+    uint4* states = reinterpret_cast<uint4*>(best + (track_best ? n_pad : 0));
     const uint4* table = reinterpret_cast<const uint4*>(cv.wide_rows);
     const int js = cv.wide_smem_slots;
 
@@ -197,8 +193,9 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
     };
     auto update = [&](const WideRow<D>& in, int row) {
         float q[D], m[D];
+        const float o1 = __uint_as_float(in.state.x), o2 = __uint_as_float(in.state.y);
 #pragma unroll
-        for (int j = 0; j < D; ++j) q[j] = __fsub_rn(value(in, j), rebuild(in.m1, in.m2, in.meta, j));
+        for (int j = 0; j < D; ++j) q[j] = __fsub_rn(value(in, j), rebuild(o1, o2, in.state.z, j));
         reg::exclusive_min<D>(q, m);
         // the compressed row: all magnitudes but at most one equal the smallest input's
         const float least = fminf(fabsf(m[0]), fabsf(m[1]));
@@ -206,7 +203,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
         unsigned signs = 0u;
         int idx = 0;
 #pragma unroll
-        for (int j = 0; j < D; ++j) most = fmaxf(most, fabsf(m[j]));
+        for (int j = 0; j < D; j += 2) most = reg::max3(most, m[j], m[j + 1 < D ? j + 1 : 0]);
 #pragma unroll
         for (int j = D - 1; j >= 0; --j) {
             signs = __funnelshift_l(__float_as_uint(m[j]), signs, 1);
@@ -221,9 +218,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
             if (j < js) reg::sts(s_raw, in.off(j), x);
             else app.put(in.off(j), x);
         }
-        r1[row] = n1;
-        r2[row] = n2;
-        meta[row] = signs | (static_cast<unsigned>(idx) << 27);
+        states[row] = make_uint4(__float_as_uint(n1), __float_as_uint(n2), signs | (static_cast<unsigned>(idx) << 27), 0u);
     };
     auto parity_of = [&](int row) -> unsigned {
         WideRow<D> r;
@@ -261,7 +256,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
         int best_w = track_best ? syndrome() : 1;
         int iter = 0, w = 0;
         WideRow<D> next;
-        if (tid < __ldg(cv.layer_start + 1)) next.load(table, tid, true, r1, r2, meta);
+        if (tid < __ldg(cv.layer_start + 1)) next.load(table, tid, true, states);
         for (;;) {
             int first = 0, rows = __ldg(cv.layer_start + 1);
             for (int L = 0; L < cv.num_layers; ++L) {
@@ -271,14 +266,14 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
                 const bool fresh = iter == 0, after_fresh = fresh && !last;
                 for (int rs = tid;; rs += kThreads) {
                     const WideRow<D> row = next;
-                    if (rs + kThreads < rows) next.load(table, first + rs + kThreads, fresh, r1, r2, meta);
-                    else if (tid < after_rows) next.load(table, after + tid, after_fresh, r1, r2, meta);
+                    if (rs + kThreads < rows) next.load(table, first + rs + kThreads, fresh, states);
+                    else if (tid < after_rows) next.load(table, after + tid, after_fresh, states);
                     if (rs < rows) update(row, first + rs);
                     if (rs + kThreads >= rows) break;
                 }
                 __syncthreads();
                 // a single layer: its rows' messages have only just been written
-                if (cv.num_layers == 1 && tid < rows) next.load(table, tid, false, r1, r2, meta);
+                if (cv.num_layers == 1 && tid < rows) next.load(table, tid, false, states);
                 first = after;
                 rows = after_rows;
             }
@@ -521,7 +516,7 @@ void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO&
     const int split = wide_split(cv.n);
     const bool all_smem = split > n_pad;
     const size_t smem = static_cast<size_t>(split) * sizeof(float);
-    long long slice = (all_smem ? 0 : n_pad + 4) + (track_best ? n_pad : 0) + 3 * mp;
+    long long slice = (all_smem ? 0 : n_pad + 4) + (track_best ? n_pad : 0) + 4 * mp;
     slice = (slice + 31) & ~31LL;  // 128-byte aligned slices
     const auto kernel = bp_layered_wide_kernel<D>;
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp wide)");
