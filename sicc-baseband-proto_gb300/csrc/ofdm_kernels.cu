@@ -7,11 +7,20 @@
 // the earliest candidate over the threshold (or the global maximum), then a
 // full-preamble cross-correlation refinement within +-radius, then the CFO
 // arg(sum conj(x[s+i]) x[s+i+L]) * fs / (2 pi L).  Candidates are scanned in
-// passes of 256 x 17 from a shared-memory copy of the samples: each pass
-// computes the window sums at 256 chunk starts warp-cooperatively and slides
-// them 17 candidates per thread (the odd chunk keeps shared-memory reads on
-// distinct banks).  Every pass publishes its result to global scratch and the
-// last pass of a frame to finish resolves the frame.
+// passes of 256 x 17 from a shared-memory copy of the samples (the odd chunk
+// keeps shared-memory reads on distinct banks):
+//   * the products of 17 consecutive samples are summed once, a window sum at a
+//     chunk start is the sum of L / 17 such blocks and the last samples, and a
+//     thread slides it over its 17 candidates (30 block sums instead of 512
+//     products per chunk at L = 512);
+//   * the fine metric is computed for four neighbouring positions at a time (one
+//     read of the preamble for four), in increasing order, and only as far as
+//     the earliest position over the threshold decides the search.
+// Every pass publishes its result to global scratch and the last pass of a
+// frame to finish resolves the frame.  Measured on GB300, 256 frames of 16,888
+// samples (1,024-sample preamble, 6-tap fading): 243 us with a product per
+// sample and chunk and every position's fine metric, 77 us now; it stays
+// bound by instruction issue (the fine correlations).
 //
 // demod_kernel (grid = frames x data-symbol groups) fuses the demodulator of
 // gpu_ofdm_pipeline.cu:566-672 / uhd_ldpc_ofdm_link.cpp:5350-5521: CFO
@@ -94,27 +103,67 @@ __device__ __forceinline__ float fine_metric(const float2* __restrict__ x, const
     return (cr * cr + ci * ci) / fmaxf(eng * pre_energy, 1e-18f);
 }
 
+// fine_metric of the positions dd .. dd + 3, all inside the shared window (at win + at): the same
+// sums, with one read of the preamble for the four.
+__device__ __forceinline__ void fine_metric4(const float2* win, int at, const float2* __restrict__ preamble, int pre,
+                                             float pre_energy, int lane, float (&out)[4])
+{
+    float cr[4] = {0.f, 0.f, 0.f, 0.f}, ci[4] = {0.f, 0.f, 0.f, 0.f}, eng[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int i = lane; i < pre; i += 32) {
+        const float2 q = __ldg(preamble + i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 y = win[at + i + k];
+            cr[k] = fmaf(y.x, q.x, fmaf(y.y, q.y, cr[k]));
+            ci[k] = fmaf(y.y, q.x, fmaf(-y.x, q.y, ci[k]));
+            eng[k] = fmaf(y.x, y.x, fmaf(y.y, y.y, eng[k]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float r = warp_sum(cr[k]), j = warp_sum(ci[k]), e = warp_sum(eng[k]);
+        out[k] = (r * r + j * j) / fmaxf(e * pre_energy, 1e-18f);
+    }
+}
+
 // Shared-memory working set of a frame search by one CTA.
 struct SyncShared {
     float2* win;      // [kSyncPass + pre_len] the pass's samples (rounded up to an even count: the
-                      // float4 chunk sums after the metric stay 16-byte aligned)
+                      // float4 block sums after the metric stay 16-byte aligned)
     float* metric;    // [kSyncPass] coarse metric
-    float4* chunk;    // [kSyncThreads] window sums at chunk starts: P.re, P.im, E1, E2
-    float* memo;      // [kSyncPass + 2 * kMaxRadius] fine metric around crossings
+    float4* block;    // [kSyncThreads + L / kSyncChunk] sums over 17 samples: P.re, P.im, E1, E2;
+                      // before the metric is complete, in memo's place
+    float* memo;      // [kSyncPass + 2 * radius] fine metric around crossings
+    uint16_t* list;   // [memo / 4] groups of four memo positions to evaluate, in increasing order
     float* red;       // [4][kSyncThreads / 32] reductions
     float* rmetric;   // [kMaxRefine] mode-1 refinement
-    int* s_key;       // [kSyncThreads / 32]
+    int* s_key;       // [kSyncThreads / 32 + 2]
     PassResult* s_res;
 };
 
-__device__ __forceinline__ SyncShared sync_shared(unsigned char* smem_raw, int pre_len, float* red, float* rmetric,
-                                                  int* s_key, PassResult* s_res)
+__host__ __device__ inline int sync_memo(int radius) { return (kSyncPass + 2 * radius + 3) & ~3; }
+__host__ __device__ inline size_t sync_memo_bytes(int pre_len, int radius)
+{  // the fine metrics, or the block sums before them
+    const size_t memo = static_cast<size_t>(sync_memo(radius)) * sizeof(float);
+    const size_t block = static_cast<size_t>(kSyncThreads + pre_len / 2 / kSyncChunk) * sizeof(float4);
+    return memo > block ? memo : block;
+}
+__host__ __device__ inline size_t sync_smem(int pre_len, int radius)
+{
+    return static_cast<size_t>((kSyncPass + pre_len + 1) & ~1) * sizeof(float2) + kSyncPass * sizeof(float) +
+           sync_memo_bytes(pre_len, radius) + static_cast<size_t>(sync_memo(radius) / 4) * sizeof(uint16_t);
+}
+
+__device__ __forceinline__ SyncShared sync_shared(unsigned char* smem_raw, int pre_len, int radius, float* red,
+                                                  float* rmetric, int* s_key, PassResult* s_res)
 {
     SyncShared sh;
     sh.win = reinterpret_cast<float2*>(smem_raw);
     sh.metric = reinterpret_cast<float*>(sh.win + ((kSyncPass + pre_len + 1) & ~1));
-    sh.chunk = reinterpret_cast<float4*>(sh.metric + kSyncPass);
-    sh.memo = reinterpret_cast<float*>(sh.chunk + kSyncThreads);
+    sh.block = reinterpret_cast<float4*>(sh.metric + kSyncPass);
+    sh.memo = sh.metric + kSyncPass;
+    sh.list = reinterpret_cast<uint16_t*>(reinterpret_cast<unsigned char*>(sh.memo) + sync_memo_bytes(pre_len, radius));
     sh.red = red;
     sh.rmetric = rmetric;
     sh.s_key = s_key;
@@ -137,30 +186,40 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
     __syncthreads();
     // chunks holding candidates below the limit (the rest only hold -1)
     const int nchunks = min(kSyncThreads, (limit - base + kSyncChunk - 1) / kSyncChunk);
-    // window sums at chunk starts, one warp per chunk
-    for (int t = warp; t < nchunks; t += kSyncThreads / 32) {
-        const int d0 = t * kSyncChunk;
-        float pr = 0.f, pi = 0.f, e1 = 0.f, e2 = 0.f;
-        for (int i = lane; i < L; i += 32) {
-            const float2 a = sh.win[d0 + i], b = sh.win[d0 + i + L];
-            const float2 c = cmulconj(b, a);  // conj(a) * b
-            pr += c.x;
-            pi += c.y;
-            e1 += cnorm(a);
-            e2 += cnorm(b);
+    const int nb = L / kSyncChunk;
+    for (int t = tid; t < nchunks + nb; t += kSyncThreads) {
+        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = t * kSyncChunk; i < (t + 1) * kSyncChunk; ++i) {
+            const float2 u = sh.win[i], v = sh.win[i + L];
+            const float2 c = cmulconj(v, u);  // conj(u) * v
+            w.x += c.x;
+            w.y += c.y;
+            w.z += cnorm(u);
+            w.w += cnorm(v);
         }
-        pr = warp_sum(pr);
-        pi = warp_sum(pi);
-        e1 = warp_sum(e1);
-        e2 = warp_sum(e2);
-        if (lane == 0) sh.chunk[t] = make_float4(pr, pi, e1, e2);
+        sh.block[t] = w;
     }
     __syncthreads();
     if (tid >= nchunks) {
         for (int c = 0; c < kSyncChunk; ++c) sh.metric[tid * kSyncChunk + c] = -1.0f;
     } else {
-        float4 w = sh.chunk[tid];
         const int d0 = tid * kSyncChunk;
+        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = d0 + nb * kSyncChunk; i < d0 + L; ++i) {  // the window's last L mod 17 samples
+            const float2 u = sh.win[i], v = sh.win[i + L];
+            const float2 c = cmulconj(v, u);
+            w.x += c.x;
+            w.y += c.y;
+            w.z += cnorm(u);
+            w.w += cnorm(v);
+        }
+        for (int b = nb - 1; b >= 0; --b) {
+            const float4 v = sh.block[tid + b];
+            w.x += v.x;
+            w.y += v.y;
+            w.z += v.z;
+            w.w += v.w;
+        }
         for (int c = 0; c < kSyncChunk; ++c) {
             const int d = d0 + c;
             const float den = fmaxf(w.z * w.w, 1e-18f);
@@ -220,41 +279,103 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
                 cnt += crossing(i + R + 1) - crossing(i - R);
             }
         }
-        __syncthreads();
-        for (int i = warp; i < mspan; i += kSyncThreads / 32) {
-            if (sh.memo[i] != -2.0f) continue;
-            const float m = fine_metric(x, sh.win, base, kSyncPass + pre, base - R + i, preamble, pre, p.pre_energy, lane);
-            if (lane == 0) sh.memo[i] = m;
+        // groups of four memo positions holding one to evaluate, listed in increasing order
+        const int groups = (mspan + 3) / 4, per = (groups + kSyncThreads - 1) / kSyncThreads;
+        if (tid < 4 * groups - mspan) sh.memo[mspan + tid] = -1.0f;
+        if (tid == 0) {
+            sh.s_key[kSyncThreads / 32] = 0x7fffffff;      // first memo position over the threshold
+            sh.s_key[kSyncThreads / 32 + 1] = 0x7fffffff;  // the crossing that succeeds
         }
         __syncthreads();
-        // earliest crossing of the pass whose window maximum reaches the threshold
-        int first = 0x7fffffff, fstart = -1;
-        float fbm = 0.0f;
-        for (int c = 0; c < kSyncChunk; ++c) {
-            const int d = tid * kSyncChunk + c;
-            if (!(sh.metric[d] >= p.threshold)) continue;
-            const int cand = base + d;
-            const int lo = max(0, cand - R);
-            const int hi = min(avail - pre, cand + R);
+        auto wanted = [&](int g) -> bool {
+            const float4 v = reinterpret_cast<const float4*>(sh.memo)[g];
+            return v.x == -2.0f || v.y == -2.0f || v.z == -2.0f || v.w == -2.0f;
+        };
+        int mine = 0;
+        for (int g = tid * per; g < min(groups, (tid + 1) * per); ++g) mine += wanted(g) ? 1 : 0;
+        int incl = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) sh.s_key[warp] = incl;
+        __syncthreads();
+        int at = incl - mine, total = 0;
+        for (int w = 0; w < kSyncThreads / 32; ++w) {
+            if (w < warp) at += sh.s_key[w];
+            total += sh.s_key[w];
+        }
+        for (int g = tid * per; g < min(groups, (tid + 1) * per); ++g)
+            if (wanted(g)) sh.list[at++] = static_cast<uint16_t>(g);
+        __syncthreads();
+        // The earliest crossing whose window (+-R) holds a fine metric over the threshold is the
+        // first crossing within R of the first such position x: the windows of earlier ones end
+        // before x.  So the positions are evaluated in order, until x and its 2R successors are.
+        int* first_over = sh.s_key + kSyncThreads / 32;
+        const bool every = !(p.threshold > 0.0f);  // any crossing succeeds then
+        for (int b = 0; b < total; b += kSyncThreads / 32) {
+            if (b + warp < total) {
+                const int i0 = 4 * sh.list[b + warp], x0 = base - R + i0;
+                float m[4];
+                if (x0 >= base && x0 + 3 + pre <= base + span) {
+                    fine_metric4(sh.win, x0 - base, preamble, pre, p.pre_energy, lane, m);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        m[k] = sh.memo[i0 + k] == -2.0f ? fine_metric(x, sh.win, base, kSyncPass + pre, x0 + k, preamble,
+                                                                       pre, p.pre_energy, lane)
+                                                        : -1.0f;
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    int over = 0x7fffffff;
+#pragma unroll
+                    for (int k = 3; k >= 0; --k) {
+                        if (sh.memo[i0 + k] != -2.0f) continue;
+                        sh.memo[i0 + k] = m[k];
+                        if (m[k] >= p.threshold) over = i0 + k;
+                    }
+                    if (over != 0x7fffffff) atomicMin(first_over, over);
+                }
+            }
+            __syncthreads();
+            const int over = *first_over;
+            __syncthreads();  // read by every thread before the next batch lowers it: all leave together
+            if (!every && over != 0x7fffffff && 4 * sh.list[min(b + kSyncThreads / 32, total) - 1] + 3 >= over + 2 * R) break;
+        }
+        // the crossing: memo index x is sample base - R + x, so candidates d in [x - 2R, x]
+        const int xo = *first_over;
+        if (every || xo != 0x7fffffff) {
+            for (int c = 0; c < kSyncChunk; ++c) {
+                const int d = tid * kSyncChunk + c;
+                if (sh.metric[d] >= p.threshold && (every || (d >= xo - 2 * R && d <= xo))) {
+                    atomicMin(first_over + 1, d);
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        const int d = first_over[1];
+        if (d != 0x7fffffff && warp == 0) {  // the first maximum of its window, if above 0
+            const int cand = base + d, lo = max(0, cand - R), hi = min(avail - pre, cand + R);
             float bm = 0.0f;
-            int bd = cand;
-            for (int dd = lo; dd <= hi; ++dd) {
+            int bd = 0x7fffffff;
+            for (int dd = lo + lane; dd <= hi; dd += 32) {
                 const float m = sh.memo[dd - base + R];
                 if (m > bm) { bm = m; bd = dd; }
             }
-            if (bm >= p.threshold) { first = d; fstart = bd; fbm = bm; break; }
+            for (int o = 16; o > 0; o >>= 1) {
+                const float om = __shfl_xor_sync(0xffffffffu, bm, o);
+                const int od = __shfl_xor_sync(0xffffffffu, bd, o);
+                if (om > bm || (om == bm && od < bd)) { bm = om; bd = od; }
+            }
+            if (lane == 0) {
+                sh.s_res->key = cand;
+                sh.s_res->start = bd == 0x7fffffff ? cand : bd;
+                sh.s_res->fine = bm;
+                sh.s_res->coarse = sh.metric[d];
+            }
         }
-        const int wmin = __reduce_min_sync(0xffffffffu, static_cast<unsigned>(first));
-        if (lane == 0) sh.s_key[warp] = wmin;
-        __syncthreads();
-        int bmin = 0x7fffffff;
-        for (int w = 0; w < kSyncThreads / 32; ++w) bmin = min(bmin, sh.s_key[w]);
-        if (bmin != 0x7fffffff && first == bmin) {
-            sh.s_res->key = base + first;
-            sh.s_res->start = fstart;
-            sh.s_res->fine = fbm;
-            sh.s_res->coarse = sh.metric[first];
-                    }
     }
     __syncthreads();
 }
@@ -346,10 +467,10 @@ sync_kernel(const float2* __restrict__ samples, long long stride, const long lon
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float red[4 * (kSyncThreads / 32)];
     __shared__ float rmetric[kMaxRefine];
-    __shared__ int s_key[kSyncThreads / 32];
+    __shared__ int s_key[kSyncThreads / 32 + 2];
     __shared__ PassResult s_res;
     __shared__ int s_flag;
-    const SyncShared sh = sync_shared(smem_raw, p.pre_len, red, rmetric, s_key, &s_res);
+    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_res);
 
     // pass-major order: the first passes of all frames run first, so later
     // passes of a frame found early skip their scans
@@ -428,11 +549,11 @@ ingest_extract_kernel(const float2* __restrict__ window, int n, const float2* __
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float red[4 * (kSyncThreads / 32)];
     __shared__ float rmetric[kMaxRefine];
-    __shared__ int s_key[kSyncThreads / 32];
+    __shared__ int s_key[kSyncThreads / 32 + 2];
     __shared__ PassResult s_res;
     __shared__ SyncOut s_out;
     __shared__ IngestState s_st;
-    const SyncShared sh = sync_shared(smem_raw, p.pre_len, red, rmetric, s_key, &s_res);
+    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_res);
     const int tid = threadIdx.x;
     if (tid == 0) {
         s_st = *state;
@@ -509,6 +630,13 @@ ingest_extract_kernel(const float2* __restrict__ window, int n, const float2* __
     if (tid == 0) *state = s_st;
 }
 
+// The preambles accepted: those whose search would fit 200 KB with the widest refinement radius.
+static size_t sync_smem_limit(int pre_len)
+{
+    return static_cast<size_t>((kSyncPass + pre_len + 1) & ~1) * sizeof(float2) + static_cast<size_t>(kSyncPass) * sizeof(float) +
+           kSyncThreads * sizeof(float4) + static_cast<size_t>(kSyncPass + 2 * kMaxRadius) * sizeof(float);
+}
+
 static long long sync_passes(long long stride, const int* counts, int count, const SyncParams& p)
 {
     // passes of the longest search: frames hold at most `stride` samples
@@ -533,11 +661,9 @@ void launch_sync(const float2* samples, long long stride, const int* counts, int
                  const long long* frame_off, const int* frames_ptr, void* caller_scratch, size_t caller_scratch_bytes)
 {
     if (frames <= 0) return;
-    const size_t smem = static_cast<size_t>((kSyncPass + p.pre_len + 1) & ~1) * sizeof(float2) +
-                        static_cast<size_t>(kSyncPass) * sizeof(float) + kSyncThreads * sizeof(float4) +
-                        static_cast<size_t>(kSyncPass + 2 * kMaxRadius) * sizeof(float);
-    if (smem > 200 * 1024) throw InvalidArgument("preamble too long for the sync kernel");
+    if (sync_smem_limit(p.pre_len) > 200 * 1024) throw InvalidArgument("preamble too long for the sync kernel");
     if (p.radius > kMaxRadius || p.radius < 0) throw InvalidArgument("refinement radius must be 0..511");
+    const size_t smem = sync_smem(p.pre_len, p.radius);
     const long long passes = sync_passes(stride, counts, count, p);
     if (passes * frames > 0x7fffffffLL) throw InvalidArgument("sync grid too large");
     const SyncScratchLayout l = sync_scratch_layout(stride, counts, count, frames, p);
@@ -1179,11 +1305,9 @@ void launch_ingest_extract(const float2* window, int n, const float2* preamble, 
                            const IngestParams& ip, const int* slots, float2* pool, IngestRecord* rec,
                            IngestState* state, cudaStream_t st)
 {
-    const size_t smem = static_cast<size_t>((kSyncPass + sp.pre_len + 1) & ~1) * sizeof(float2) +
-                        static_cast<size_t>(kSyncPass) * sizeof(float) + kSyncThreads * sizeof(float4) +
-                        static_cast<size_t>(kSyncPass + 2 * kMaxRadius) * sizeof(float);
-    if (smem > 200 * 1024) throw InvalidArgument("preamble too long for the sync kernel");
+    if (sync_smem_limit(sp.pre_len) > 200 * 1024) throw InvalidArgument("preamble too long for the sync kernel");
     if (sp.radius > kMaxRadius || sp.radius < 0) throw InvalidArgument("refinement radius must be 0..511");
+    const size_t smem = sync_smem(sp.pre_len, sp.radius);
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(ingest_extract_kernel), smem),
                "cudaFuncSetAttribute(ingest)");
     ingest_extract_kernel<<<1, kSyncThreads, smem, st>>>(window, n, preamble, sp, ip, slots, pool, rec, state);
