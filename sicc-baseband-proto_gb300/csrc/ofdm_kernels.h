@@ -63,12 +63,24 @@ struct DemodView {
     const int* interp_p1;      // [num_data]
     const float* interp_alpha; // [num_data]
     const float2* pilot_grid;  // [num_pilots][active_sc]
-    const float2* twiddle;     // [nfft]: exp(-2 pi i j / nfft)
+    const float2* twiddle;     // [fft_twiddles(nfft)] exp(-2 pi i j / nfft) in the order the FFT reads them
     const float* axis_levels;  // [2^(bps/2)] constellation amplitude by Gray axis index (bps >= 2)
     int max_pilots_per_cta;    // pilot symbols one CTA's data symbols refer to, at most kDemodMaxPilots
 };
 
 constexpr int kDemodMaxPilots = 4;
+
+// Twiddles of the shared-memory FFT of nfft points, in reading order (rounded up to an even count,
+// so the buffers after them stay 16-byte aligned): for each radix-4 stage of span ns = 4, 16, ...
+// exp(-2 pi i r k / (4 ns)) for r = 1, 2, 3 and k < ns, then exp(-2 pi i k / nfft), k < nfft / 2, of
+// the radix-2 stage when log2 nfft is odd.
+constexpr int fft_twiddles(int nfft)
+{
+    int n = 0, ns = 1;
+    for (; ns * 4 <= nfft; ns *= 4) n += ns > 1 ? 3 * ns : 0;
+    if (ns < nfft) n += ns;
+    return (n + 1) & ~1;
+}
 
 // Fused demodulator: CFO derotation + CP strip + FFT + LS pilot estimate +
 // interpolation + MMSE equalisation + max-log LLR.  Frame f's samples start at
@@ -128,9 +140,10 @@ struct TxView {
     const float2* preamble;      // [pre_len]
     const float2* precomp_h;     // [num_symbols][active_sc] or null
     const float2* actual_h;      // [num_symbols][active_sc] or null
-    const float2* twiddle;       // [nfft] exp(-2 pi i j / nfft)
+    const float2* twiddle;       // [fft_twiddles(nfft)] as DemodView's
     const uint32_t* gen_words;   // [code_k][gen_stride] bit-packed generator rows (bit j of word w: column 32w + j)
     int gen_stride;
+    int systematic;              // 1: the generator is [I | P]
     const uint32_t* gen_tab;     // [ceil(code_k/8)][256][gen_stride]: XOR of the 8 rows 8g.. selected by a byte, or null
     const int* acc_offsets;      // accumulator encoder: [m + 1] row starts in acc_cols (null: generator encoder)
     const int* acc_cols;         // information columns of each parity row

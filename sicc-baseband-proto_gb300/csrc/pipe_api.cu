@@ -327,12 +327,19 @@ int sicc_pipe_upload_static_tables(unsigned long long handle, const sicc_pipe_ta
         for (int i = 0; i < c.preamble_len; ++i)
             e += t->preamble[2 * i] * t->preamble[2 * i] + t->preamble[2 * i + 1] * t->preamble[2 * i + 1];
         p->pre_energy = e;
-        // twiddles exp(-2 pi i j / N), computed in double
-        std::vector<float2> tw(c.nfft);
-        for (int j = 0; j < c.nfft; ++j) {
+        // twiddles exp(-2 pi i j / N) in the FFT's reading order, computed in double
+        std::vector<float2> tw;
+        auto twiddle = [&](int j) {
             const double a = -2.0 * 3.141592653589793238462643383279502884 * j / c.nfft;
-            tw[j] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
-        }
+            tw.push_back(make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a))));
+        };
+        int ns = 1;
+        for (; ns * 4 <= c.nfft; ns *= 4)
+            for (int r = 1; ns > 1 && r <= 3; ++r)
+                for (int k = 0; k < ns; ++k) twiddle(r * k * (c.nfft / (4 * ns)));
+        if (ns < c.nfft)
+            for (int k = 0; k < ns; ++k) twiddle(k * (c.nfft / (2 * ns)));
+        tw.resize(std::max(fft_twiddles(c.nfft), 1), make_float2(1.0f, 0.0f));
         upload(p->twiddle, tw.data(), tw.size());
         // axis amplitudes of Gray square QAM, scaled to unit average power as the
         // reference constellation (uhd_ldpc_ofdm_link.cpp:2362-2414)
@@ -698,6 +705,10 @@ int sicc_pipe_upload_tx_tables(unsigned long long handle, const sicc_pipe_tx_tab
             }
             p->acc_off.release();
             p->acc_cols.release();
+            x.systematic = k % 32 == 0 ? 1 : 0;  // [I | P]: what the systematic encoder takes
+            for (int r = 0; r < k && x.systematic; ++r)
+                for (int w = 0; w < k / 32; ++w)
+                    if (words[static_cast<size_t>(r) * gw + w] != (w == r / 32 ? 1u << (r % 32) : 0u)) x.systematic = 0;
             x.gen_words = p->gen.p;
             x.gen_tab = p->gen_tab.p;
             x.gen_stride = gw;
