@@ -13,16 +13,19 @@
 //      single precision; the first candidate with the smallest metric wins
 //      (strict <, cpu_bp_osd_decode.m:222), realised as a minimum over
 //      (metric bits, test index) keys.
-// Candidates are evaluated by all 32 lanes in parallel; each candidate's
-// difference vector is the base difference XOR at most three reduced rows.
-// A lane stops summing a candidate once its partial metric exceeds the best
-// metric it knows; the warp exchanges its best every `share_rounds` rounds of
-// 32 candidates (a launch parameter, chosen by the autotuner).  Pruning only
-// drops candidates that cannot win, so the winner is the same for any value.
+// Candidates are tested by all 32 lanes in parallel; each candidate's
+// difference vector is the base difference XOR at most three reduced rows.  A
+// lower bound of the metric from nibble tables screens them; the few that pass
+// are summed in order, stopping once over the best metric.  Both only drop
+// candidates that cannot win.
+//
+// What bounds it: instruction issue and the ALU pipe.  Measured on GB300, the
+// 13,000 failed codewords of 65,536 (128,64) frames at 2 dB (13,400 warp
+// instructions each before): 265 us with a broadcast pivot row per column and
+// every surviving candidate summed in order, 187 us now.
 #include "bp_kernels.h"
 
 #include <algorithm>
-#include <type_traits>
 
 namespace sicc {
 
@@ -35,26 +38,33 @@ constexpr int kOsdWarps = 8;
 template <int NW, int KR>
 constexpr bool kFlipRows = NW * KR <= 4;
 
+// The tail: sorted positions from 64 (NW / 2) on, the less reliable half (all of them at NW = 1),
+// where nearly all parity positions lie.
+template <int NW>
+constexpr int kTailWord = NW / 2;
+template <int NW>
+constexpr int kTailNibbles = (NW - NW / 2) * 16;
+
 template <int NW, int KR>
 struct OsdSmem {
     float rel_sorted[NW * 64];
     int16_t perm[NW * 64];
     int16_t rowpiv[KR * 32];  // row id -> pivot index
     int16_t flip[KR * 32];    // weakness rank -> pivot index
-    uint32_t hard_orig[NW * 2];
-    unsigned long long rows[KR * 32][NW];  // reduced rows by pivot index
+    union {
+        unsigned long long rows[KR * 32][NW];  // reduced rows by pivot index
+        struct {  // before them, during the elimination:
+            unsigned long long raw[8][NW];     // the round's pivot rows as the round found them
+            unsigned long long tab[32][NW];    // XORs of raw[0..3] by 4-bit index, then of raw[4..7]
+        } el;
+    };
     unsigned long long frows[kFlipRows<NW, KR> ? KR * 32 : 1][NW];  // the same rows by flip-pool rank
     int16_t mrb_pos[KR * 32];
     float prel[KR * 32];      // flip-pool rank -> |llr| of its position (non-decreasing)
+    float low[KR * 32];       // the same where the position lies below kTail, else 0
+    float nib[kTailNibbles<NW>][16];  // sums of |llr| over the set bits of each nibble of the tail
     int16_t rstart[KR * 32];  // order-2 rows: first surviving pair of row a in the compact list
 };
-
-__device__ __forceinline__ unsigned long long shfl_u64(unsigned long long v, int src)
-{
-    const unsigned lo = __shfl_sync(0xffffffffu, static_cast<unsigned>(v), src);
-    const unsigned hi = __shfl_sync(0xffffffffu, static_cast<unsigned>(v >> 32), src);
-    return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
 
 // Word `w` of a register array, selected without dynamic indexing (which
 // would move the array to local memory).
@@ -107,74 +117,87 @@ osd_kernel(OsdView ov0, OsdIO io)
                                                        : io.out_info + static_cast<size_t>(cw) * io.info_stride)
                                         : nullptr;
         // ---- 1. reliabilities, hard decisions, stable descending sort ----
-        // Bitonic sort of 64-bit keys in registers (element q*32 + lane in v[q]):
-        // ascending key = descending |llr|, ties by ascending index (the order of
-        // MATLAB's stable sort, cpu_bp_osd_decode.m:194).
+        // Bitonic sort of 64-bit keys in registers (element lane * KPL + q in v[q]): ascending key =
+        // descending |llr|, ties by ascending index (the order of MATLAB's stable sort,
+        // cpu_bp_osd_decode.m:194).  The lowest bit carries the hard decision (the index above it is
+        // unique, so it orders nothing).  The merge levels and the distances across lanes are
+        // run-time loops: unrolled, the sort alone would be 30 KB of code and every warp would
+        // wait for instructions.
         constexpr int NP = NW * 64, KPL = NP / 32;
         unsigned long long v[KPL];
+        auto key = [&](int i, float x) -> unsigned long long {
+            return (static_cast<unsigned long long>(0x7fffffffu - __float_as_uint(fabsf(x))) << 32) |
+                   static_cast<unsigned>(2 * i + (x < 0.0f ? 1 : 0));
+        };
+        if (n == NP && (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && KPL % 4 == 0) {
 #pragma unroll
-        for (int q = 0; q < KPL; ++q) {
-            const int i = q * 32 + lane;
-            const float x = (i < n) ? src[i] : 0.0f;
-            v[q] = (i < n) ? ((static_cast<unsigned long long>(0x7fffffffu - __float_as_uint(fabsf(x))) << 32) |
-                              static_cast<unsigned>(i))
-                           : ~0ull;
-            const unsigned hb = __ballot_sync(0xffffffffu, (i < n) && (x < 0.0f));
-            if (lane == 0) s.hard_orig[q] = hb;
+            for (int q = 0; q + 4 <= KPL; q += 4) {
+                const int i = lane * KPL + q;
+                const float4 x = *reinterpret_cast<const float4*>(src + i);
+                v[q] = key(i, x.x);
+                v[q + 1] = key(i + 1, x.y);
+                v[q + 2] = key(i + 2, x.z);
+                v[q + 3] = key(i + 3, x.w);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < KPL; ++q) {
+                const int i = lane * KPL + q;
+                v[q] = (i < n) ? key(i, src[i]) : ~0ull;
+            }
         }
-#pragma unroll
+#pragma unroll 1
         for (int k2 = 2; k2 <= NP; k2 <<= 1) {
+            const bool up = ((lane * KPL) & k2) == 0;  // the order of my elements, for k2 >= KPL
+#pragma unroll 1
+            for (int j2 = k2 >> 1; j2 >= KPL; j2 >>= 1) {  // partner in another lane
+                const int m = j2 / KPL;
+                const bool take_min = ((lane & m) == 0) == up;
 #pragma unroll
-            for (int j2 = k2 >> 1; j2 > 0; j2 >>= 1) {
-                if (j2 >= 32) {  // partner in this lane
+                for (int q = 0; q < KPL; ++q) {
+                    const unsigned long long o = shfl_xor_u64(v[q], m);
+                    v[q] = ((o < v[q]) == take_min) ? o : v[q];
+                }
+            }
 #pragma unroll
-                    for (int q = 0; q < KPL; ++q) {
-                        if (q & (j2 >> 5)) continue;
-                        const int q2 = q | (j2 >> 5);
-                        const bool asc = ((q * 32 + lane) & k2) == 0;
-                        const unsigned long long a = v[q], b = v[q2];
-                        if ((a > b) == asc) {
-                            v[q] = b;
-                            v[q2] = a;
-                        }
-                    }
-                } else {  // partner in lane ^ j2
+            for (int j2 = KPL / 2; j2 > 0; j2 >>= 1) {  // partner in this lane
+                if (j2 >= k2) continue;
 #pragma unroll
-                    for (int q = 0; q < KPL; ++q) {
-                        const unsigned long long o = shfl_xor_u64(v[q], j2);
-                        const bool asc = ((q * 32 + lane) & k2) == 0;
-                        const bool take_min = ((lane & j2) == 0) == asc;
-                        v[q] = take_min ? (o < v[q] ? o : v[q]) : (o > v[q] ? o : v[q]);
+                for (int q = 0; q < KPL; ++q) {
+                    if (q & j2) continue;
+                    const bool asc = k2 >= KPL ? up : (q & k2) == 0;
+                    const unsigned long long x = v[q], y = v[q | j2];
+                    if ((x > y) == asc) {
+                        v[q] = y;
+                        v[q | j2] = x;
                     }
                 }
             }
         }
+        unsigned hb = 0u;  // hard decisions of my KPL sorted positions
 #pragma unroll
         for (int q = 0; q < KPL; ++q) {
-            const int r = q * 32 + lane;
+            const int r = lane * KPL + q;
             if (r < n) {
-                s.perm[r] = static_cast<int16_t>(v[q] & 0xffffffffull);
+                s.perm[r] = static_cast<int16_t>((v[q] & 0xffffffffull) >> 1);
                 s.rel_sorted[r] = __uint_as_float(0x7fffffffu - static_cast<unsigned>(v[q] >> 32));
+                hb |= (static_cast<unsigned>(v[q]) & 1u) << q;
             }
         }
-        __syncwarp();
-        // hard decisions in sorted order
+        // hard decisions in sorted order: 32 / KPL lanes per half-word
         unsigned long long hard_sorted[NW];
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
-            unsigned lo, hi;
-            {
-                const int j = w * 64 + lane;
-                const int o = (j < n) ? s.perm[j] : 0;
-                lo = __ballot_sync(0xffffffffu, (j < n) && ((s.hard_orig[o >> 5] >> (o & 31)) & 1u));
+            unsigned half[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                constexpr int per = 32 / KPL;
+                const unsigned mine = lane / per == 2 * w + h ? hb << ((lane % per) * KPL) : 0u;
+                half[h] = __reduce_or_sync(0xffffffffu, mine);
             }
-            {
-                const int j = w * 64 + 32 + lane;
-                const int o = (j < n) ? s.perm[j] : 0;
-                hi = __ballot_sync(0xffffffffu, (j < n) && ((s.hard_orig[o >> 5] >> (o & 31)) & 1u));
-            }
-            hard_sorted[w] = (static_cast<unsigned long long>(hi) << 32) | lo;
+            hard_sorted[w] = (static_cast<unsigned long long>(half[1]) << 32) | half[0];
         }
+        __syncwarp();
         // ---- 2. permuted generator rows via ballots over column vectors ----
         unsigned long long rows[KR][NW];
 #pragma unroll
@@ -213,56 +236,85 @@ osd_kernel(OsdView ov0, OsdIO io)
             }
         }
         // ---- 3. column-scan elimination: pivots = most reliable basis ----
-        // Column j lives in bit j % 32 of 32-bit half (j / 32) % 2 of word j / 64 of every row:
-        // the scan runs half-word by half-word, so the column's half is a register known at
-        // compile time and each row test is one 32-bit operation.
-        unsigned avail = 0;  // bit a: my row in slot a exists (r < k) and is not yet a pivot row
+        // Columns are taken 8 at a time (a byte of every row).  Within a round only the bytes are
+        // eliminated, column by column: val[a] holds my row's byte (bits 0-7) and which of the
+        // round's pivot rows it has taken (bits 8-15, over the rows as they were before the
+        // round), so one shuffle and one XOR per column update both.  The rows themselves take
+        // the round at once, from the XORs of the 8 pivot rows tabulated by 4-bit index: two
+        // table reads per row instead of a broadcast row and a test per column.
+        unsigned avail[KR];  // 0xff while my row in slot a exists (r < k) and is not yet a pivot row
 #pragma unroll
-        for (int a = 0; a < KR; ++a) avail |= (a * 32 + lane < k) ? 1u << a : 0u;
+        for (int a = 0; a < KR; ++a) avail[a] = (a * 32 + lane < k) ? 0xffu : 0u;
         int rank = 0;
+        {
+#pragma unroll 1
+            for (int j0 = 0; j0 < n && rank < k; j0 += 8) {
+                unsigned val[KR];
+                int took[KR];  // this round: column << 8 | rank of the pivot my row became, -1 for none
 #pragma unroll
-        for (int W = 0; W < NW; ++W) {
+                for (int a = 0; a < KR; ++a) {
+                    val[a] = static_cast<unsigned>(pick<NW>(rows[a], j0 >> 6) >> (j0 & 63)) & 0xffu;
+                    took[a] = -1;
+                }
+                const int before = rank;
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                for (int b = 0; b < 32 && rank < k; ++b) {
-                    const int j = W * 64 + hh * 32 + b;
-                    if (j >= n) break;
-                    const unsigned bm = 1u << b;
-                    auto has = [&](int a) { return (static_cast<unsigned>(rows[a][W] >> (hh * 32)) & bm) != 0u; };
+                for (int r = 0; r < 8; ++r) {
+                    if (j0 + r >= n || rank >= k) break;
                     int ps = -1, pl = 0;
+                    unsigned pv = 0u;
 #pragma unroll
                     for (int a = 0; a < KR; ++a) {
-                        const unsigned bal = __ballot_sync(0xffffffffu, ((avail >> a) & 1u) && has(a));
+                        const unsigned bal = __ballot_sync(0xffffffffu, (val[a] & avail[a] & (1u << r)) != 0u);
                         if (ps < 0 && bal) {
                             ps = a;
                             pl = __ffs(bal) - 1;
+                            pv = val[a];
                         }
                     }
                     if (ps < 0) continue;  // dependent position
-                    unsigned long long pw[NW];
-#pragma unroll
-                    for (int w = 0; w < NW; ++w) {
-                        unsigned long long mine = 0ull;
-#pragma unroll
-                        for (int a = 0; a < KR; ++a)
-                            if (a == ps) mine = rows[a][w];
-                        pw[w] = shfl_u64(mine, pl);
-                    }
+                    pv = __shfl_sync(0xffffffffu, pv, pl) ^ (0x100u << r);
 #pragma unroll
                     for (int a = 0; a < KR; ++a) {
-                        const bool is_p = (a == ps) && (lane == pl);
-                        if (!is_p && has(a)) {
-#pragma unroll
-                            for (int w = 0; w < NW; ++w) rows[a][w] ^= pw[w];
+                        const bool is_p = lane == pl && a == ps;
+                        if ((val[a] & (1u << r)) && !is_p) val[a] ^= pv;
+                        if (is_p) {
+                            avail[a] = 0u;
+                            took[a] = (r << 8) | rank;
                         }
-                        if (is_p) avail &= ~(1u << a);
-                    }
-                    if (lane == 0) {
-                        s.rowpiv[ps * 32 + pl] = static_cast<int16_t>(rank);
-                        s.mrb_pos[rank] = static_cast<int16_t>(j);
                     }
                     ++rank;
                 }
+                if (rank == before) continue;
+#pragma unroll
+                for (int a = 0; a < KR; ++a) {
+                    if (took[a] >= 0) {  // the row as it was before the round
+                        const int r = took[a] >> 8, t = took[a] & 0xff;
+#pragma unroll
+                        for (int w = 0; w < NW; ++w) s.el.raw[r][w] = rows[a][w];
+                        s.rowpiv[a * 32 + lane] = static_cast<int16_t>(t);
+                        s.mrb_pos[t] = static_cast<int16_t>(j0 + r);
+                    }
+                }
+                __syncwarp();
+                {  // entry `lane`: XOR of the rows its low 4 bits select (rows of dependent columns are never selected)
+                    const int h = (lane >> 4) * 4;
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) {
+                        unsigned long long x = 0ull;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if ((lane >> i) & 1) x ^= s.el.raw[h + i][w];
+                        s.el.tab[lane][w] = x;
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int a = 0; a < KR; ++a) {
+                    const unsigned lo = (val[a] >> 8) & 15u, hi = 16u + ((val[a] >> 12) & 15u);
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) rows[a][w] ^= s.el.tab[lo][w] ^ s.el.tab[hi][w];
+                }
+                __syncwarp();  // read before the next round writes
             }
         }
         __syncwarp();
@@ -320,10 +372,20 @@ osd_kernel(OsdView ov0, OsdIO io)
             if (r < ov.pool) {
                 s.flip[r] = static_cast<int16_t>(t);
                 s.prel[r] = s.rel_sorted[s.mrb_pos[t]];
+                s.low[r] = s.mrb_pos[t] < kTailWord<NW> * 64 ? s.prel[r] : 0.0f;
                 if (kFlipRows<NW, KR>)
 #pragma unroll
                     for (int w = 0; w < NW; ++w) s.frows[kFlipRows<NW, KR> ? r : 0][w] = s.rows[t][w];
             }
+        }
+        // sums of |llr| over the set bits of every nibble of the tail
+        for (int e = lane; e < kTailNibbles<NW> * 16; e += 32) {
+            const float* rel = s.rel_sorted + kTailWord<NW> * 64 + (e >> 4) * 4;
+            float x = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (((e >> i) & 1) && kTailWord<NW> * 64 + (e >> 4) * 4 + i < n) x += rel[i];
+            (&s.nib[0][0])[e] = x;
         }
         __syncwarp();
         // ---- 6. all candidates in parallel ----
@@ -331,36 +393,61 @@ osd_kernel(OsdView ov0, OsdIO io)
         // its partial sums never decrease: once one exceeds the smallest metric
         // already found the candidate cannot win and its sum stops.  Ties are not
         // pruned (strict >), so the first minimum in test order still wins.
+        // Before that walk a candidate meets a bound: its differing positions of the tail summed
+        // from the nibble tables, plus its flips before the tail.  All terms are non-negative; the
+        // metric's own sum (up to 256 terms in order) lies below the exact one by less than 255
+        // rounding units and the bound above its exact value by less than 30, so a candidate whose
+        // bound is over the best metric by a factor 1 + 2^-15 (512 units) cannot win.  The bound
+        // takes the same 16 (or 32) steps in every lane, and few candidates pass it.
         unsigned long long best_key = ~0ull;
         float thr = INFINITY;
-        const int share = io.share_rounds > 0 ? io.share_rounds : 2;
-        // The metric of test q, whose flips are pool ranks f0, f1, f2, pruned against thr.  The
-        // first `kSure` flips are known to exist (no test); the others may be -1 (none).
-        auto evaluate = [&](auto sure, int q, int f0, int f1, int f2) {
-            constexpr int kSure = decltype(sure)::value;
+        auto flip_row = [&](int rank) -> const unsigned long long* {
+            if constexpr (kFlipRows<NW, KR>) return s.frows[rank];
+            else return s.rows[s.flip[rank]];
+        };
+        auto bound = [&](int f0, int f1, int f2) -> float {  // flips: pool ranks, -1 for none
+            const int fl[3] = {f0, f1, f2};
+            float lb = 0.0f;
+            unsigned long long d[NW - kTailWord<NW>];
+#pragma unroll
+            for (int w = kTailWord<NW>; w < NW; ++w) d[w - kTailWord<NW>] = acc[w];
+#pragma unroll
+            for (int f = 0; f < 3; ++f) {
+                const int fi = fl[f];
+                if (fi >= 0) {
+                    lb += s.low[fi];
+                    const unsigned long long* row = flip_row(fi);
+#pragma unroll
+                    for (int w = kTailWord<NW>; w < NW; ++w) d[w - kTailWord<NW>] ^= row[w];
+                }
+            }
+            float part[2] = {lb, 0.0f};
+#pragma unroll
+            for (int i = 0; i < kTailNibbles<NW>; ++i) {
+                const unsigned x = static_cast<unsigned>(d[i >> 4] >> ((i & 8) * 4));
+                part[i & 1] += s.nib[i][(x >> ((i & 7) * 4)) & 15u];
+            }
+            return part[0] + part[1];
+        };
+        constexpr float kSlack = 1.0f + 3.0517578125e-05f;  // 1 + 2^-15
+        // The metric of test q, whose flips are pool ranks f0, f1, f2 (-1: none), pruned against thr.
+        auto evaluate = [&](int q, int f0, int f1, int f2) {
             unsigned long long d[NW];
 #pragma unroll
             for (int w = 0; w < NW; ++w) d[w] = acc[w];
             const int fl[3] = {f0, f1, f2};
 #pragma unroll
             for (int f = 0; f < 3; ++f) {
-                const int fi = fl[f];
-                if (f < kSure || fi >= 0) {
-                    if (kFlipRows<NW, KR>) {
+                if (fl[f] < 0) continue;
+                const unsigned long long* row = flip_row(fl[f]);
 #pragma unroll
-                        for (int w = 0; w < NW; ++w) d[w] ^= s.frows[kFlipRows<NW, KR> ? fi : 0][w];
-                    } else {
-                        const int t = s.flip[fi];
-#pragma unroll
-                        for (int w = 0; w < NW; ++w) d[w] ^= s.rows[t][w];
-                    }
-                }
+                for (int w = 0; w < NW; ++w) d[w] ^= row[w];
             }
             float metric = 0.0f;
             bool pruned = false;
-#pragma unroll
-            for (int h = 0; h < 2 * NW; ++h) {
-                unsigned bits = static_cast<unsigned>(d[h >> 1] >> ((h & 1) * 32));
+#pragma unroll 1
+            for (int h = 0; h < 2 * NW && !pruned; ++h) {
+                unsigned bits = static_cast<unsigned>(pick<NW>(d, h >> 1) >> ((h & 1) * 32));
                 const float* rel = s.rel_sorted + h * 32;
                 while (bits && !pruned) {
                     const int b = __ffs(bits) - 1;
@@ -386,34 +473,18 @@ osd_kernel(OsdView ov0, OsdIO io)
             }
             if (best_key != ~0ull) thr = __uint_as_float(static_cast<unsigned>(best_key >> 32));
         };
-        auto flips_of = [&](int q, int& f0, int& f1, int& f2) {
-            f0 = f1 = f2 = -1;
-            if (q > 0) {
-                const uint32_t cmb = ov.combos[q - 1];
-                const uint32_t a = cmb & 0x3FFu, b = (cmb >> 10) & 0x3FFu, c = (cmb >> 20) & 0x3FFu;
-                f0 = a != 0x3FFu ? static_cast<int>(a) : -1;
-                f1 = b != 0x3FFu ? static_cast<int>(b) : -1;
-                f2 = c != 0x3FFu ? static_cast<int>(c) : -1;
-            }
-        };
         const int P = ov.pool;
+        // Complete order 2: the tests are the base, the P single flips, then every pair (a, b),
+        // a < b, in lexicographic order (test 1 + P + a (2P - a - 1) / 2 + b - a - 1).  A candidate
+        // differs from the hard decision at its flipped positions, and the metric, summed in
+        // position order, is at least those terms summed alone (each rounded partial sum of a sum
+        // of non-negative terms is at least that of any of its subsequences): a pair whose two
+        // |llr| already add up above the best metric of the base and single-flip tests cannot win.
+        // The pool is weakest first, so within row a the bound grows with b and each row keeps a
+        // prefix (binary search); only those pairs are tested, 32 at a time from a compact list.
         const bool complete2 = P >= 2 && ov.num_tests == 1 + P + P * (P - 1) / 2;
-        if (complete2) {
-            // The tests are the base, the P single flips, then every pair (a, b), a < b, in
-            // lexicographic order (test 1 + P + a (2P - a - 1) / 2 + b - a - 1).  A candidate
-            // differs from the hard decision at its flipped positions, and the metric, summed in
-            // position order, is at least those terms summed alone (each rounded partial sum of
-            // a sum of non-negative terms is at least that of any of its subsequences): a pair
-            // whose two |llr| already add up above the best metric of the base and single-flip
-            // tests cannot win.  The pool is weakest first, so within row a the bound grows
-            // with b and each row keeps a prefix (binary search); only those pairs are
-            // evaluated, 32 at a time from a compact list.
-            const int single = 1 + P;
-            for (int rd = 0; rd * 32 < single; ++rd) {
-                const int q = rd * 32 + lane;
-                if (q < single) evaluate(std::integral_constant<int, 0>(), q, q > 0 ? q - 1 : -1, -1, -1);
-            }
-            share_best();
+        const int single = 1 + P;
+        auto list_pairs = [&]() -> int {  // rstart of every row; the number of pairs kept
             const int R = (P - 1 + 31) / 32;  // rows a = 0 .. P-2, R consecutive rows per lane
             int mine = 0;
             for (int i = 0; i < R; ++i) {
@@ -438,35 +509,57 @@ osd_kernel(OsdView ov0, OsdIO io)
                 const int up = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += up;
             }
-            const int base = incl - mine, total = __shfl_sync(0xffffffffu, incl, 31);
+            const int base = incl - mine;
             for (int i = 0; i < R; ++i) {
                 const int a = lane * R + i;
                 if (a < P - 1) s.rstart[a] = static_cast<int16_t>(s.rstart[a] + base);
             }
             __syncwarp();
-            int rd = 0, a = 0;  // a: the last row with rstart[a] <= idx (idx only grows: walk forward)
-            for (int i0 = 0; i0 < total; i0 += 32, ++rd) {
-                const int idx = i0 + lane;
-                if (idx < total) {
-                    while (a < P - 2 && s.rstart[a + 1] <= idx) ++a;
-                    const int b = a + 1 + (idx - s.rstart[a]);
-                    evaluate(std::integral_constant<int, 2>(), single + a * (2 * P - a - 1) / 2 + (b - a - 1), a, b, -1);
+            return __shfl_sync(0xffffffffu, incl, 31);
+        };
+        // 32 tests per pass (one site for the bound and the sum keeps the code small): first the base
+        // test alone, then the tests from 1 on, and for complete order 2 the single flips, then the pairs.
+        int stage = 0, i0 = 0, end = 1, row = 0;
+#pragma unroll 1
+        while (true) {
+            if (i0 >= end) {
+                if (stage == 0) {
+                    i0 = 1;
+                    end = complete2 ? single : ov.num_tests;
+                } else if (stage == 1 && complete2) {
+                    i0 = 0;
+                    end = list_pairs();
+                } else {
+                    break;
                 }
-                if (rd % share == share - 1) share_best();
+                ++stage;
+                continue;
             }
-        } else {
-            const int rounds = (ov.num_tests + 31) / 32;
-            for (int rd = 0; rd < rounds; ++rd) {
-                const int q = rd * 32 + lane;
-                if (q < ov.num_tests) {
-                    int f0, f1, f2;
-                    flips_of(q, f0, f1, f2);
-                    evaluate(std::integral_constant<int, 0>(), q, f0, f1, f2);
+            const int i = i0 + lane;
+            int q = i, f0 = -1, f1 = -1, f2 = -1;
+            bool go = i < end;
+            if (go && stage > 0) {
+                if (!complete2) {
+                    const uint32_t cmb = ov.combos[q - 1];
+                    const uint32_t a = cmb & 0x3FFu, b = (cmb >> 10) & 0x3FFu, c = (cmb >> 20) & 0x3FFu;
+                    f0 = a != 0x3FFu ? static_cast<int>(a) : -1;
+                    f1 = b != 0x3FFu ? static_cast<int>(b) : -1;
+                    f2 = c != 0x3FFu ? static_cast<int>(c) : -1;
+                } else if (stage == 1) {
+                    f0 = q - 1;
+                } else {  // the last row with rstart[row] <= i (i only grows: walk forward)
+                    while (row < P - 2 && s.rstart[row + 1] <= i) ++row;
+                    f0 = row;
+                    f1 = row + 1 + (i - s.rstart[row]);
+                    q = single + f0 * (2 * P - f0 - 1) / 2 + (f1 - f0 - 1);
                 }
-                if (rd % share == share - 1) share_best();
+                go = !(bound(f0, f1, f2) > thr * kSlack);
             }
+            i0 += 32;
+            if (!__any_sync(0xffffffffu, go)) continue;
+            if (go) evaluate(q, f0, f1, f2);
+            share_best();
         }
-        share_best();
         // ---- 7. winner -> original positions ----
         const int qbest = static_cast<int>(best_key & 0xffffffffull);
         unsigned long long d[NW];

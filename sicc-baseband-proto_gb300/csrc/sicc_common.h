@@ -156,10 +156,6 @@ struct OsdIO {
     const long long* llr_off;
     const long long* info_off;
     const long long* row_off;
-    // warp OSD: rounds of 32 candidates (one per lane) between exchanges of the
-    // warp's best metric, which tightens every lane's pruning bound (0 = 2);
-    // the winner does not depend on it
-    int share_rounds;
     // Work counters (device ints the launcher zeroes on the stream): each warp (warp kernel) or
     // CTA (large-code kernel, one counter per class) takes its next item from them, so a few
     // expensive codewords do not hold up one warp's share.  Null: items by static striding.
