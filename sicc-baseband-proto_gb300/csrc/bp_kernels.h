@@ -66,12 +66,12 @@ struct OsdHBounds {
     void add(int n, int m, int pool, int nnz);
     bool empty() const { return nmax == 0; }
 };
-// The large-code OSD runs in classes by m: m <= 512 and m <= 640 on 256-thread CTAs (two per SM:
-// their serial pivot selections overlap; the second without staged column lists), m <= 1024 on
-// 512-thread CTAs (one per SM: T fills it).
-constexpr int kOsdHClasses = 3;
-constexpr int kOsdHClassMaxM[kOsdHClasses] = {512, 640, 1024};
-inline int osd_h_class(int m) { return m <= 512 ? 0 : m <= 640 ? 1 : 2; }
+// The large-code OSD runs in classes by m, so that short codes get small CTAs and many of them per SM
+// (a round's serial pivot choice leaves issue slots that only other CTAs fill): m <= 256 on 128
+// threads, m <= 512 and m <= 640 on 256, m <= 1024 on 512 (T fills the SM's shared memory).
+constexpr int kOsdHClasses = 4;
+constexpr int kOsdHClassMaxM[kOsdHClasses] = {256, 512, 640, 1024};
+inline int osd_h_class(int m) { return m <= 256 ? 0 : m <= 512 ? 1 : m <= 640 ? 2 : 3; }
 // Large-code OSD over the items of io, one launch per class present in cls[kOsdHClasses]; with more
 // than one class and side streams given (kOsdHClasses - 1 of them, and as many join events), the
 // classes run side by side, forked from `st` and joined back to it.

@@ -15,11 +15,13 @@
 //   * those m columns are found by Gauss-Jordan elimination on H: the
 //     accumulated row operations T (m x m bits, 128 KiB at m = 1024) live in
 //     shared memory column-major, column c's reduced form is T h_c, the XOR
-//     of the few columns of T that h_c selects (column weight <= 16).  The
-//     pivots are taken 8 at a time; their combined row operation is linear in
-//     a column's 8 pivot-row bits (a -> a + sum_r a_{p_r} U_r), so each
-//     column of T takes it in one pass, and one warp picks the next round's
-//     pivots while the others apply the current round to T;
+//     of the few columns of T that h_c selects (column weight <= 16).  Only the
+//     columns of T at pivoted rows are stored, in pivot order: the others are
+//     unit vectors.  The pivots are taken 8 at a time; their combined row
+//     operation is linear in a column's 8 pivot-row bits (a -> a + sum_r
+//     a_{p_r} U_r), so each stored column takes it in one pass from tables of
+//     U, and one warp picks the next round's pivots while the others apply the
+//     current round to T;
 //   * with T H in reduced form on those columns, a candidate that keeps the
 //     hard decisions on the MRB except a flip set F differs from the hard
 //     decisions at the pivot positions selected by T s XOR (XOR over f in F of
@@ -35,10 +37,9 @@ namespace sicc {
 
 namespace {
 
-constexpr int kOsdHClassThreads[kOsdHClasses] = {256, 256, 512};  // CTA size by class
+constexpr int kOsdHClassThreads[kOsdHClasses] = {256, 256, 256, 512};  // CTA size by class
 constexpr int kOsdHMaxPool = 128;
 constexpr int kRound = 8;  // columns of H per elimination round
-constexpr int kHitsPerWarp = 96;  // a worker's list of touched columns (applied whenever it fills)
 constexpr int kTabStride = 33;  // words per table entry: lanes reading different entries hit different banks
 
 struct OsdHLayout {
@@ -48,28 +49,26 @@ struct OsdHLayout {
     int ts;       // column stride of T in words (odd: a warp reading one word of 32 columns hits 32 banks)
     int poolmax;
     int nnzmax;   // > 0: the columns' row lists are staged in shared memory (16-bit rows)
-    int warps;    // warps per CTA
     int mlo, mhi; // the launch decodes the items of codes with mlo < m <= mhi
 };
 
 struct OsdHSmem {
-    uint32_t* T;             // [32*mw + 2*kRound][ts] column-major: column i of the row-operation matrix,
-                             // then two buffers of kRound reduced candidate columns
+    uint32_t* T;             // [32*mw + 2*kRound][ts] column-major: the column of the row-operation matrix at the
+                             // t-th pivot's row, then two buffers of kRound reduced candidate columns; after the
+                             // elimination the tables and terms of the candidate tests
     unsigned long long* keys;// [np] sort keys; shares T's space
     int* colinfo;            // [nmax] first edge << 8 | weight of the column at each sorted position
     float* rel;              // [nmax] |llr| by sorted position j
     int16_t* perm;           // [nmax] code position at sorted position j
     int16_t* row_of_col;     // [nmax] pivot rank of a code position, -1 for the MRB
     uint32_t* hard;          // [nmax/32+1] hard decisions by code position
-    uint32_t* tab;           // [2][32][kTabStride] by round parity: entry g < 16 the XOR of U_0..3 selected by g, entry
-                             // 16 + g that of U_4..7; aliases vs..relq, which are first written after the
-                             // elimination
+    uint32_t* tab;           // [32][kTabStride]: entry g < 16 the XOR of U_0..3 selected by g, entry 16 + g that of
+                             // U_4..7; aliases vs..relq, which are first written after the elimination
     uint32_t* wv;            // [2][kRound][32] by round parity: the round's basis U_r (0 for a dependent candidate)
-    uint32_t* hits;          // [warps][kHitsPerWarp] per warp: the columns a round changes, word offset in T
-                             // (16 bits) | pivot-row index << 16
-    uint32_t* piv;           // [mw] pivoted rows
+    uint8_t* tidx;           // [32*mw] each stored column's bits at the pending round's pivot rows
+    int16_t* rank;           // [32*mw] pivot rank of a row of H (its column's place in T), -1 while it has none
     int16_t* order;          // [32*mw] row of the t-th pivot
-    uint32_t* vs;            // [poolmax+1][32] T s and T h_f by row (before reordering)
+    uint32_t* vs;            // [poolmax+1][mw] T s and T h_f by row (before reordering)
     uint32_t* syn;           // [mw] s = H * hard by row of H
     int16_t* pivj;           // [32*mw] sorted position of the t-th pivot's column
     float* relq;             // [32*mw] |llr| of the t-th pivot's column
@@ -80,6 +79,8 @@ struct OsdHSmem {
     int16_t* rows;           // [nnzmax] rows of H's columns (when staged)
 };
 
+// Floats of one warp's metric terms: m pivots, 3 flips, padding to a group of four.
+__host__ __device__ inline size_t osd_h_terms(int mw) { return 32 * static_cast<size_t>(mw) + 8; }
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
 
 __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base, OsdHSmem* s)
@@ -94,7 +95,9 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
     OsdHSmem t{};
     {  // the sort keys, then T (the keys are dead once the sorted order is extracted)
         const size_t bt = (rows + 2 * kRound) * l.ts * 4, bk = static_cast<size_t>(l.np) * 8;
-        unsigned char* g = take(bt > bk ? bt : bk);
+        const size_t bc = (l.mw * 128 + 16 * osd_h_terms(l.mw)) * sizeof(float);  // nibble sums, 16 warps' terms
+        const size_t most = bt > bk ? bt : bk;
+        unsigned char* g = take(most > bc ? most : bc);
         t.T = reinterpret_cast<uint32_t*>(g);
         t.keys = reinterpret_cast<unsigned long long*>(g);
     }
@@ -104,19 +107,19 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
     t.row_of_col = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nmax) * 2));
     t.hard = reinterpret_cast<uint32_t*>(take((static_cast<size_t>(l.nmax) / 32 + 1) * 4));
     t.wv = reinterpret_cast<uint32_t*>(take(2 * kRound * 32 * 4));
-    t.hits = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(l.warps) * kHitsPerWarp * 4));
-    t.piv = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(l.mw) * 4));
+    t.rank = reinterpret_cast<int16_t*>(take(rows * 2));
+    t.tidx = reinterpret_cast<uint8_t*>(take(rows));
     t.order = reinterpret_cast<int16_t*>(take(rows * 2));
     t.syn = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(l.mw) * 4));
     t.pivj = reinterpret_cast<int16_t*>(take(rows * 2));
     t.mrb = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nmax) * 2));
     t.pool_j = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.poolmax) * 2));
     {  // the tables of the elimination, then the vectors of the candidate search
-        const size_t b_vs = a16((static_cast<size_t>(l.poolmax) + 1) * 32 * 4);
+        const size_t b_vs = a16((static_cast<size_t>(l.poolmax) + 1) * l.mw * 4);
         const size_t b_avec = a16(static_cast<size_t>(l.poolmax) * l.mw * 4);
         const size_t b_aug = a16(static_cast<size_t>(l.mw) * 4);
         const size_t b_relq = a16(rows * 4);
-        const size_t b_vec = b_vs + b_avec + b_aug + b_relq, b_tab = 2 * 32 * 33 * 4;
+        const size_t b_vec = b_vs + b_avec + b_aug + b_relq, b_tab = 32 * kTabStride * 4;
         unsigned char* g = take(b_vec > b_tab ? b_vec : b_tab);
         t.tab = reinterpret_cast<uint32_t*>(g);
         t.vs = reinterpret_cast<uint32_t*>(g);
@@ -131,16 +134,13 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
 
 __device__ __forceinline__ unsigned tbit(const uint32_t* row, int q) { return (row[q >> 5] >> (q & 31)) & 1u; }
 
-// Slot of column q of T.  The columns a pivot touches come in runs of
-// consecutive rows (the parity part of these codes is a chain); a transposed
-// placement spreads a run over the 32-column chunks, hence over the warps
-// that apply the pivot, instead of loading one warp with the whole run.
-__device__ __forceinline__ int tslot(int q, int mw) { return (q & 31) * mw + (q >> 5); }
+// CTAs per SM the registers are bounded for (shared memory sets the same or less).
+constexpr int osd_h_ctas(int threads) { return threads == 128 ? 5 : threads == 256 ? 2 : 1; }
 
 }  // namespace
 
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, osd_h_ctas(kThreads))
 osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
 {
     constexpr int kWarps = kThreads / 32;
@@ -149,7 +149,9 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
     carve(lay, smem_raw, &s);
     __shared__ int s_rp[2][kRound];
     __shared__ int s_np[2], s_used[2], s_jstop[2];
+    __shared__ unsigned s_found[2];  // the round's candidates that gave a pivot
     __shared__ unsigned long long s_best;
+    __shared__ unsigned s_least;  // the least estimated metric (bits)
     __shared__ int s_item;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int TS = lay.ts;
@@ -233,11 +235,8 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             s.rel[j] = __uint_as_float(0x7fffffffu - static_cast<unsigned>(key >> 32));
         }
         __syncthreads();  // T overwrites the keys
-        // ---- 2. T = identity (column-major), syndrome of the hard decisions ----
-        for (int i = tid; i < rows * TS; i += kThreads) s.T[i] = 0u;
-        __syncthreads();
-        for (int col = tid; col < m; col += kThreads)
-            s.T[static_cast<size_t>(tslot(col, MW)) * TS + (col >> 5)] = 1u << (col & 31);
+        // ---- 2. no row pivoted yet, syndrome of the hard decisions ----
+        for (int r = tid; r < rows; r += kThreads) s.rank[r] = -1;
         for (int r = tid; r < rows; r += kThreads) {
             unsigned par = 0;
             if (r < m)
@@ -245,16 +244,14 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             const unsigned b = __ballot_sync(0xffffffffu, par);
             if (lane == 0) s.syn[r >> 5] = b;
         }
-        for (int w = tid; w < MW; w += kThreads) s.piv[w] = 0u;
         // column of H at each sorted position: first edge << 8 | weight
         const bool staged = lay.nnzmax > 0;
         if (staged)
             for (int e = tid; e < hv.col_ptr[n]; e += kThreads) s.rows[e] = static_cast<int16_t>(hv.col_rows[e]);
-        int* colinfo = s.colinfo;
         for (int j = tid; j < n; j += kThreads) {
             const int c = s.perm[j];
             const int e0 = hv.col_ptr[c];
-            colinfo[j] = (e0 << 8) | (hv.col_ptr[c + 1] - e0);
+            s.colinfo[j] = (e0 << 8) | (hv.col_ptr[c + 1] - e0);
         }
         __syncthreads();
 
@@ -263,107 +260,135 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
         // h_c selects); its pivot is the lowest unpivoted row p with v_p = 1, and
         // the pivot's row operation T <- (I + W e_p^T) T, W = v + e_p, turns
         // column c into e_p and leaves earlier pivot columns alone.
-        // Columns are taken kRound at a time, in rounds pipelined over one
-        // barrier each.  In the barrier interval of round k:
-        //   * warp 0 takes round k's candidates (reduced against T before
-        //     round k-1), applies round k-1's operation to them, and picks
-        //     their pivots in order; each pivot's operation is applied at once
-        //     to the later candidates and to the round's basis,
-        //       a -> a + sum_r a_{p_r} U_r,  U_r <- U_r + U_r[p] W for a new pivot p
-        //     (a_{p_r} a column's bits before the round, U_r = 0 for a dependent
-        //     candidate);
-        //   * warps 1..15 tabulate round k-1's basis by index nibble, and the
-        //     worker warps apply round k-1's operation to the columns of T they
-        //     own (the pivot-row bits of a column form its index; columns with a
-        //     nonzero index take its two table entries), meet on a named
-        //     barrier, and kRound of them reduce round k+1's candidates against
-        //     T.  In 512-thread CTAs (m > 640, the update bounds the round) the
-        //     workers are warps 1..15; in 256-thread CTAs (the selection bounds
-        //     it) warp 0 keeps its scheduler (warps w = 0 mod 4) to itself and
-        //     the workers are the warps w != 0 mod 4.
-        auto rows_of = [&](int jj, int& e0, int& cnt) -> int {  // one row of column jj per lane
-            const int ci = colinfo[jj];
-            e0 = ci >> 8;
-            cnt = ci & 255;
-            return lane < cnt ? (staged ? static_cast<int>(s.rows[e0 + lane]) : hv.col_rows[e0 + lane]) : -1;
-        };
-        auto reduce_column = [&](int myrow, int e0, int cnt) -> unsigned {  // T h_c, word `lane`
-            unsigned v = 0u;
-            for (int e = 0; e < cnt && e < 32; e += 8) {  // groups of 8 loads in flight together
-                unsigned part[8];
-#pragma unroll
-                for (int x = 0; x < 8; ++x) {
-                    const int q = __shfl_sync(0xffffffffu, myrow, (e + x) & 31);
-                    part[x] = (e + x < cnt && lane < MW) ? s.T[static_cast<size_t>(tslot(q, MW)) * TS + lane] : 0u;
-                }
-                v ^= (part[0] ^ part[1]) ^ (part[2] ^ part[3]) ^ (part[4] ^ part[5]) ^ (part[6] ^ part[7]);
-            }
-            for (int e = 32; e < cnt; ++e)  // columns heavier than 32
-                if (lane < MW) v ^= s.T[static_cast<size_t>(tslot(hv.col_rows[e0 + e], MW)) * TS + lane];
-            return v;
-        };
-        // candidate slot r of buffer b: rows + b * kRound + r
-        auto reduce_candidate = [&](int jj, int slot) {
+        // Columns are taken kRound at a time.  Interval k of the pipeline:
+        //   1. all warps: tabulate round k-1's basis U by index nibble, note its pivots, gather the
+        //      stored columns' bits at its pivot rows (their indices), and apply its operation to
+        //      round k's candidates (a warp each);
+        //   2. warp 0 picks round k's pivots in order; each pivot's operation is applied at once to
+        //      the later candidates and to the round's basis,
+        //        a -> a + sum_r a_{p_r} U_r,  U_r <- U_r + U_r[p] W for a new pivot p
+        //      (a_{p_r} a column's bits before the round, U_r = 0 for a dependent candidate);
+        //      the other warps apply round k-1's operation to the stored columns of T (one thread
+        //      per column, two table entries per word), append
+        //      the columns of its pivot rows (e_p + U_p), meet on a named barrier and reduce round
+        //      k+1's candidates against T.
+        auto reduce_candidate = [&](int jj, uint32_t* dst) {  // T h_c of the column at position jj, word `lane`
             unsigned v = 0u;
             if (jj >= 0) {
-                int e0, cnt;
-                const int rw = rows_of(jj, e0, cnt);
-                v = reduce_column(rw, e0, cnt);
+                const int ci = s.colinfo[jj], e0 = ci >> 8, cnt = ci & 255;
+                // lane e: row of the column's e-th one (none: a row no lane holds), and that row's
+                // column's place in T (-1: a unit vector)
+                int mine = (2047 << 16) | 0xffff;
+                if (lane < cnt) {
+                    const int q = staged ? static_cast<int>(s.rows[e0 + lane]) : hv.col_rows[e0 + lane];
+                    mine = (q << 16) | static_cast<uint16_t>(s.rank[q]);
+                }
+                // the word of row u >> 16's column of T: loaded whether or not it is stored (place 0
+                // then), so that no branch stands between the loads of a group
+                auto word = [&](int u) -> unsigned {
+                    const int at = static_cast<int16_t>(u & 0xffff), row = u >> 16;
+                    const unsigned x = s.T[max(at, 0) * TS + lane];
+                    return at >= 0 ? x : lane == (row >> 5) ? 1u << (row & 31) : 0u;
+                };
+                for (int e = 0; e < cnt && e < 32; e += 4) {
+                    unsigned part[4];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) part[x] = word(__shfl_sync(0xffffffffu, mine, (e + x) & 31));
+                    v ^= (part[0] ^ part[1]) ^ (part[2] ^ part[3]);
+                }
+                for (int e = 32; e < cnt; ++e) {  // columns heavier than 32
+                    const int row = hv.col_rows[e0 + e];
+                    v ^= word((row << 16) | static_cast<uint16_t>(s.rank[row]));
+                }
             }
-            if (lane < MW) s.T[static_cast<size_t>(slot) * TS + lane] = v;
+            if (lane < MW) dst[lane] = v;
         };
-        for (int c = warp; c < kRound; c += kWarps) reduce_candidate(n - 1 - c, rows + c);
+        // candidate c of buffer b
+        auto candidate = [&](int b, int c) -> uint32_t* { return s.T + (rows + b * kRound + c) * TS; };
+        for (int c = warp; c < kRound; c += kWarps) reduce_candidate(n - 1 - c, candidate(0, c));
         __syncthreads();
-        const int lg = MW <= 1 ? 0 : 32 - __clz(MW - 1);  // table words per entry: 2^lg >= MW
-        uint32_t* seg = s.hits + warp * kHitsPerWarp;
-        constexpr bool narrow = kThreads < 512;  // the small-T classes: selection-bound
-        const int nworkers = narrow ? kWarps - kWarps / 4 : kWarps - 1;
-        const bool worker = warp != 0 && (!narrow || (warp & 3) != 0);
-        const int wi = narrow ? warp - (warp >> 2) - 1 : warp - 1;  // worker index
         int t = 0, j = n - 1, nd = 0, jstop = -1;          // after the rounds selected so far
         int pt = 0, pj = 0, pnd = 0, pnp = 0, pused = 0;   // the round whose update is pending
         bool pending = false;
         unsigned pivw = 0u;  // warp 0: pivoted rows, word `lane`
-        unsigned Up[kRound];  // warp 0: the pending round's basis, and its pivot rows as word offset + bit
-        int pwo[kRound];
-        unsigned pwb[kRound];
-#pragma unroll
-        for (int r = 0; r < kRound; ++r) {
-            Up[r] = 0u;
-            pwo[r] = 0;
-            pwb[r] = 0u;
-        }
         for (int k = 0;; ++k) {
             const bool select = j >= 0 && t < m;
             if (!select && !pending) break;
-            const int cb = k & 1;
-            if (warp == 0) {
-                if (select) {
-                    // branch-free, so that the loads and the candidates' chains overlap
-                    unsigned v[kRound], U[kRound];
-                    int P[kRound];
+            const int cb = k & 1, pb = cb ^ 1;
+            if (pending) {
+                const uint32_t* U = s.wv + pb * kRound * 32;
+                if (pnp > 0) {
+                    // tables of the pending round's basis, one index nibble per warp, word `lane`
+                    if (warp >= kWarps - 2 && lane < MW) {
+                        const int h = warp - (kWarps - 2);
+                        uint32_t* tb = s.tab + h * 16 * kTabStride + lane;
+                        unsigned u[4], acc[16];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) u[b] = U[(h * 4 + b) * 32 + lane];
+                        acc[0] = 0u;
+#pragma unroll
+                        for (int e = 1; e < 16; ++e) {
+                            const int low = (e & 1) ? 0 : (e & 2) ? 1 : (e & 4) ? 2 : 3;
+                            acc[e] = acc[e & (e - 1)] ^ u[low];
+                        }
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) tb[e * kTabStride] = acc[e];
+                    }
+                    // every stored column's index into them
+                    int woff[kRound];
+                    unsigned wbit[kRound];
 #pragma unroll
                     for (int r = 0; r < kRound; ++r) {
-                        v[r] = lane < MW ? s.T[static_cast<size_t>(rows + cb * kRound + r) * TS + lane] : 0u;
-                        U[r] = 0u;
-                        P[r] = -1;
+                        const int p = s_rp[pb][r];
+                        woff[r] = p >= 0 ? p >> 5 : 0;
+                        wbit[r] = p >= 0 ? 1u << (p & 31) : 0u;
                     }
-                    {  // the previous round's operation, not yet in the reduced candidates (a no-op in round 0)
-                        // lane l: candidate l mod kRound's bits at that round's pivot rows
-                        const uint32_t* col = s.T + static_cast<size_t>(rows + cb * kRound + (lane & (kRound - 1))) * TS;
+                    for (int at = tid; at < pt; at += kThreads) {
+                        const uint32_t* c = s.T + at * TS;
                         unsigned idx = 0u;
 #pragma unroll
-                        for (int i = 0; i < kRound; ++i)
-                            if (col[pwo[i]] & pwb[i]) idx |= 1u << i;
+                        for (int r = 0; r < kRound; ++r)
+                            if (c[woff[r]] & wbit[r]) idx |= 1u << r;
+                        s.tidx[at] = static_cast<uint8_t>(idx);
+                    }
+                    // the pending operation on this round's candidates, not in them yet
+                    if (select)
+                        for (int c = warp; c < kRound; c += kWarps) {
+                            uint32_t* col = candidate(cb, c);
+                            const int p = lane < kRound ? s_rp[pb][lane] : -1;
+                            const unsigned idx = __ballot_sync(0xffffffffu, p >= 0 && ((col[p >> 5] >> (p & 31)) & 1u));
+                            unsigned v = lane < MW ? col[lane] : 0u;
 #pragma unroll
-                        for (int r = 0; r < kRound; ++r) {
-                            const unsigned ir = __shfl_sync(0xffffffffu, idx, r);
-#pragma unroll
-                            for (int i = 0; i < kRound; ++i) v[r] ^= ((ir >> i) & 1u) ? Up[i] : 0u;
+                            for (int r = 0; r < kRound; ++r) v ^= U[r * 32 + lane] & (0u - ((idx >> r) & 1u));
+                            if (lane < MW) col[lane] = v;
                         }
+                }
+                if (warp == kWarps - 3 && lane < pused) {  // pivot ranks and dependent positions
+                    const int pr = s_rp[pb][lane];
+                    const unsigned found = s_found[pb], below = (1u << lane) - 1u;
+                    if (pr >= 0) {
+                        const int rk = pt + __popc(found & below);
+                        s.order[rk] = static_cast<int16_t>(pr);
+                        s.rank[pr] = static_cast<int16_t>(rk);
+                        s.row_of_col[s.perm[pj - lane]] = static_cast<int16_t>(rk);
+                        s.pivj[rk] = static_cast<int16_t>(pj - lane);
+                    } else {
+                        s.mrb[pnd + __popc(~found & below)] = static_cast<int16_t>(pj - lane);  // an MRB position
+                    }
+                }
+                __syncthreads();
+            }
+            if (warp == 0) {
+                if (select) {
+                    unsigned v[kRound], U[kRound];
+#pragma unroll
+                    for (int r = 0; r < kRound; ++r) {
+                        v[r] = lane < MW ? candidate(cb, r)[lane] : 0u;
+                        U[r] = 0u;
                     }
                     int np = 0, used = 0, js = -1;
-                    int pl[kRound];  // the pivot's position on its lane, -1 elsewhere
+                    unsigned found = 0u;
+                    int pl[kRound];  // the pivot's row + 1 on its lane, 0 elsewhere
 #pragma unroll
                     for (int r = 0; r < kRound; ++r) {
                         const bool valid = j - r >= 0 && t + np < m;  // warp-uniform
@@ -372,17 +397,19 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                         // each lane's row are balloted at once, before the pivot lane is known, so
                         // the chain from one candidate to the next is one ballot deep: the pivot
                         // lane's bit of each ballot is that vector's bit at the pivot row.
+                        used = valid ? r + 1 : used;
                         const unsigned x = valid ? (v[r] & ~pivw) : 0u;
-                        const unsigned lb = x & (0u - x);
                         const unsigned bx = __ballot_sync(0xffffffffu, x != 0u);
+                        pl[r] = 0;
+                        if (bx == 0u) continue;  // dependent: a third or more of the columns scanned
+                        const unsigned lb = x & (0u - x);
                         unsigned bc[kRound];
 #pragma unroll
                         for (int c = 0; c < kRound; ++c)
                             bc[c] = c > r   ? __ballot_sync(0xffffffffu, (v[c] & lb) != 0u)
                                     : c < r ? __ballot_sync(0xffffffffu, (U[c] & lb) != 0u)
                                             : 0u;
-                        const bool piv = bx != 0u;
-                        const unsigned sel = bx & (0u - bx);  // the pivot lane's bit (0: no pivot)
+                        const unsigned sel = bx & (0u - bx);  // the pivot lane's bit
                         const bool me = (sel >> lane) & 1u;
                         const unsigned W = me ? (v[r] ^ lb) : v[r];
 #pragma unroll
@@ -390,125 +417,67 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                             if (c > r) v[c] ^= (bc[c] & sel) ? W : 0u;
                             if (c < r) U[c] ^= (bc[c] & sel) ? W : 0u;
                         }
-                        U[r] = piv ? W : 0u;
-                        pl[r] = me ? lane * 32 + __ffs(lb) - 1 : -1;
+                        U[r] = W;
+                        pl[r] = me ? lane * 32 + __ffs(lb) : 0;
                         pivw |= me ? lb : 0u;
-                        np += piv ? 1 : 0;
-                        js = (piv && t + np == m) ? j - r : js;
-                        used = valid ? r + 1 : used;
+                        ++np;
+                        found |= 1u << r;
+                        js = t + np == m ? j - r : js;
                     }
+#pragma unroll
+                    for (int r = 0; r < kRound; ++r) s.wv[(cb * kRound + r) * 32 + lane] = U[r];
+                    if (lane < kRound) s_rp[cb][lane] = -1;
+                    __syncwarp();
 #pragma unroll
                     for (int r = 0; r < kRound; ++r)
-                        P[r] = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(pl[r] + 1))) - 1;
-#pragma unroll
-                    for (int r = 0; r < kRound; ++r) {  // every lane stores (same values): no divergence
-                        s.wv[(cb * kRound + r) * 32 + lane] = U[r];
-                        s_rp[cb][r] = P[r];
-                        Up[r] = U[r];
-                        pwo[r] = P[r] >= 0 ? P[r] >> 5 : 0;
-                        pwb[r] = P[r] >= 0 ? 1u << (P[r] & 31) : 0u;
+                        if (pl[r] > 0) s_rp[cb][r] = pl[r] - 1;
+                    if (lane == 0) {
+                        s_np[cb] = np;
+                        s_found[cb] = found;
+                        s_used[cb] = used;
+                        s_jstop[cb] = js;
                     }
-                    s_np[cb] = np;
-                    s_used[cb] = used;
-                    s_jstop[cb] = js;
                 }
             } else {
-                if (pending) {
-                    const int pb = cb ^ 1;
-                    if (pnp > 0) {  // tables of the pending round's basis (entries 0 and 16 are 0)
-                        uint32_t* tb = s.tab + pb * 32 * kTabStride;
-                        const uint32_t* U = s.wv + pb * kRound * 32;
-                        for (int q = tid - 32; q < (32 << lg); q += kThreads - 32) {
-                            const int e = q >> lg, w = q & ((1 << lg) - 1), h = (e >> 4) * 4;
-                            unsigned acc = 0u;
-#pragma unroll
-                            for (int b = 0; b < 4; ++b)
-                                if ((e >> b) & 1) acc ^= U[(h + b) * 32 + w];
-                            tb[e * kTabStride + w] = acc;
+                if (pending && pnp > 0) {
+                    // a warp takes 32 columns, and above 16 words a half of their words: smaller pieces
+                    // share out better (three loads and a store per word: shared-memory bandwidth
+                    // bounds this at m = 1024)
+                    const int halves = MW > 16 ? 2 : 1, per = (MW / halves + 3) & ~3;
+                    for (int piece = warp - 1; piece < ((pt + 31) >> 5) * halves; piece += kWarps - 1) {
+                        const int at = (halves == 2 ? piece >> 1 : piece) * 32 + lane;
+                        const int w0 = halves == 2 ? (piece & 1) * per : 0, w1 = min(MW, w0 + per);
+                        if (at >= pt) continue;
+                        uint32_t* c = s.T + at * TS;
+                        const unsigned idx = s.tidx[at];
+                        if (idx == 0u) continue;
+                        const uint32_t* lo = s.tab + (idx & 15u) * kTabStride;
+                        const uint32_t* hi = s.tab + (16u + (idx >> 4)) * kTabStride;
+                        int w = w0;
+                        for (; w + 4 <= w1; w += 4) {
+                            const unsigned a0 = c[w] ^ lo[w] ^ hi[w];
+                            const unsigned a1 = c[w + 1] ^ lo[w + 1] ^ hi[w + 1];
+                            const unsigned a2 = c[w + 2] ^ lo[w + 2] ^ hi[w + 2];
+                            const unsigned a3 = c[w + 3] ^ lo[w + 3] ^ hi[w + 3];
+                            c[w] = a0;
+                            c[w + 1] = a1;
+                            c[w + 2] = a2;
+                            c[w + 3] = a3;
                         }
-                        asm volatile("bar.sync 1, %0;" ::"r"(kThreads - 32) : "memory");
+                        for (; w < w1; ++w) c[w] ^= lo[w] ^ hi[w];
                     }
-                    int P[kRound];
-#pragma unroll
-                    for (int r = 0; r < kRound; ++r) P[r] = s_rp[pb][r];
-                    if (warp == kWarps - 1 && lane < pused) {  // pivot ranks and dependent positions
-                        int bp = 0, bd = 0, pr = -1;
-#pragma unroll
-                        for (int r = 0; r < kRound; ++r) {
-                            if (r < lane) {
-                                if (P[r] >= 0) ++bp;
-                                else ++bd;
-                            }
-                            if (r == lane) pr = P[r];
-                        }
-                        if (pr >= 0) {
-                            s.order[pt + bp] = static_cast<int16_t>(pr);
-                            s.row_of_col[s.perm[pj - lane]] = static_cast<int16_t>(pt + bp);
-                            s.pivj[pt + bp] = static_cast<int16_t>(pj - lane);
-                        } else {
-                            s.mrb[pnd + bd] = static_cast<int16_t>(pj - lane);  // dependent: an MRB position
-                        }
-                    }
-                    if (pnp > 0 && worker) {
-                        // gather: one thread per owned column, the touched ones listed; then one
-                        // thread per listed column walks its MW words (three loads, one store each)
-                        const uint32_t* tb = s.tab + pb * 32 * kTabStride;
-                        int woff[kRound];
-                        unsigned wbit[kRound];
-#pragma unroll
-                        for (int r = 0; r < kRound; ++r) {
-                            woff[r] = P[r] >= 0 ? P[r] >> 5 : 0;
-                            wbit[r] = P[r] >= 0 ? 1u << (P[r] & 31) : 0u;
-                        }
-                        auto walk = [&](int nh) {
-                            __syncwarp();
-                            for (int h = lane; h < nh; h += 32) {
-                                const unsigned e = seg[h];
-                                uint32_t* c = s.T + (e & 0xffffu);
-                                const unsigned idx = e >> 16;
-                                const uint32_t* lo = tb + (idx & 15u) * kTabStride;
-                                const uint32_t* hi = tb + (16u + (idx >> 4)) * kTabStride;
-                                int w = 0;
-                                for (; w + 4 <= MW; w += 4) {
-                                    const unsigned a0 = c[w] ^ lo[w] ^ hi[w];
-                                    const unsigned a1 = c[w + 1] ^ lo[w + 1] ^ hi[w + 1];
-                                    const unsigned a2 = c[w + 2] ^ lo[w + 2] ^ hi[w + 2];
-                                    const unsigned a3 = c[w + 3] ^ lo[w + 3] ^ hi[w + 3];
-                                    c[w] = a0;
-                                    c[w + 1] = a1;
-                                    c[w + 2] = a2;
-                                    c[w + 3] = a3;
-                                }
-                                for (; w < MW; ++w) c[w] ^= lo[w] ^ hi[w];
-                            }
-                            __syncwarp();  // the list is rewritten next
-                        };
-                        int nh = 0;
-                        for (int b0 = wi * 32; b0 < rows; b0 += nworkers * 32) {
-                            if (nh > kHitsPerWarp - 32) {  // the list is full: apply it first
-                                walk(nh);
-                                nh = 0;
-                            }
-                            const int slot = b0 + lane;
-                            unsigned idx = 0u;
-                            if (slot < rows) {
-                                const uint32_t* col = s.T + slot * TS;
-#pragma unroll
-                                for (int r = 0; r < kRound; ++r)
-                                    if (col[woff[r]] & wbit[r]) idx |= 1u << r;
-                            }
-                            const unsigned bal = __ballot_sync(0xffffffffu, idx != 0u);
-                            if (idx) seg[nh + __popc(bal & ((1u << lane) - 1u))] = static_cast<unsigned>(slot * TS) | (idx << 16);
-                            nh += __popc(bal);
-                        }
-                        walk(nh);
+                    for (int r = warp - 1; r < kRound; r += kWarps - 1) {  // the pivot rows' columns: e_p + U_p
+                        const int p = s_rp[pb][r];
+                        if (p >= 0 && lane < MW)
+                            s.T[(pt + __popc(s_found[pb] & ((1u << r) - 1u))) * TS + lane] =
+                                s.wv[(pb * kRound + r) * 32 + lane] ^ (lane == (p >> 5) ? 1u << (p & 31) : 0u);
                     }
                 }
                 // T is final for the pending round before the next candidates read it
                 asm volatile("bar.sync 1, %0;" ::"r"(kThreads - 32) : "memory");
-                if (select && worker)
-                    for (int c = wi; c < kRound; c += nworkers)
-                        reduce_candidate(j - kRound - c, rows + (cb ^ 1) * kRound + c);
+                if (select)
+                    for (int c = warp - 1; c < kRound; c += kWarps - 1)
+                        reduce_candidate(j - kRound - c, candidate(cb ^ 1, c));
             }
             __syncthreads();
             pending = select;
@@ -563,23 +532,22 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
 
         // ---- 5. T s and the reduced pool columns, then in pivot order ----
         const int pool = hv.pool;
-        for (int i = tid; i < (pool + 1) * 32; i += kThreads) s.vs[i] = 0u;
+        for (int i = tid; i < (pool + 1) * MW; i += kThreads) s.vs[i] = 0u;
         __syncthreads();
         {
             // T s: XOR of the columns of T selected by s, spread over the warps
             unsigned acc = 0u;
-            for (int q = warp; q < m; q += kWarps)
-                if (lane < MW && tbit(s.syn, q)) acc ^= s.T[static_cast<size_t>(tslot(q, MW)) * TS + lane];
+            for (int q0 = warp; q0 < m; q0 += 4 * kWarps) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int q = min(q0 + x * kWarps, m - 1);
+                    const unsigned on = q0 + x * kWarps < m ? tbit(s.syn, q) : 0u;
+                    acc ^= s.T[s.rank[q] * TS + lane] & (0u - on);
+                }
+            }
             if (lane < MW && acc) atomicXor(&s.vs[lane], acc);
             // T h_f for the flip pool, one warp per column
-            for (int i = warp; i < pool; i += kWarps) {
-                const int c = s.perm[s.pool_j[i]];
-                unsigned v = 0u;
-                if (lane < MW)
-                    for (int e = hv.col_ptr[c]; e < hv.col_ptr[c + 1]; ++e)
-                        v ^= s.T[static_cast<size_t>(tslot(hv.col_rows[e], MW)) * TS + lane];
-                if (lane < MW) s.vs[(i + 1) * 32 + lane] = v;
-            }
+            for (int i = warp; i < pool; i += kWarps) reduce_candidate(s.pool_j[i], s.vs + (i + 1) * MW);
         }
         __syncthreads();
         // bit t of an ordered vector = bit order[t] of the row-indexed one (8 vectors' loads in flight)
@@ -590,7 +558,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             for (int v0 = 0; v0 <= pool; v0 += 8) {
                 unsigned bits[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) bits[u] = v0 + u <= pool ? s.vs[(v0 + u) * 32 + qw] & qb : 0u;
+                for (int u = 0; u < 8; ++u) bits[u] = v0 + u <= pool ? s.vs[(v0 + u) * MW + qw] & qb : 0u;
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const unsigned b = __ballot_sync(0xffffffffu, bits[u] != 0u);
@@ -600,94 +568,145 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             }
         }
         for (int r = tid; r < rows; r += kThreads) s.relq[r] = r < m ? s.rel[s.pivj[r]] : 0.0f;
+        if (tid == 0) s_least = 0x7f800000u;
         __syncthreads();
-
-        // ---- 6. candidates: metric in increasing sorted position, exact pruning ----
-        // Bit t of T s (+ T h_f) marks a differing pivot position; pivot ranks in descending
-        // order hold the positions in ascending order, so the metric walks the bits from the
-        // top.  A flipped position f joins the sum before the first rank t < cut(f), the
-        // number of pivots after it.  Four set bits are taken at a time, their |llr| loaded
-        // together; the additions stay in order.
-        for (int ti = tid; ti < hv.num_tests; ti += kThreads) {
-            int fa = -1, fb = -1, fc = -1;  // pool indices of the flips
+        // ---- 6. candidates ----
+        // Bit t of T s (+ T h_f) marks a differing pivot position; pivot ranks in descending order
+        // hold the positions in ascending order, the order of the metric's sum.  A flipped position f
+        // joins the sum before the first rank t < cut(f), the number of pivots after it.
+        // Every test meets an estimate of its metric first: its differing pivot positions summed
+        // from tables of |llr| sums by nibble (in T's place, which is done with), plus its flips.
+        // Estimate and in-order sum are both within 650 rounding units (1,027 terms, 262 additions)
+        // of the exact sum, so a test whose estimate is over the least estimate seen by a factor
+        // 1 + 2^-12 (4,096 units) cannot win.  The few others are summed in order, a warp each: its
+        // lanes lay the terms out in order, one adds them up.
+        float* nib = reinterpret_cast<float*>(s.T);                         // [8 MW][16]
+        float* terms = nib + MW * 128 + warp * osd_h_terms(MW);             // this warp's terms in order
+        for (int e = tid; e < MW * 128; e += kThreads) {
+            const float* r4 = s.relq + (e >> 4) * 4;
+            float x = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if ((e >> i) & 1) x += r4[i];
+            nib[e] = x;
+        }
+        __syncthreads();
+        struct Test {
+            int f[3];          // pool indices of the flips, -1 for none
+            int j[3];          // their positions, ascending (absent: INT_MAX)
+        };
+        auto test_at = [&](int ti) -> Test {
+            Test q{{-1, -1, -1}, {INT_MAX, INT_MAX, INT_MAX}};
             if (ti > 0) {
                 const uint32_t pk = hv.combos[ti - 1];
-                const int f0 = pk & 1023, f1 = (pk >> 10) & 1023, f2 = (pk >> 20) & 1023;
-                fa = f0 != 1023 ? f0 : -1;
-                fb = f1 != 1023 ? f1 : -1;
-                fc = f2 != 1023 ? f2 : -1;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int f = (pk >> (10 * i)) & 1023;
+                    q.f[i] = f != 1023 ? f : -1;
+                    q.j[i] = f != 1023 ? s.pool_j[f] : INT_MAX;
+                }
             }
-            // flip positions ascending (absent: INT_MAX), their |llr| and cuts
-            int j0 = fa >= 0 ? s.pool_j[fa] : INT_MAX, j1 = fb >= 0 ? s.pool_j[fb] : INT_MAX,
-                j2 = fc >= 0 ? s.pool_j[fc] : INT_MAX;
-            if (j0 > j1) { const int z = j0; j0 = j1; j1 = z; }
-            if (j1 > j2) { const int z = j1; j1 = j2; j2 = z; }
-            if (j0 > j1) { const int z = j0; j0 = j1; j1 = z; }
-            auto cut_of = [&](int jf) -> int {  // pivots at positions above jf (pivj decreases with rank)
-                if (jf == INT_MAX) return -1;
+            auto order2 = [&](int a, int b) {
+                const int lo = min(q.j[a], q.j[b]), hi = max(q.j[a], q.j[b]);
+                q.j[a] = lo;
+                q.j[b] = hi;
+            };
+            order2(0, 1);
+            order2(1, 2);
+            order2(0, 1);
+            return q;
+        };
+        auto word_at = [&](const Test& q, int w) -> unsigned {
+            unsigned word = s.aug[w];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                if (q.f[i] >= 0) word ^= s.avec[q.f[i] * MW + w];
+            return word;
+        };
+        auto estimate = [&](const Test& q) -> float {
+            float part[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                if (q.j[i] != INT_MAX) part[0] += s.rel[q.j[i]];
+            for (int w = 0; w < MW; ++w) {
+                const unsigned word = word_at(q, w);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part[i & 1] += nib[(w * 8 + i) * 16 + ((word >> (4 * i)) & 15u)];
+            }
+            return part[0] + part[1];
+        };
+        auto note = [&](float est) {  // lower the least estimate by this warp's
+            const unsigned least = __reduce_min_sync(0xffffffffu, __float_as_uint(est));
+            if (lane == 0 && least < *reinterpret_cast<volatile unsigned*>(&s_least)) atomicMin(&s_least, least);
+        };
+        auto in_order = [&](int ti) {  // the whole warp: the metric of test ti, kept if the best
+            const Test q = test_at(ti);
+            const unsigned word = lane < MW ? word_at(q, lane) : 0u;
+            int above = __popc(word);  // set bits in this word and the later ones, then in the later ones
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_down_sync(0xffffffffu, above, o);
+                if (lane + o < 32) above += x;
+            }
+            const int total_bits = __shfl_sync(0xffffffffu, above, 0);
+            above -= __popc(word);
+            int cut[3], flips = 0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {  // pivots at positions above the flip's (pivj decreases with rank)
+                cut[i] = -1;
+                if (q.j[i] == INT_MAX) continue;
                 int lo = 0, hi = m;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if (s.pivj[mid] > jf) lo = mid + 1;
+                    if (s.pivj[mid] > q.j[i]) lo = mid + 1;
                     else hi = mid;
                 }
-                return lo;
-            };
-            const int c0 = cut_of(j0), c1 = cut_of(j1), c2 = cut_of(j2);
-            const float r0 = j0 != INT_MAX ? s.rel[j0] : 0.0f, r1 = j1 != INT_MAX ? s.rel[j1] : 0.0f,
-                        r2 = j2 != INT_MAX ? s.rel[j2] : 0.0f;
-            {  // the flipped positions' own sum (in position order) bounds the metric from below
-                const float lb = __fadd_rn(__fadd_rn(r0, r1), r2);
-                const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_best);
-                if (cur != ~0ull && lb > __uint_as_float(static_cast<unsigned>(cur >> 32))) continue;
+                cut[i] = lo;
+                // its place: after the differing pivots of rank >= cut and the flips before it
+                const int c = lo - 32 * lane;  // bits c .. 31 of this word have rank >= cut
+                const unsigned later = c <= 0 ? word : c >= 32 ? 0u : word & ~((1u << c) - 1u);
+                const int at = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(__popc(later)))) + i;
+                if (lane == 0) terms[at] = s.rel[q.j[i]];
+                ++flips;
             }
-            int fi = 0;  // flips added so far
-            int ncut = c0;
-            float nrel = r0;
-            const uint32_t* va = fa >= 0 ? s.avec + fa * MW : nullptr;
-            const uint32_t* vb = fb >= 0 ? s.avec + fb * MW : nullptr;
-            const uint32_t* vc = fc >= 0 ? s.avec + fc * MW : nullptr;
-            float acc = 0.0f;
-            bool pruned = false;
-            for (int w = MW - 1; w >= 0 && !pruned; --w) {
-                unsigned word = s.aug[w];
-                if (va) word ^= va[w];
-                if (vb) word ^= vb[w];
-                if (vc) word ^= vc[w];
-                while (word) {
-                    int bq[4];
-                    float rq[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        bq[u] = word ? 31 - __clz(word) : -1;
-                        if (bq[u] >= 0) word &= ~(1u << bq[u]);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) rq[u] = bq[u] >= 0 ? s.relq[w * 32 + bq[u]] : 0.0f;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (bq[u] < 0) break;
-                        const int t = w * 32 + bq[u];
-                        while (t < ncut) {  // flipped positions below this pivot's
-                            acc = __fadd_rn(acc, nrel);
-                            ++fi;
-                            ncut = fi == 1 ? c1 : fi == 2 ? c2 : -1;
-                            nrel = fi == 1 ? r1 : r2;
-                        }
-                        acc = __fadd_rn(acc, rq[u]);
-                    }
+            for (unsigned left = word; left;) {
+                const int b = 31 - __clz(left), rank = 32 * lane + b;
+                left &= ~(1u << b);
+                terms[above + (cut[0] > rank) + (cut[1] > rank) + (cut[2] > rank)] = s.relq[rank];
+                ++above;
+            }
+            const int total = total_bits + flips;
+            if (lane < 4) terms[total + lane] = 0.0f;  // the last group of four adds zeros: no change
+            __syncwarp();
+            if (lane == 0) {
+                float acc = 0.0f;
+                for (int i = 0; i < total; i += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(terms + i);
+                    acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, x.x), x.y), x.z), x.w);
                 }
-                const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_best);
-                if (cur != ~0ull && acc > __uint_as_float(static_cast<unsigned>(cur >> 32))) pruned = true;
+                atomicMin(&s_best, (static_cast<unsigned long long>(__float_as_uint(acc)) << 32) | static_cast<unsigned>(ti));
             }
-            if (pruned) continue;
-            while (ncut >= 0) {  // flipped positions above every differing pivot position
-                acc = __fadd_rn(acc, nrel);
-                ++fi;
-                ncut = fi == 1 ? c1 : fi == 2 ? c2 : -1;
-                nrel = fi == 1 ? r1 : r2;
+            __syncwarp();  // the terms are rewritten by the next test
+        };
+        {
+            // a warp's first 32 tests are estimated before any is summed, so that those meet the least
+            // estimate of all the first tests
+            float first = INFINITY;
+            const int ti0 = warp * 32 + lane;
+            if (ti0 < hv.num_tests) first = estimate(test_at(ti0));
+            if (warp * 32 < hv.num_tests) note(first);
+            __syncthreads();
+            for (int t0 = warp * 32; t0 < hv.num_tests; t0 += kThreads) {
+                const int ti = t0 + lane;
+                float est = first;
+                if (t0 != warp * 32) {
+                    est = ti < hv.num_tests ? estimate(test_at(ti)) : INFINITY;
+                    note(est);
+                }
+                const float least = __uint_as_float(*reinterpret_cast<volatile unsigned*>(&s_least));
+                unsigned pass = __ballot_sync(0xffffffffu, ti < hv.num_tests && !(est > least * (1.0f + 2.44140625e-04f)));
+                for (; pass; pass &= pass - 1) in_order(t0 + __ffs(pass) - 1);
             }
-            atomicMin(&s_best, (static_cast<unsigned long long>(__float_as_uint(acc)) << 32) | static_cast<unsigned>(ti));
         }
         __syncthreads();
 
@@ -732,7 +751,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
 
 namespace {
 
-OsdHLayout osd_h_layout(const OsdHBounds& bd, int threads, int mlo, int mhi)
+OsdHLayout osd_h_layout(const OsdHBounds& bd, int mlo, int mhi)
 {
     OsdHLayout l{};
     l.nmax = bd.nmax;
@@ -741,7 +760,6 @@ OsdHLayout osd_h_layout(const OsdHBounds& bd, int threads, int mlo, int mhi)
     l.mw = (bd.mmax + 31) / 32;
     l.ts = l.mw | 1;
     l.poolmax = std::max(bd.poolmax, 1);
-    l.warps = threads / 32;
     l.mlo = mlo;
     l.mhi = mhi;
     l.nnzmax = 0;
@@ -754,13 +772,15 @@ void launch_osd_h_class(const OsdHBounds& bd, int mlo, int mhi, const OsdIO& io_
 {
     OsdIO io = io_all;  // the class's own work counter
     io.work_h = io_all.work_h ? io_all.work_h + cls : nullptr;
-    OsdHLayout l = osd_h_layout(bd, kThreads, mlo, mhi);
+    OsdHLayout l = osd_h_layout(bd, mlo, mhi);
     size_t smem = carve(l, nullptr, nullptr);
     if (smem > 227 * 1024) throw InvalidArgument("large-code OSD tables exceed shared memory (m <= 1024, n <= 4096)");
-    // stage the columns' row lists when they fit as well, and keep the class's CTAs per SM
-    const size_t per_sm_bytes = kThreads == 512 ? 227 * 1024 : 112 * 1024;  // two 256-thread CTAs per SM
+    // stage the columns' row lists when they cost no CTA per SM
+    constexpr size_t sm_bytes = 227 * 1024, reserved = 1024;  // the latter per CTA
+    const auto per_sm_by = [&](size_t bytes) { return std::min<size_t>(osd_h_ctas(kThreads), sm_bytes / (bytes + reserved)); };
     l.nnzmax = bd.nnzmax;
-    if (bd.nnzmax <= 0 || carve(l, nullptr, nullptr) > (smem <= per_sm_bytes ? per_sm_bytes : 227 * 1024)) l.nnzmax = 0;
+    if (bd.nnzmax <= 0 || carve(l, nullptr, nullptr) > 227 * 1024 || per_sm_by(carve(l, nullptr, nullptr)) < per_sm_by(smem))
+        l.nnzmax = 0;
     smem = carve(l, nullptr, nullptr);
     // the two 256-thread classes share this kernel with different sizes: the limit only grows
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(osd_h_kernel<kThreads>), smem),
@@ -788,8 +808,7 @@ size_t osd_h_smem_bytes(int nmax, int mmax, int poolmax)
 {  // without the staged row lists
     OsdHBounds bd;
     bd.add(nmax, mmax, poolmax, 0);
-    const int c = osd_h_class(mmax);
-    const OsdHLayout l = osd_h_layout(bd, kOsdHClassThreads[c], 0, 1024);
+    const OsdHLayout l = osd_h_layout(bd, 0, 1024);
     return carve(l, nullptr, nullptr);
 }
 
@@ -819,7 +838,8 @@ void launch_osd_h(const OsdHBounds* cls, const OsdIO& io, int max_items, cudaStr
             check_cuda(cudaStreamWaitEvent(cs, fork, 0), "cudaStreamWaitEvent(osd fork)");
         }
         const int mlo = c == 0 ? 0 : kOsdHClassMaxM[c - 1];
-        if (kOsdHClassThreads[c] == 256) launch_osd_h_class<256>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
+        if (kOsdHClassThreads[c] == 128) launch_osd_h_class<128>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
+        else if (kOsdHClassThreads[c] == 256) launch_osd_h_class<256>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
         else launch_osd_h_class<512>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
         if (fan && used > 0) {
             check_cuda(cudaEventRecord(join[used - 1], cs), "cudaEventRecord(osd join)");
