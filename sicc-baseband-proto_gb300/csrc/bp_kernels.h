@@ -59,16 +59,16 @@ void launch_osd(const OsdView& ov, const OsdIO& io, int max_items, cudaStream_t 
                 int ctas = 0);
 
 // OSD of long codes, one CTA per codeword (io.hviews for mixed batches, else
-// `hv`); nmax/mmax/poolmax/nnzmax (edges of H) bound the codes of the launch.
+// `hv`); nmax/mmax/poolmax bound the codes of the launch.
 // Launch bounds of the large-code OSD over a set of codes.
 struct OsdHBounds {
-    int nmax = 0, mmax = 0, poolmax = 0, nnzmax = 0;
-    void add(int n, int m, int pool, int nnz);
+    int nmax = 0, mmax = 0, poolmax = 0;
+    void add(int n, int m, int pool);
     bool empty() const { return nmax == 0; }
 };
-// The large-code OSD runs in classes by m, so that short codes get small CTAs and many of them per SM
-// (a round's serial pivot choice leaves issue slots that only other CTAs fill): m <= 256 on 128
-// threads, m <= 512 and m <= 640 on 256, m <= 1024 on 512 (T fills the SM's shared memory).
+// The large-code OSD runs in classes by m, each with the shared memory its longest code needs, so that
+// up to m = 640 two CTAs of 256 threads share an SM (a round's serial pivot choice leaves issue slots
+// that only another CTA fills); above, T fills the SM's shared memory and a CTA has 512 threads.
 constexpr int kOsdHClasses = 4;
 constexpr int kOsdHClassMaxM[kOsdHClasses] = {256, 512, 640, 1024};
 inline int osd_h_class(int m) { return m <= 256 ? 0 : m <= 512 ? 1 : m <= 640 ? 2 : 3; }

@@ -979,7 +979,7 @@ int sicc_engine_add_code(unsigned long long handle, const sicc_engine_code_t* co
             e->osd_nmax = std::max(e->osd_nmax, d.n);
             e->osd_kmax = std::max(e->osd_kmax, d.k);
         }
-        if (ec.osd_h) e->h_cls[osd_h_class(code->m)].add(d.n, code->m, ec.code->osd_h_view().pool, ec.code->edges());
+        if (ec.osd_h) e->h_cls[osd_h_class(code->m)].add(d.n, code->m, ec.code->osd_h_view().pool);
         e->codes.push_back(std::move(ec));
         e->dirty = true;
         *out_code_id = static_cast<int>(e->codes.size()) - 1;

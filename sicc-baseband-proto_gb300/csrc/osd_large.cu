@@ -37,7 +37,9 @@ namespace sicc {
 
 namespace {
 
-constexpr int kOsdHClassThreads[kOsdHClasses] = {256, 256, 256, 512};  // CTA size by class
+// CTA size by class.  128 threads for m <= 256 was no better: 500 codewords of 27 mixed codes 520 us
+// against 510, 20,000 the same within the runs.
+constexpr int kOsdHClassThreads[kOsdHClasses] = {256, 256, 256, 512};
 constexpr int kOsdHMaxPool = 128;
 constexpr int kRound = 8;  // columns of H per elimination round
 constexpr int kTabStride = 33;  // words per table entry: lanes reading different entries hit different banks
@@ -48,7 +50,6 @@ struct OsdHLayout {
     int mw;       // words per row of T for the largest m
     int ts;       // column stride of T in words (odd: a warp reading one word of 32 columns hits 32 banks)
     int poolmax;
-    int nnzmax;   // > 0: the columns' row lists are staged in shared memory (16-bit rows)
     int mlo, mhi; // the launch decodes the items of codes with mlo < m <= mhi
 };
 
@@ -57,7 +58,6 @@ struct OsdHSmem {
                              // t-th pivot's row, then two buffers of kRound reduced candidate columns; after the
                              // elimination the tables and terms of the candidate tests
     unsigned long long* keys;// [np] sort keys; shares T's space
-    int* colinfo;            // [nmax] first edge << 8 | weight of the column at each sorted position
     float* rel;              // [nmax] |llr| by sorted position j
     int16_t* perm;           // [nmax] code position at sorted position j
     int16_t* row_of_col;     // [nmax] pivot rank of a code position, -1 for the MRB
@@ -72,11 +72,10 @@ struct OsdHSmem {
     uint32_t* syn;           // [mw] s = H * hard by row of H
     int16_t* pivj;           // [32*mw] sorted position of the t-th pivot's column
     float* relq;             // [32*mw] |llr| of the t-th pivot's column
-    int16_t* mrb;            // [nmax] dependent positions met during the scan (descending j)
+    int16_t* mrb;            // [nmax] dependent positions met during the scan (descending j); shares vs..relq's space
     int16_t* pool_j;         // [poolmax] flip pool (sorted positions, weakest first)
     uint32_t* avec;          // [poolmax][mw] T h_f for the pool, bit t = pivot rank t
     uint32_t* aug;           // [mw] T s, bit t = pivot rank t
-    int16_t* rows;           // [nnzmax] rows of H's columns (when staged)
 };
 
 // Floats of one warp's metric terms: m pivots, 3 flips, padding to a group of four.
@@ -101,7 +100,6 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
         t.T = reinterpret_cast<uint32_t*>(g);
         t.keys = reinterpret_cast<unsigned long long*>(g);
     }
-    t.colinfo = reinterpret_cast<int*>(take(static_cast<size_t>(l.nmax) * 4));
     t.rel = reinterpret_cast<float*>(take(static_cast<size_t>(l.nmax) * 4));
     t.perm = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nmax) * 2));
     t.row_of_col = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nmax) * 2));
@@ -112,22 +110,21 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
     t.order = reinterpret_cast<int16_t*>(take(rows * 2));
     t.syn = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(l.mw) * 4));
     t.pivj = reinterpret_cast<int16_t*>(take(rows * 2));
-    t.mrb = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nmax) * 2));
     t.pool_j = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.poolmax) * 2));
-    {  // the tables of the elimination, then the vectors of the candidate search
+    {  // the tables and dependent positions of the elimination, then the vectors of the candidate search
         const size_t b_vs = a16((static_cast<size_t>(l.poolmax) + 1) * l.mw * 4);
         const size_t b_avec = a16(static_cast<size_t>(l.poolmax) * l.mw * 4);
         const size_t b_aug = a16(static_cast<size_t>(l.mw) * 4);
         const size_t b_relq = a16(rows * 4);
-        const size_t b_vec = b_vs + b_avec + b_aug + b_relq, b_tab = 32 * kTabStride * 4;
-        unsigned char* g = take(b_vec > b_tab ? b_vec : b_tab);
+        const size_t b_vec = b_vs + b_avec + b_aug + b_relq, b_tab = a16(32 * kTabStride * 4), b_mrb = a16(static_cast<size_t>(l.nmax) * 2);
+        unsigned char* g = take(b_vec > b_tab + b_mrb ? b_vec : b_tab + b_mrb);
         t.tab = reinterpret_cast<uint32_t*>(g);
+        t.mrb = reinterpret_cast<int16_t*>(g ? g + b_tab : nullptr);
         t.vs = reinterpret_cast<uint32_t*>(g);
         t.avec = reinterpret_cast<uint32_t*>(g ? g + b_vs : nullptr);
         t.aug = reinterpret_cast<uint32_t*>(g ? g + b_vs + b_avec : nullptr);
         t.relq = reinterpret_cast<float*>(g ? g + b_vs + b_avec + b_aug : nullptr);
     }
-    t.rows = reinterpret_cast<int16_t*>(take(static_cast<size_t>(l.nnzmax) * 2));
     if (s) *s = t;
     return o;
 }
@@ -135,7 +132,7 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
 __device__ __forceinline__ unsigned tbit(const uint32_t* row, int q) { return (row[q >> 5] >> (q & 31)) & 1u; }
 
 // CTAs per SM the registers are bounded for (shared memory sets the same or less).
-constexpr int osd_h_ctas(int threads) { return threads == 128 ? 5 : threads == 256 ? 2 : 1; }
+constexpr int osd_h_ctas(int threads) { return threads == 256 ? 2 : 1; }
 
 }  // namespace
 
@@ -244,15 +241,6 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             const unsigned b = __ballot_sync(0xffffffffu, par);
             if (lane == 0) s.syn[r >> 5] = b;
         }
-        // column of H at each sorted position: first edge << 8 | weight
-        const bool staged = lay.nnzmax > 0;
-        if (staged)
-            for (int e = tid; e < hv.col_ptr[n]; e += kThreads) s.rows[e] = static_cast<int16_t>(hv.col_rows[e]);
-        for (int j = tid; j < n; j += kThreads) {
-            const int c = s.perm[j];
-            const int e0 = hv.col_ptr[c];
-            s.colinfo[j] = (e0 << 8) | (hv.col_ptr[c + 1] - e0);
-        }
         __syncthreads();
 
         // ---- 3. Gauss-Jordan scan of H's columns in increasing reliability ----
@@ -261,51 +249,73 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
         // the pivot's row operation T <- (I + W e_p^T) T, W = v + e_p, turns
         // column c into e_p and leaves earlier pivot columns alone.
         // Columns are taken kRound at a time.  Interval k of the pipeline:
-        //   1. all warps: tabulate round k-1's basis U by index nibble, note its pivots, gather the
-        //      stored columns' bits at its pivot rows (their indices), and apply its operation to
-        //      round k's candidates (a warp each);
+        //   1. all warps tabulate round k-1's basis by index nibble, gather the stored columns' bits
+        //      at its pivot rows (their indices) and apply its operation to round k's candidates (a
+        //      warp each);
         //   2. warp 0 picks round k's pivots in order; each pivot's operation is applied at once to
         //      the later candidates and to the round's basis,
         //        a -> a + sum_r a_{p_r} U_r,  U_r <- U_r + U_r[p] W for a new pivot p
         //      (a_{p_r} a column's bits before the round, U_r = 0 for a dependent candidate);
-        //      the other warps apply round k-1's operation to the stored columns of T (one thread
-        //      per column, two table entries per word), append
-        //      the columns of its pivot rows (e_p + U_p), meet on a named barrier and reduce round
-        //      k+1's candidates against T.
-        auto reduce_candidate = [&](int jj, uint32_t* dst) {  // T h_c of the column at position jj, word `lane`
-            unsigned v = 0u;
+        //      the other warps note round k-1's pivots, apply its operation to the stored columns
+        //      (one thread per column, two table entries per word), append the columns of its pivot
+        //      rows (e_p + U_p), meet on a named barrier and reduce round k+1's candidates against T,
+        //      whose rows they fetched from H during round k-1.
+        // Warp 0's chain takes about 2,000 cycles of a round, the step before it 700-1,000; with the
+        // rows fetched at the reduction instead, staged in shared memory, 500 codewords of 27 mixed
+        // codes took 533 us (500 now; 20,000 took the same 4.2 ms).  Tables and indices built by the
+        // other warps in 2 instead of by all in 1: 512 us and 4.25 ms.  Windows of 16 candidates to
+        // fill each round with 8 pivots: 538 us and 4.8 ms.
+        // The column at position jj: first edge << 8 | weight (0: none), and its row for this lane.
+        struct Column {
+            int info, row;
+        };
+        auto column_at = [&](int jj) -> Column {
+            Column c{0, 0};
             if (jj >= 0) {
-                const int ci = s.colinfo[jj], e0 = ci >> 8, cnt = ci & 255;
-                // lane e: row of the column's e-th one (none: a row no lane holds), and that row's
-                // column's place in T (-1: a unit vector)
-                int mine = (2047 << 16) | 0xffff;
-                if (lane < cnt) {
-                    const int q = staged ? static_cast<int>(s.rows[e0 + lane]) : hv.col_rows[e0 + lane];
-                    mine = (q << 16) | static_cast<uint16_t>(s.rank[q]);
-                }
-                // the word of row u >> 16's column of T: loaded whether or not it is stored (place 0
-                // then), so that no branch stands between the loads of a group
-                auto word = [&](int u) -> unsigned {
-                    const int at = static_cast<int16_t>(u & 0xffff), row = u >> 16;
-                    const unsigned x = s.T[max(at, 0) * TS + lane];
-                    return at >= 0 ? x : lane == (row >> 5) ? 1u << (row & 31) : 0u;
-                };
-                for (int e = 0; e < cnt && e < 32; e += 4) {
-                    unsigned part[4];
+                const int v = s.perm[jj], e0 = __ldg(hv.col_ptr + v);
+                c.info = (e0 << 8) | (__ldg(hv.col_ptr + v + 1) - e0);
+                if (lane < (c.info & 255)) c.row = __ldg(hv.col_rows + e0 + lane);
+            }
+            return c;
+        };
+        auto reduce_column = [&](const Column& c, uint32_t* dst) {  // T h_c, word `lane`
+            unsigned v = 0u;
+            const int e0 = c.info >> 8, cnt = c.info & 255;
+            // lane e: row of the column's e-th one (none: a row no lane holds), and that row's
+            // column's place in T (-1: a unit vector)
+            const int mine = lane < cnt ? (c.row << 16) | static_cast<uint16_t>(s.rank[c.row]) : (2047 << 16) | 0xffff;
+            // the word of row u >> 16's column of T: loaded whether or not it is stored (place 0
+            // then), so that no branch stands between the loads of a group
+            auto word = [&](int u) -> unsigned {
+                const int at = static_cast<int16_t>(u & 0xffff), row = u >> 16;
+                const unsigned x = s.T[max(at, 0) * TS + lane];
+                return at >= 0 ? x : lane == (row >> 5) ? 1u << (row & 31) : 0u;
+            };
+            for (int e = 0; e < cnt && e < 32; e += 4) {
+                unsigned part[4];
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) part[x] = word(__shfl_sync(0xffffffffu, mine, (e + x) & 31));
-                    v ^= (part[0] ^ part[1]) ^ (part[2] ^ part[3]);
-                }
-                for (int e = 32; e < cnt; ++e) {  // columns heavier than 32
-                    const int row = hv.col_rows[e0 + e];
-                    v ^= word((row << 16) | static_cast<uint16_t>(s.rank[row]));
-                }
+                for (int x = 0; x < 4; ++x) part[x] = word(__shfl_sync(0xffffffffu, mine, (e + x) & 31));
+                v ^= (part[0] ^ part[1]) ^ (part[2] ^ part[3]);
+            }
+            for (int e = 32; e < cnt; ++e) {  // columns heavier than 32
+                const int row = __ldg(hv.col_rows + e0 + e);
+                v ^= word((row << 16) | static_cast<uint16_t>(s.rank[row]));
             }
             if (lane < MW) dst[lane] = v;
         };
+        auto workers_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kThreads - 32) : "memory"); };  // all but warp 0
         // candidate c of buffer b
         auto candidate = [&](int b, int c) -> uint32_t* { return s.T + (rows + b * kRound + c) * TS; };
-        for (int c = warp; c < kRound; c += kWarps) reduce_candidate(n - 1 - c, candidate(0, c));
+        for (int c = warp; c < kRound; c += kWarps) reduce_column(column_at(n - 1 - c), candidate(0, c));
+        // the columns this warp reduces next (round 1's), fetched a round ahead: candidates warp - 1
+        // and, with fewer than 8 workers, warp - 1 + kWarps - 1, ...
+        constexpr int kMine = (kRound + kWarps - 2) / (kWarps - 1);
+        Column ahead[kMine];
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+            const int c = warp - 1 + i * (kWarps - 1);
+            ahead[i] = column_at(warp > 0 && c < kRound ? n - 1 - kRound - c : -1);
+        }
         __syncthreads();
         int t = 0, j = n - 1, nd = 0, jstop = -1;          // after the rounds selected so far
         int pt = 0, pj = 0, pnd = 0, pnp = 0, pused = 0;   // the round whose update is pending
@@ -315,8 +325,8 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             const bool select = j >= 0 && t < m;
             if (!select && !pending) break;
             const int cb = k & 1, pb = cb ^ 1;
+            const uint32_t* Up = s.wv + pb * kRound * 32;  // the pending round's basis
             if (pending) {
-                const uint32_t* U = s.wv + pb * kRound * 32;
                 if (pnp > 0) {
                     // tables of the pending round's basis, one index nibble per warp, word `lane`
                     if (warp >= kWarps - 2 && lane < MW) {
@@ -324,7 +334,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                         uint32_t* tb = s.tab + h * 16 * kTabStride + lane;
                         unsigned u[4], acc[16];
 #pragma unroll
-                        for (int b = 0; b < 4; ++b) u[b] = U[(h * 4 + b) * 32 + lane];
+                        for (int b = 0; b < 4; ++b) u[b] = Up[(h * 4 + b) * 32 + lane];
                         acc[0] = 0u;
 #pragma unroll
                         for (int e = 1; e < 16; ++e) {
@@ -351,31 +361,17 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                             if (c[woff[r]] & wbit[r]) idx |= 1u << r;
                         s.tidx[at] = static_cast<uint8_t>(idx);
                     }
-                    // the pending operation on this round's candidates, not in them yet
-                    if (select)
-                        for (int c = warp; c < kRound; c += kWarps) {
-                            uint32_t* col = candidate(cb, c);
-                            const int p = lane < kRound ? s_rp[pb][lane] : -1;
-                            const unsigned idx = __ballot_sync(0xffffffffu, p >= 0 && ((col[p >> 5] >> (p & 31)) & 1u));
-                            unsigned v = lane < MW ? col[lane] : 0u;
+                }
+                if (select && pnp > 0)  // the pending operation on this round's candidates, not in them yet
+                    for (int c = warp; c < kRound; c += kWarps) {
+                        uint32_t* col = candidate(cb, c);
+                        const int p = lane < kRound ? s_rp[pb][lane] : -1;
+                        const unsigned idx = __ballot_sync(0xffffffffu, p >= 0 && ((col[p >> 5] >> (p & 31)) & 1u));
+                        unsigned v = lane < MW ? col[lane] : 0u;
 #pragma unroll
-                            for (int r = 0; r < kRound; ++r) v ^= U[r * 32 + lane] & (0u - ((idx >> r) & 1u));
-                            if (lane < MW) col[lane] = v;
-                        }
-                }
-                if (warp == kWarps - 3 && lane < pused) {  // pivot ranks and dependent positions
-                    const int pr = s_rp[pb][lane];
-                    const unsigned found = s_found[pb], below = (1u << lane) - 1u;
-                    if (pr >= 0) {
-                        const int rk = pt + __popc(found & below);
-                        s.order[rk] = static_cast<int16_t>(pr);
-                        s.rank[pr] = static_cast<int16_t>(rk);
-                        s.row_of_col[s.perm[pj - lane]] = static_cast<int16_t>(rk);
-                        s.pivj[rk] = static_cast<int16_t>(pj - lane);
-                    } else {
-                        s.mrb[pnd + __popc(~found & below)] = static_cast<int16_t>(pj - lane);  // an MRB position
+                        for (int r = 0; r < kRound; ++r) v ^= Up[r * 32 + lane] & (0u - ((idx >> r) & 1u));
+                        if (lane < MW) col[lane] = v;
                     }
-                }
                 __syncthreads();
             }
             if (warp == 0) {
@@ -439,6 +435,19 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                     }
                 }
             } else {
+                if (pending && warp == 1 && lane < pused) {  // pivot ranks and dependent positions
+                    const int pr = s_rp[pb][lane];
+                    const unsigned found = s_found[pb], below = (1u << lane) - 1u;
+                    if (pr >= 0) {
+                        const int rk = pt + __popc(found & below);
+                        s.order[rk] = static_cast<int16_t>(pr);
+                        s.rank[pr] = static_cast<int16_t>(rk);
+                        s.row_of_col[s.perm[pj - lane]] = static_cast<int16_t>(rk);
+                        s.pivj[rk] = static_cast<int16_t>(pj - lane);
+                    } else {
+                        s.mrb[pnd + __popc(~found & below)] = static_cast<int16_t>(pj - lane);  // an MRB position
+                    }
+                }
                 if (pending && pnp > 0) {
                     // a warp takes 32 columns, and above 16 words a half of their words: smaller pieces
                     // share out better (three loads and a store per word: shared-memory bandwidth
@@ -470,14 +479,19 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                         const int p = s_rp[pb][r];
                         if (p >= 0 && lane < MW)
                             s.T[(pt + __popc(s_found[pb] & ((1u << r) - 1u))) * TS + lane] =
-                                s.wv[(pb * kRound + r) * 32 + lane] ^ (lane == (p >> 5) ? 1u << (p & 31) : 0u);
+                                Up[r * 32 + lane] ^ (lane == (p >> 5) ? 1u << (p & 31) : 0u);
                     }
                 }
-                // T is final for the pending round before the next candidates read it
-                asm volatile("bar.sync 1, %0;" ::"r"(kThreads - 32) : "memory");
-                if (select)
-                    for (int c = warp - 1; c < kRound; c += kWarps - 1)
-                        reduce_candidate(j - kRound - c, candidate(cb ^ 1, c));
+                workers_sync();  // T is final for the pending round before the next candidates read it
+                if (select) {
+#pragma unroll
+                    for (int i = 0; i < kMine; ++i) {
+                        const int c = warp - 1 + i * (kWarps - 1);
+                        if (c >= kRound) break;
+                        reduce_column(ahead[i], candidate(cb ^ 1, c));
+                        ahead[i] = column_at(j - 2 * kRound - c);
+                    }
+                }
             }
             __syncthreads();
             pending = select;
@@ -547,7 +561,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             }
             if (lane < MW && acc) atomicXor(&s.vs[lane], acc);
             // T h_f for the flip pool, one warp per column
-            for (int i = warp; i < pool; i += kWarps) reduce_candidate(s.pool_j[i], s.vs + (i + 1) * MW);
+            for (int i = warp; i < pool; i += kWarps) reduce_column(column_at(s.pool_j[i]), s.vs + (i + 1) * MW);
         }
         __syncthreads();
         // bit t of an ordered vector = bit order[t] of the row-indexed one (8 vectors' loads in flight)
@@ -762,7 +776,6 @@ OsdHLayout osd_h_layout(const OsdHBounds& bd, int mlo, int mhi)
     l.poolmax = std::max(bd.poolmax, 1);
     l.mlo = mlo;
     l.mhi = mhi;
-    l.nnzmax = 0;
     return l;
 }
 
@@ -773,16 +786,9 @@ void launch_osd_h_class(const OsdHBounds& bd, int mlo, int mhi, const OsdIO& io_
     OsdIO io = io_all;  // the class's own work counter
     io.work_h = io_all.work_h ? io_all.work_h + cls : nullptr;
     OsdHLayout l = osd_h_layout(bd, mlo, mhi);
-    size_t smem = carve(l, nullptr, nullptr);
+    const size_t smem = carve(l, nullptr, nullptr);
     if (smem > 227 * 1024) throw InvalidArgument("large-code OSD tables exceed shared memory (m <= 1024, n <= 4096)");
-    // stage the columns' row lists when they cost no CTA per SM
-    constexpr size_t sm_bytes = 227 * 1024, reserved = 1024;  // the latter per CTA
-    const auto per_sm_by = [&](size_t bytes) { return std::min<size_t>(osd_h_ctas(kThreads), sm_bytes / (bytes + reserved)); };
-    l.nnzmax = bd.nnzmax;
-    if (bd.nnzmax <= 0 || carve(l, nullptr, nullptr) > 227 * 1024 || per_sm_by(carve(l, nullptr, nullptr)) < per_sm_by(smem))
-        l.nnzmax = 0;
-    smem = carve(l, nullptr, nullptr);
-    // the two 256-thread classes share this kernel with different sizes: the limit only grows
+    // the 256-thread classes share this kernel with different sizes: the limit only grows
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(osd_h_kernel<kThreads>), smem),
                "cudaFuncSetAttribute(osd_h)");
     int per_sm = 0;
@@ -796,18 +802,17 @@ void launch_osd_h_class(const OsdHBounds& bd, int mlo, int mhi, const OsdIO& io_
 
 }  // namespace
 
-void OsdHBounds::add(int n, int m, int pool, int nnz)
+void OsdHBounds::add(int n, int m, int pool)
 {
     nmax = std::max(nmax, n);
     mmax = std::max(mmax, m);
     poolmax = std::max(poolmax, pool);
-    nnzmax = std::max(nnzmax, nnz);
 }
 
 size_t osd_h_smem_bytes(int nmax, int mmax, int poolmax)
-{  // without the staged row lists
+{
     OsdHBounds bd;
-    bd.add(nmax, mmax, poolmax, 0);
+    bd.add(nmax, mmax, poolmax);
     const OsdHLayout l = osd_h_layout(bd, 0, 1024);
     return carve(l, nullptr, nullptr);
 }
@@ -838,8 +843,7 @@ void launch_osd_h(const OsdHBounds* cls, const OsdIO& io, int max_items, cudaStr
             check_cuda(cudaStreamWaitEvent(cs, fork, 0), "cudaStreamWaitEvent(osd fork)");
         }
         const int mlo = c == 0 ? 0 : kOsdHClassMaxM[c - 1];
-        if (kOsdHClassThreads[c] == 128) launch_osd_h_class<128>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
-        else if (kOsdHClassThreads[c] == 256) launch_osd_h_class<256>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
+        if (kOsdHClassThreads[c] == 256) launch_osd_h_class<256>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
         else launch_osd_h_class<512>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
         if (fan && used > 0) {
             check_cuda(cudaEventRecord(join[used - 1], cs), "cudaEventRecord(osd join)");
