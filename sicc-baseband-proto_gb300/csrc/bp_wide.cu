@@ -128,12 +128,16 @@ template <int D>
 struct WideRow {
     static constexpr int kQuads = (D + 3) / 4;
     uint4 o[kQuads];
-    uint4 state;  // messages: min1, min2 (scaled), signs and argmin
+    uint4 state;  // min1, min2 (scaled), signs and argmin; the messages themselves where D <= 4
+
+    __device__ __forceinline__ static unsigned word(const uint4& x, int j)
+    {
+        return (j & 3) == 0 ? x.x : (j & 3) == 1 ? x.y : (j & 3) == 2 ? x.z : x.w;
+    }
 
     __device__ __forceinline__ unsigned off(int j) const
     {
-        const uint4& x = o[j >> 2];
-        return (j & 3) == 0 ? x.x : (j & 3) == 1 ? x.y : (j & 3) == 2 ? x.z : x.w;
+        return word(o[j >> 2], j);
     }
     __device__ __forceinline__ void load_offsets(const uint4* __restrict__ table, int row)
     {
@@ -152,7 +156,7 @@ struct WideRow {
 // latency of tables and messages).  608 codewords of (64800,32400), D = 7: 768 threads 6.41 ms,
 // 1,024 (64 registers, spilling) 6.83; 600 of (16200,3240), D = 4: 2.58 and 2.35.
 template <int D>
-constexpr int wide_threads() { return D <= 4 ? 1024 : D <= 10 ? 768 : 512; }
+constexpr int wide_threads() { return D <= 4 ? 1024 : D <= 7 ? 896 : D <= 10 ? 768 : 512; }
 
 }  // namespace
 
@@ -166,7 +170,7 @@ constexpr int wide_threads() { return D <= 4 ? 1024 : D <= 10 ? 768 : 512; }
 // Measured on GB300, 608 codewords of (64800,32400) at 2 dB: 12.1 ms before (512 threads, a
 // branch per posterior access, variable indices slot by slot, (min1, min2, argmin) row
 // arithmetic, full syndrome: 78 instructions per edge and iteration), 6.41 ms now.
-template <int D>
+template <int D, int kFar>
 __global__ void __launch_bounds__(wide_threads<D>(), 1)
 bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long long slice, int split, int track_best)
 {
@@ -186,13 +190,28 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
     float* best = all_smem ? g : g + n_pad + 4;
     uint4* states = reinterpret_cast<uint4*>(best + (track_best ? n_pad : 0));
     const uint4* table = reinterpret_cast<const uint4*>(cv.wide_rows);
-    const int js = cv.wide_smem_slots;
+    constexpr int js = D - kFar;  // slots below it are in shared memory in every row
 
-    auto value = [&](const WideRow<D>& row, int j) -> float {
+    using Row = WideRow<D>;
+    auto value = [&](const Row& row, int j) -> float {
         return j < js ? reg::lds(s_raw, row.off(j)) : app.at(row.off(j));
     };
-    auto update = [&](const WideRow<D>& in, int row) {
+    auto put = [&](const Row& row, int j, float x) {
+        if (j < js) reg::sts(s_raw, row.off(j), x);
+        else app.put(row.off(j), x);
+    };
+    auto update = [&](const Row& in, int row) {
         float q[D], m[D];
+        if constexpr (D <= 4) {
+#pragma unroll
+            for (int j = 0; j < D; ++j) q[j] = __fsub_rn(value(in, j), __uint_as_float(Row::word(in.state, j)));
+            reg::row_messages<D>(q, p.alpha, p.beta, m);
+#pragma unroll
+            for (int j = 0; j < D; ++j) put(in, j, __fadd_rn(q[j], m[j]));
+            auto word = [&](int j) { return j < D ? __float_as_uint(m[j < D ? j : 0]) : 0u; };
+            states[row] = make_uint4(word(0), word(1), word(2), word(3));
+            return;
+        }
         const float o1 = __uint_as_float(in.state.x), o2 = __uint_as_float(in.state.y);
 #pragma unroll
         for (int j = 0; j < D; ++j) q[j] = __fsub_rn(value(in, j), rebuild(o1, o2, in.state.z, j));
@@ -214,14 +233,12 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
         for (int j = 0; j < D; ++j) {
             // the message, signed: the scaled magnitude with the sign of m
             const float mag = fabsf(m[j]) == most ? n2 : n1;
-            const float x = __fadd_rn(q[j], __uint_as_float(__float_as_uint(mag) ^ (__float_as_uint(m[j]) & 0x80000000u)));
-            if (j < js) reg::sts(s_raw, in.off(j), x);
-            else app.put(in.off(j), x);
+            put(in, j, __fadd_rn(q[j], __uint_as_float(__float_as_uint(mag) ^ (__float_as_uint(m[j]) & 0x80000000u))));
         }
         states[row] = make_uint4(__float_as_uint(n1), __float_as_uint(n2), signs | (static_cast<unsigned>(idx) << 27), 0u);
     };
     auto parity_of = [&](int row) -> unsigned {
-        WideRow<D> r;
+        Row r;
         r.load_offsets(table, row);
         unsigned par = 0u;
 #pragma unroll
@@ -255,7 +272,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
         __syncthreads();
         int best_w = track_best ? syndrome() : 1;
         int iter = 0, w = 0;
-        WideRow<D> next;
+        Row next;
         if (tid < __ldg(cv.layer_start + 1)) next.load(table, tid, true, states);
         for (;;) {
             int first = 0, rows = __ldg(cv.layer_start + 1);
@@ -265,7 +282,7 @@ bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long
                 const int after_rows = __ldg(cv.layer_start + (last ? 1 : L + 2)) - after;
                 const bool fresh = iter == 0, after_fresh = fresh && !last;
                 for (int rs = tid;; rs += kThreads) {
-                    const WideRow<D> row = next;
+                    const Row row = next;
                     if (rs + kThreads < rows) next.load(table, first + rs + kThreads, fresh, states);
                     else if (tid < after_rows) next.load(table, after + tid, after_fresh, states);
                     if (rs < rows) update(row, first + rs);
@@ -508,7 +525,7 @@ void launch_flooding_wide_d(const FloodView& cv, const BpParams& p, const BpIO& 
     }
 }
 
-template <int D>
+template <int D, int kFar>
 void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
 {
     const long long n_pad = (cv.n + 3) & ~3;
@@ -518,7 +535,7 @@ void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO&
     const size_t smem = static_cast<size_t>(split) * sizeof(float);
     long long slice = (all_smem ? 0 : n_pad + 4) + (track_best ? n_pad : 0) + 4 * mp;
     slice = (slice + 31) & ~31LL;  // 128-byte aligned slices
-    const auto kernel = bp_layered_wide_kernel<D>;
+    const auto kernel = bp_layered_wide_kernel<D, kFar>;
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp wide)");
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, wide_threads<D>(), smem) != cudaSuccess || per_sm <= 0)
@@ -535,6 +552,14 @@ void launch_layered_wide_t(const LayeredView& cv, const BpParams& p, const BpIO&
     const cudaError_t ferr = cudaFreeAsync(scratch, st);
     check_cuda(err, "bp wide kernel launch");
     check_cuda(ferr, "cudaFreeAsync(bp wide)");
+}
+
+template <int D>
+void launch_layered_wide_d(const LayeredView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
+{
+    if (cv.wide_smem_slots >= D) launch_layered_wide_t<D, 0>(cv, p, io, track_best, st);
+    else if (cv.wide_smem_slots >= D - 2) launch_layered_wide_t<D, 2>(cv, p, io, track_best, st);
+    else launch_layered_wide_t<D, D>(cv, p, io, track_best, st);
 }
 
 }  // namespace
@@ -569,13 +594,13 @@ void launch_bp_layered_wide(const LayeredView& cv, const BpParams& p, const BpIO
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
     check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
     switch (wide_slots(cv.maxdeg)) {
-        case 4: launch_layered_wide_t<4>(cv, p, io, track_best, st); break;
-        case 6: launch_layered_wide_t<6>(cv, p, io, track_best, st); break;
-        case 7: launch_layered_wide_t<7>(cv, p, io, track_best, st); break;
-        case 10: launch_layered_wide_t<10>(cv, p, io, track_best, st); break;
-        case 14: launch_layered_wide_t<14>(cv, p, io, track_best, st); break;
-        case 18: launch_layered_wide_t<18>(cv, p, io, track_best, st); break;
-        default: launch_layered_wide_t<27>(cv, p, io, track_best, st); break;
+        case 4: launch_layered_wide_d<4>(cv, p, io, track_best, st); break;
+        case 6: launch_layered_wide_d<6>(cv, p, io, track_best, st); break;
+        case 7: launch_layered_wide_d<7>(cv, p, io, track_best, st); break;
+        case 10: launch_layered_wide_d<10>(cv, p, io, track_best, st); break;
+        case 14: launch_layered_wide_d<14>(cv, p, io, track_best, st); break;
+        case 18: launch_layered_wide_d<18>(cv, p, io, track_best, st); break;
+        default: launch_layered_wide_d<27>(cv, p, io, track_best, st); break;
     }
 }
 
