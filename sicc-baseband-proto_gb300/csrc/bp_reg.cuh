@@ -224,13 +224,13 @@ __device__ __forceinline__ void update_row(unsigned char* smem, const Rows<D, NL
     for (int j = 0; j < D; ++j) sts(smem, r.off(t, j), __fadd_rn(q[j], msg[j]));
 }
 
-// Unsatisfied checks among the lane's rows.
-template <bool kPlain, int D, int NL>
+// Unsatisfied checks among the lane's rows kFrom .. kTo - 1.
+template <bool kPlain, int kFrom, int kTo, int D, int NL>
 __device__ __forceinline__ unsigned lane_syndrome(const unsigned char* smem, const Rows<D, NL>& r, int nrows)
 {
     unsigned cnt = 0u;
-    static_for<NL>([&](auto ti) {
-        constexpr int t = decltype(ti)::value;
+    static_for<kTo - kFrom>([&](auto ti) {
+        constexpr int t = kFrom + decltype(ti)::value;
         if (kPlain || t < nrows) {
             unsigned par = 0u;
 #pragma unroll

@@ -6,7 +6,7 @@
 // Measured on GB300 against the kernels before it (compressed row state, in
 // registers for the (128,64) code, else in shared memory): 65,536 frames of
 // (128,64) at 2 dB with OSD 506 -> 390 us, of which BP 235 -> about 120 (ALU
-// pipe 80% busy before); 7,680 codewords of (1024,512) at 2 dB 1,000 -> 301 us;
+// pipe 80% busy before); 7,680 codewords of (1024,512) at 2 dB 1,000 -> 245 us;
 // 1,000 of (2048,1024) at 2.5 dB 645 -> 82 us.
 #include "bp_kernels.h"
 #include "bp_reg.cuh"
@@ -49,7 +49,7 @@ bp_layered_reg_kernel(LayeredView cv, BpParams p, BpIO io, int slots_per_cta, in
             for (int j = 0; j < D; ++j) msg[decltype(ti)::value][j] = 0.0f;
         });
         g.sync();
-        best_w = g.sum(lane_syndrome<kPlain>(smem, rows, nrows));
+        best_w = track_best ? g.sum(lane_syndrome<kPlain, 0, NL>(smem, rows, nrows)) : 1;
         iter = 0;
     };
     if (g.gl == 0) app[n_pad] = __int_as_float(0x7f800000);  // +inf, before init's sync
@@ -64,7 +64,15 @@ bp_layered_reg_kernel(LayeredView cv, BpParams p, BpIO io, int slots_per_cta, in
                 if (kPlain || (t + 1) % cv.reg_rpl == 0) g.sync();  // end of a layer
             }
         });
-        const int w = g.sum(lane_syndrome<kPlain>(smem, rows, nrows));
+        // without tracking only "zero or not" matters: a lane's other rows are read only when the
+        // group's first rows all hold (7,680 codewords of (1024,512) at 2 dB 300 -> 245 us)
+        unsigned bad = lane_syndrome<kPlain, 0, 1>(smem, rows, nrows);
+        int w = track_best ? 0 : g.sum(bad);
+        if (w == 0) {
+            bad += lane_syndrome<kPlain, 1, NL>(smem, rows, nrows);
+            if (W > 1 && !track_best) g.sync();  // between two sums
+            w = g.sum(bad);
+        }
         ++iter;
         // the best posterior so far (a zero syndrome always is, and then it is app itself)
         if (track_best && w < best_w && w != 0) {

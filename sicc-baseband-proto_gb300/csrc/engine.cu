@@ -358,7 +358,7 @@ struct RegUnit {
             for (int j = 0; j < D; ++j) msg[decltype(ti)::value][j] = 0.0f;
         });
         g.sync();
-        best_w = g.sum(reg::lane_syndrome<true>(smem, rows, NL));
+        best_w = g.sum(reg::lane_syndrome<true, 0, NL>(smem, rows, NL));
         iter = 0;
     }
     // One iteration; true when the codeword has stopped (its outputs are written then).
@@ -369,7 +369,7 @@ struct RegUnit {
             reg::update_row(smem, rows, t, d.alpha, d.beta, msg[t]);
             g.sync();
         });
-        const int w = g.sum(reg::lane_syndrome<true>(smem, rows, NL));
+        const int w = g.sum(reg::lane_syndrome<true, 0, NL>(smem, rows, NL));
         ++iter;
         if (route && w < best_w && w != 0) {
             reg::copy_slot(g, best, app, (d.n + 3) & ~3);
