@@ -452,7 +452,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                     // a warp takes 32 columns, and above 16 words a half of their words: smaller pieces
                     // share out better (three loads and a store per word: shared-memory bandwidth
                     // bounds this at m = 1024)
-                    const int halves = MW > 16 ? 2 : 1, per = (MW / halves + 3) & ~3;
+                    const int halves = MW > 16 ? 2 : 1, per = ((MW + halves - 1) / halves + 3) & ~3;
                     for (int piece = warp - 1; piece < ((pt + 31) >> 5) * halves; piece += kWarps - 1) {
                         const int at = (halves == 2 ? piece >> 1 : piece) * 32 + lane;
                         const int w0 = halves == 2 ? (piece & 1) * per : 0, w1 = min(MW, w0 + per);
