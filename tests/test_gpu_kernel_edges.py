@@ -229,3 +229,48 @@ def test_transmit(cuda, phy, systematic):
     torch.cuda.synchronize()
     coded = tx_oracle.encode_generator(info.reshape(-1, code.k), G).reshape(3, -1)
     _close(out.cpu().numpy(), tx_oracle.tx_frames(coded, **_kw(t)), phy)
+
+
+# --- mixed batches ----------------------------------------------------------------------------------
+
+MIXED = [(4, 8, 9), (5, 16, 17), (3, 6, 20), (8, 16, 65), (8, 16, 128), (4, 8, 8), (4, 16, 32), (4, 18, 40), (5, 16, 64)]
+
+
+@pytest.mark.parametrize("more", [[], [(8, 16, 256)]], ids=["small", "large"])
+def test_mixed_shapes(cuda, oracle, more):
+    """Codes of the register-resident and the general row arithmetic, and (large) a code whose posteriors
+    take the whole batch to the general one; unaligned soft values."""
+    torch = cuda
+    cs = [codes.qc_code(*b, seed=13) for b in MIXED + more]
+    eng = engine.Engine(max_codewords=256, max_llr_floats=1 << 18)
+    for c in cs:
+        eng.add_code(c, 8, alpha=0.8, beta=0.1)
+    ids, rows = [], []
+    for ci, c in enumerate(cs):
+        for x in _soft(c, 7, 2.5, 80 + ci):
+            ids.append(ci)
+            rows.append(x)
+    perm = np.random.default_rng(4).permutation(len(ids))
+    ids, rows = [ids[i] for i in perm], [rows[i] for i in perm]
+    lo, io, at, bits = [], [], 1, 0
+    for ci, x in zip(ids, rows):
+        lo.append(at)
+        io.append(bits)
+        at += x.size + 1
+        bits += cs[ci].k
+    llr = np.zeros(at, np.float32)
+    for o, x in zip(lo, rows):
+        llr[o:o + x.size] = x
+    info = torch.zeros(bits, dtype=torch.uint8, device="cuda")
+    ok, used, it = (torch.zeros(len(ids), dtype=torch.uint8, device="cuda") for _ in range(3))
+    eng.decode_device(len(ids), torch.from_numpy(np.asarray(ids, np.uint8)).cuda(), torch.from_numpy(llr).cuda(),
+                      torch.tensor(lo, dtype=torch.int64, device="cuda"), info,
+                      torch.tensor(io, dtype=torch.int64, device="cuda"), ok, used, it,
+                      stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    got, gok, git = info.cpu().numpy(), ok.cpu().numpy(), it.cpu().numpy()
+    ocs = [oracle.code(c.n, c.m, c.row_ptr, c.col_ind) for c in cs]
+    for i, (ci, x) in enumerate(zip(ids, rows)):
+        o = ocs[ci].layered(x, 8, 0.8, 0.1)
+        assert gok[i] == o[0] and git[i] == o[4], (ci, i)
+        assert np.array_equal(got[io[i]:io[i] + cs[ci].k], o[1][: cs[ci].k]), (ci, i)
