@@ -412,7 +412,7 @@ void launch_bp_layered(const LayeredView& cv, const BpParams& p, const BpIO& io,
     if (io.count <= 0) return;
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
     if (cv.reg_group > 0) {
-        check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
+        if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
         launch_bp_layered_reg(cv, p, io, shape, track_best, st);
         return;
     }
@@ -425,7 +425,7 @@ void launch_bp_layered(const LayeredView& cv, const BpParams& p, const BpIO& io,
     slots = std::max(step, slots - slots % step);
     if (slots * cv.group > kBpThreads) slots = kBpThreads / cv.group;
     while (slots > step && layered_smem_bytes(cv, slots, track_best, nullptr) > 227 * 1024) slots -= step;
-    check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
+    if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
     // the row loops are unrolled to D slots: the closest D above the code's row degree
     if (cv.maxdeg <= 6) launch_layered_t<6>(cv, p, io, slots, shape.ctas, track_best, st);
     else if (cv.maxdeg <= 8) launch_layered_t<8>(cv, p, io, slots, shape.ctas, track_best, st);

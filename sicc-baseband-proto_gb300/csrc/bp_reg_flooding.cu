@@ -140,7 +140,7 @@ void launch_bp_flooding_reg(const LayeredView& cv, const BpParams& p, const BpIO
 {
     if (io.count <= 0) return;
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
-    check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
+    if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
     const auto go = [&](auto damp) {
         constexpr bool kDamp = decltype(damp)::value;
         if (cv.num_layers == 4 && cv.maxdeg <= 6) launch_shape<6, 4, kDamp>(cv, p, io, track_best, st);

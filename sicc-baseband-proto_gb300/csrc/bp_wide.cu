@@ -592,7 +592,7 @@ void launch_bp_layered_wide(const LayeredView& cv, const BpParams& p, const BpIO
 {
     if (io.count <= 0) return;
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
-    check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
+    if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
     switch (wide_slots(cv.maxdeg)) {
         case 4: launch_layered_wide_d<4>(cv, p, io, track_best, st); break;
         case 6: launch_layered_wide_d<6>(cv, p, io, track_best, st); break;
@@ -609,7 +609,7 @@ void launch_bp_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO&
     if (io.count <= 0) return;
     if (cv.maxdeg > 27) throw InvalidArgument("flooding schedule supports row degree <= 27");
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
-    check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
+    if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
     if (cv.maxdeg <= 6) launch_flooding_wide_d<6>(cv, p, io, track_best, st);
     else if (cv.maxdeg <= 10) launch_flooding_wide_d<10>(cv, p, io, track_best, st);
     else if (cv.maxdeg <= 18) launch_flooding_wide_d<18>(cv, p, io, track_best, st);

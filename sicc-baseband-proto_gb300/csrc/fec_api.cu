@@ -175,7 +175,9 @@ void run_bp_osd(const DeviceCode& code, const BpParams& bp, const BpLaunch& shap
         io.osd_llr = s.osd_llr.p;
         io.osd_index = s.osd_index.p;
         io.osd_count = s.counters.p;
-        check_cuda(cudaMemsetAsync(s.counters.p, 0, sizeof(int), st), "reset osd count");
+        // the three counters in one go: each reset is a launch of its own in front of a kernel
+        check_cuda(cudaMemsetAsync(s.counters.p, 0, 3 * sizeof(int), st), "reset counters");
+        io.work_zeroed = true;
     }
     if (rec) check_cuda(cudaEventRecord(rec->ev[0], st), "cudaEventRecord");
     if (code.layered()) launch_bp_layered(code.layered_view(), p, io, shape, st);
@@ -192,6 +194,7 @@ void run_bp_osd(const DeviceCode& code, const BpParams& bp, const BpLaunch& shap
         oio.info_stride = out_stride;
         oio.used_osd = d_used_osd;
         oio.work = s.counters.p + 2;
+        oio.work_zeroed = true;
         launch_osd(code.osd_view(), oio, count, st, 0, shape.osd_ctas);
     }
     if (rec) {
@@ -819,8 +822,9 @@ int decode_with_caller_scratch(unsigned long long handle, const float* d_llr, in
     io.work_counter = counters + 1;
     BpParams p = d->bp;
     p.route_failures_to_osd = d->osd_enabled ? 1 : 0;
-    // both counters start at zero on every call: the array keeps the previous call's contents
-    check_cuda(cudaMemsetAsync(counters, 0, 2 * sizeof(int), st), "clear static scratch counters");
+    // the counters start at zero on every call: the array keeps the previous call's contents
+    check_cuda(cudaMemsetAsync(counters, 0, 3 * sizeof(int), st), "clear static scratch counters");
+    io.work_zeroed = true;
     if (d->osd_enabled) {
         io.osd_llr = rows;
         io.osd_index = index;
@@ -838,6 +842,7 @@ int decode_with_caller_scratch(unsigned long long handle, const float* d_llr, in
         oio.info_stride = d->k;
         oio.used_osd = d_used_osd;
         oio.work = counters + 2;  // inside the counters' 256 bytes
+        oio.work_zeroed = true;
         launch_osd(d->code->osd_view(), oio, count, st, 0, d->shape.osd_ctas);
     }
     return CUDA_OSD_STATUS_OK;

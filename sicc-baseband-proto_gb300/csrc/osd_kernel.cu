@@ -613,7 +613,7 @@ void launch_osd(const OsdView& ov, const OsdIO& io, int max_items, cudaStream_t 
 {
     (void)warps_per_cta;
     if (max_items <= 0) return;
-    if (io.work) check_cuda(cudaMemsetAsync(io.work, 0, sizeof(int), st), "reset OSD work counter");
+    if (io.work && !io.work_zeroed) check_cuda(cudaMemsetAsync(io.work, 0, sizeof(int), st), "reset OSD work counter");
     // for a mixed-code batch `ov` carries the largest n and k of its codes
     const int nw = (ov.n + 63) / 64;
     const int kr = (ov.k + 31) / 32;

@@ -830,7 +830,8 @@ void launch_osd_h(const OsdHBounds* cls, const OsdIO& io, int max_items, cudaStr
         if (cls[c].mmax > kOsdHClassMaxM[c]) throw InvalidArgument("large-code OSD: code in the wrong class (m <= 1024)");
     }
     if (present == 0) return;
-    if (io.work_h) check_cuda(cudaMemsetAsync(io.work_h, 0, kOsdHClasses * sizeof(int), st), "reset OSD work counters");
+    if (io.work_h && !io.work_zeroed)
+        check_cuda(cudaMemsetAsync(io.work_h, 0, kOsdHClasses * sizeof(int), st), "reset OSD work counters");
     // the classes run side by side: the first present one on st, the others on side streams
     const bool fan = present > 1 && side && fork && join;
     if (fan) check_cuda(cudaEventRecord(fork, st), "cudaEventRecord(osd fork)");

@@ -109,7 +109,8 @@ struct BpIO {
     int* osd_index;        // [cap]
     int* osd_count;        // [1]
     uint8_t* used_osd;     // [count]
-    int* work_counter;     // [1] dynamic-scheduling counter (zeroed by the launcher)
+    int* work_counter;     // [1] dynamic-scheduling counter (zeroed by the launcher, unless work_zeroed)
+    bool work_zeroed;      // the caller has zeroed it on the stream
 };
 
 // Ordered-statistics decoding of one code.
@@ -156,11 +157,12 @@ struct OsdIO {
     const long long* llr_off;
     const long long* info_off;
     const long long* row_off;
-    // Work counters (device ints the launcher zeroes on the stream): each warp (warp kernel) or
+    // Work counters (device ints the launcher zeroes on the stream unless work_zeroed): each warp (warp kernel) or
     // CTA (large-code kernel, one counter per class) takes its next item from them, so a few
     // expensive codewords do not hold up one warp's share.  Null: items by static striding.
     int* work;      // warp kernel
     int* work_h;    // [kOsdHClasses] large-code kernel
+    bool work_zeroed;
 };
 
 }  // namespace sicc
