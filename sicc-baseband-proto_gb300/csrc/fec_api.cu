@@ -249,14 +249,18 @@ struct StreamDecoder : Decoder {
     cuda_osd_stream_config_t cfg{};
     struct Batch {
         DevBuf<float> llr;
-        DevBuf<uint8_t> info, used_osd, success;
-        HostBuf<uint8_t> h_info, h_used_osd, h_success;
+        // info bits, used-OSD flags and success flags of the batch's `count` codewords one after
+        // the other, so that one copy brings them back
+        DevBuf<uint8_t> out;
+        HostBuf<uint8_t> h_out;
         std::vector<unsigned long long> ts, ids;
         std::vector<unsigned> blocks;
         int count = 0;
         uint64_t first_arrival_us = 0;  // decoder clock when the batch took its first codeword
         bool in_flight = false;
         bool held = false;  // retired: its results wait in the ready queue, read in place
+        const uint8_t* h_used_osd(int k) const { return h_out.p + static_cast<size_t>(count) * k; }
+        const uint8_t* h_success(int k) const { return h_used_osd(k) + count; }
         cudaEvent_t done = nullptr;
         cudaEvent_t start = nullptr;
         ~Batch()
@@ -328,12 +332,8 @@ struct StreamDecoder : Decoder {
         for (int i = 0; i < kRing; ++i) {
             auto b = std::make_unique<Batch>();
             b->llr.alloc(static_cast<size_t>(max_batch) * n);
-            b->info.alloc(static_cast<size_t>(max_batch) * k);
-            b->used_osd.alloc(max_batch);
-            b->success.alloc(max_batch);
-            b->h_info.alloc(static_cast<size_t>(max_batch) * k);
-            b->h_used_osd.alloc(max_batch);
-            b->h_success.alloc(max_batch);
+            b->out.alloc(static_cast<size_t>(max_batch) * (k + 2));
+            b->h_out.alloc(static_cast<size_t>(max_batch) * (k + 2));
             check_cuda(cudaEventCreate(&b->done), "cudaEventCreate");
             check_cuda(cudaEventCreate(&b->start), "cudaEventCreate");
             b->ts.reserve(max_batch);
@@ -352,15 +352,12 @@ struct StreamDecoder : Decoder {
         check_cuda(cudaEventRecord(copied, copy_stream), "cudaEventRecord(copy)");
         check_cuda(cudaStreamWaitEvent(stream, copied, 0), "cudaStreamWaitEvent(copy)");
         check_cuda(cudaEventRecord(b.start, stream), "cudaEventRecord");
-        run_bp_osd(*code, bp, shape, osd_enabled, b.llr.p, b.count, b.info.p, k, k, b.success.p, b.used_osd.p,
-                   nullptr, nullptr, scratch, stream, &timing);
-        check_cuda(cudaMemcpyAsync(b.h_info.p, b.info.p, static_cast<size_t>(b.count) * k, cudaMemcpyDeviceToHost,
+        uint8_t* used = b.out.p + static_cast<size_t>(b.count) * k;
+        run_bp_osd(*code, bp, shape, osd_enabled, b.llr.p, b.count, b.out.p, k, k, used + b.count, used, nullptr,
+                   nullptr, scratch, stream, &timing);
+        check_cuda(cudaMemcpyAsync(b.h_out.p, b.out.p, static_cast<size_t>(b.count) * (k + 2), cudaMemcpyDeviceToHost,
                                    stream),
-                   "copy info bits");
-        check_cuda(cudaMemcpyAsync(b.h_used_osd.p, b.used_osd.p, b.count, cudaMemcpyDeviceToHost, stream),
-                   "copy used_osd");
-        check_cuda(cudaMemcpyAsync(b.h_success.p, b.success.p, b.count, cudaMemcpyDeviceToHost, stream),
-                   "copy success");
+                   "copy results");
         check_cuda(cudaEventRecord(b.done, stream), "cudaEventRecord");
         b.in_flight = true;
         flight.push_back(filling);
@@ -396,8 +393,8 @@ struct StreamDecoder : Decoder {
         Batch& b = *batches[id];
         for (auto& sg : ready) {
             if (sg.batch != id) continue;
-            sg.info.assign(b.h_info.p, b.h_info.p + static_cast<size_t>(b.count) * k);
-            sg.used.assign(b.h_used_osd.p, b.h_used_osd.p + b.count);
+            sg.info.assign(b.h_out.p, b.h_out.p + static_cast<size_t>(b.count) * k);
+            sg.used.assign(b.h_used_osd(k), b.h_used_osd(k) + b.count);
             sg.ts = b.ts;
             sg.ids = b.ids;
             sg.blocks = b.blocks;
@@ -418,8 +415,8 @@ struct StreamDecoder : Decoder {
         sg.batch = id;
         sg.count = static_cast<size_t>(b.count);
         for (int i = 0; i < b.count; ++i) {
-            stats.osd_fallback_codewords += b.h_used_osd.p[i] ? 1 : 0;
-            stats.bp_success_codewords += b.h_success.p[i] ? 1 : 0;
+            stats.osd_fallback_codewords += b.h_used_osd(k)[i] ? 1 : 0;
+            stats.bp_success_codewords += b.h_success(k)[i] ? 1 : 0;
         }
         ready.push_back(std::move(sg));
         stats.decoded_codewords += static_cast<unsigned long long>(b.count);
@@ -510,13 +507,18 @@ struct StreamDecoder : Decoder {
             stats.submitted_codewords += static_cast<unsigned long long>(take);
             if (b.count >= max_batch) launch_filling();
         }
-        // the caller may reuse its buffer as soon as this returns
         check_cuda(cudaEventRecord(copied, copy_stream), "cudaEventRecord(copy)");
-        check_cuda(cudaEventSynchronize(copied), "synchronize submit copy");
         stats.last_submit_timestamp_us = ts && count > 0 ? ts[count - 1] : now;
         stats.current_pending_codewords = pending();
         stats.max_pending_codewords = std::max(stats.max_pending_codewords, stats.current_pending_codewords);
+        // a batch that is due is launched while the copy runs; the caller may reuse its buffer as soon
+        // as this returns, so the copy is waited for also when the launch throws
+        struct Copied {
+            cudaEvent_t ev;
+            ~Copied() { cudaEventSynchronize(ev); }
+        } wait{copied};
         maybe_launch();
+        check_cuda(cudaEventSynchronize(copied), "synchronize submit copy");
     }
 
     int poll(int max_cw, unsigned char* out_info, unsigned long long* out_ts, unsigned long long* out_ids,
@@ -535,8 +537,8 @@ struct StreamDecoder : Decoder {
         while (out < max_cw && !ready.empty()) {
             ReadySeg& sg = ready.front();
             Batch* b = sg.batch >= 0 ? batches[sg.batch].get() : nullptr;
-            const uint8_t* info = b ? b->h_info.p : sg.info.data();
-            const uint8_t* used = b ? b->h_used_osd.p : sg.used.data();
+            const uint8_t* info = b ? b->h_out.p : sg.info.data();
+            const uint8_t* used = b ? b->h_used_osd(k) : sg.used.data();
             const unsigned long long* ts = b ? b->ts.data() : sg.ts.data();
             const unsigned long long* ids = b ? b->ids.data() : sg.ids.data();
             const unsigned* blocks = b ? b->blocks.data() : sg.blocks.data();
