@@ -49,9 +49,10 @@ namespace sicc {
 
 namespace {
 
-constexpr int kSyncThreads = 256;
+constexpr int kSyncThreads = 512;
+constexpr int kSyncOwners = 256;  // threads that own a chunk of coarse candidates
 constexpr int kSyncChunk = 17;
-constexpr int kSyncPass = kSyncThreads * kSyncChunk;
+constexpr int kSyncPass = kSyncOwners * kSyncChunk;
 constexpr int kMaxRefine = 1024;  // 2 * radius + 1
 constexpr int kMaxRadius = 511;
 
@@ -138,11 +139,11 @@ struct SyncShared {
     float2* win;      // [kSyncPass + pre_len] the pass's samples (rounded up to an even count: the
                       // float4 block sums after the metric stay 16-byte aligned)
     float* metric;    // [kSyncPass] coarse metric
-    float4* block;    // [kSyncThreads + L / kSyncChunk] sums over 17 samples: P.re, P.im, E1, E2;
+    float4* block;    // [kSyncOwners + L / kSyncChunk] sums over 17 samples: P.re, P.im, E1, E2;
                       // before the metric is complete, in memo's place
     float* memo;      // [kSyncPass + 2 * radius] fine metric around crossings
     uint16_t* list;   // [memo / 4] groups of four memo positions to evaluate, in increasing order
-    float* red;       // [4][kSyncThreads / 32] reductions
+    float* red;       // [4][kSyncOwners / 32] reductions
     float* rmetric;   // [kMaxRefine] mode-1 refinement
     int* s_key;       // [kSyncThreads / 32 + 2]
     PassResult* s_res;
@@ -152,7 +153,7 @@ __host__ __device__ inline int sync_memo(int radius) { return (kSyncPass + 2 * r
 __host__ __device__ inline size_t sync_memo_bytes(int pre_len, int radius)
 {  // the fine metrics, or the block sums before them
     const size_t memo = static_cast<size_t>(sync_memo(radius)) * sizeof(float);
-    const size_t block = static_cast<size_t>(kSyncThreads + pre_len / 2 / kSyncChunk) * sizeof(float4);
+    const size_t block = static_cast<size_t>(kSyncOwners + pre_len / 2 / kSyncChunk) * sizeof(float4);
     return memo > block ? memo : block;
 }
 __host__ __device__ inline size_t sync_smem(int pre_len, int radius)
@@ -191,7 +192,7 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
     for (int i = tid; i < kSyncPass + pre; i += kSyncThreads) sh.win[i] = (i < span) ? x[base + i] : make_float2(0.f, 0.f);
     __syncthreads();
     // chunks holding candidates below the limit (the rest only hold -1)
-    const int nchunks = min(kSyncThreads, (limit - base + kSyncChunk - 1) / kSyncChunk);
+    const int nchunks = min(kSyncOwners, (limit - base + kSyncChunk - 1) / kSyncChunk);
     const int nb = L / kSyncChunk;
     for (int t = tid; t < nchunks + nb; t += kSyncThreads) {
         float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -206,7 +207,9 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
         sh.block[t] = w;
     }
     __syncthreads();
-    if (tid >= nchunks) {
+    if (tid >= kSyncOwners) {
+        // the other threads share in the loads, the block sums and the fine metric
+    } else if (tid >= nchunks) {
         for (int c = 0; c < kSyncChunk; ++c) sh.metric[tid * kSyncChunk + c] = -1.0f;
     } else {
         const int d0 = tid * kSyncChunk;
@@ -243,7 +246,7 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
         // maximum of the pass, first occurrence (strict >)
         float bm = -1.0f;
         int bd = 0x7fffffff;
-        for (int c = 0; c < kSyncChunk; ++c) {
+        for (int c = 0; c < kSyncChunk && tid < kSyncOwners; ++c) {
             const int d = tid * kSyncChunk + c;
             const float m = sh.metric[d];
             if (m > bm) { bm = m; bd = d; }
@@ -253,10 +256,10 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
             const int od = __shfl_xor_sync(0xffffffffu, bd, o);
             if (om > bm || (om == bm && od < bd)) { bm = om; bd = od; }
         }
-        if (lane == 0) { sh.red[warp] = bm; sh.red[8 + warp] = __int_as_float(bd); }
+        if (lane == 0 && tid < kSyncOwners) { sh.red[warp] = bm; sh.red[8 + warp] = __int_as_float(bd); }
         __syncthreads();
         if (tid == 0) {
-            for (int w = 0; w < kSyncThreads / 32; ++w) {
+            for (int w = 0; w < kSyncOwners / 32; ++w) {
                 const float m = sh.red[w];
                 const int d = __float_as_int(sh.red[8 + w]);
                 if (d == 0x7fffffff) continue;  // no valid candidate in that warp's chunks
@@ -351,7 +354,7 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
         }
         // the crossing: memo index x is sample base - R + x, so candidates d in [x - 2R, x]
         const int xo = *first_over;
-        if (every || xo != 0x7fffffff) {
+        if (tid < kSyncOwners && (every || xo != 0x7fffffff)) {
             for (int c = 0; c < kSyncChunk; ++c) {
                 const int d = tid * kSyncChunk + c;
                 if (sh.metric[d] >= p.threshold && (every || (d >= xo - 2 * R && d <= xo))) {
@@ -433,18 +436,18 @@ __device__ SyncOut sync_finish(const float2* __restrict__ x, int avail, int limi
     if (res.found == 1 || res.found == 2) {  // an incomplete frame also gets its CFO (for one-frame buffers)
         const int s0 = res.start;
         float ar = 0.f, ai = 0.f;
-        for (int i = tid; i < L; i += kSyncThreads) {
+        for (int i = tid; i < L && tid < kSyncOwners; i += kSyncOwners) {
             const float2 c = cmulconj(x[s0 + i + L], x[s0 + i]);  // conj(x[s0+i]) * x[s0+i+L]
             ar += c.x;
             ai += c.y;
         }
         ar = warp_sum(ar);
         ai = warp_sum(ai);
-        if (lane == 0) { sh.red[16 + warp] = ar; sh.red[24 + warp] = ai; }
+        if (lane == 0 && tid < kSyncOwners) { sh.red[16 + warp] = ar; sh.red[24 + warp] = ai; }
         __syncthreads();
         if (tid == 0) {
             float sr = 0.f, si = 0.f;
-            for (int w = 0; w < kSyncThreads / 32; ++w) { sr += sh.red[16 + w]; si += sh.red[24 + w]; }
+            for (int w = 0; w < kSyncOwners / 32; ++w) { sr += sh.red[16 + w]; si += sh.red[24 + w]; }
             res.cfo_hz = atan2f(si, sr) * p.sample_rate / (2.0f * 3.14159265358979323846f * static_cast<float>(L));
         }
     }
@@ -471,7 +474,7 @@ sync_kernel(const float2* __restrict__ samples, long long stride, const long lon
             const int* __restrict__ frames_ptr)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ float red[4 * (kSyncThreads / 32)];
+    __shared__ float red[4 * (kSyncOwners / 32)];
     __shared__ float rmetric[kMaxRefine];
     __shared__ int s_key[kSyncThreads / 32 + 2];
     __shared__ PassResult s_res;
@@ -553,7 +556,7 @@ ingest_extract_kernel(const float2* __restrict__ window, int n, const float2* __
                       IngestRecord* __restrict__ rec, IngestState* __restrict__ state)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ float red[4 * (kSyncThreads / 32)];
+    __shared__ float red[4 * (kSyncOwners / 32)];
     __shared__ float rmetric[kMaxRefine];
     __shared__ int s_key[kSyncThreads / 32 + 2];
     __shared__ PassResult s_res;
@@ -640,7 +643,7 @@ ingest_extract_kernel(const float2* __restrict__ window, int n, const float2* __
 static size_t sync_smem_limit(int pre_len)
 {
     return static_cast<size_t>((kSyncPass + pre_len + 1) & ~1) * sizeof(float2) + static_cast<size_t>(kSyncPass) * sizeof(float) +
-           kSyncThreads * sizeof(float4) + static_cast<size_t>(kSyncPass + 2 * kMaxRadius) * sizeof(float);
+           kSyncOwners * sizeof(float4) + static_cast<size_t>(kSyncPass + 2 * kMaxRadius) * sizeof(float);
 }
 
 static long long sync_passes(long long stride, const int* counts, int count, const SyncParams& p)
