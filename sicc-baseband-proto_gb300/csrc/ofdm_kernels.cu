@@ -110,27 +110,75 @@ __device__ __forceinline__ float fine_metric(const float2* __restrict__ x, const
     return (cr * cr + ci * ci) / fmaxf(eng * pre_energy, 1e-18f);
 }
 
-// fine_metric of the positions dd .. dd + 3, all inside the shared window (at win + at): the same
-// sums, with one read of the preamble for the four.
+// Samples of the preamble's first half, a multiple of a warp's 32.
+__device__ __forceinline__ int fine_half(int pre) { return (pre >> 6) << 5; }
+
+// fine_metric of the positions dd .. dd + 3, all inside the shared window (at win + at), pre >= 4,
+// with one read of the preamble for the four and one energy sum: the samples common to the four,
+// then each position's own ones (sums of non-negative terms only).  After the first half of the
+// preamble |c| <= |c1| + sqrt(e2 E2) (e2, E2: energies of the other half of the samples and of the
+// preamble), widened by 1e-5 of sqrt(e E) for the rounding of the sums (at most 40 of 6e-8 each for
+// the lengths that fit); when that puts all four below the threshold they are reported as -1 and the
+// other half is not correlated.  Away from the preamble c1 is small and the bound about 1/4: most
+// groups stop there (256 frames at threshold 0.45, search
+// and demodulation: 120 us without the early stop and the shared energy, 106 with them).
 __device__ __forceinline__ void fine_metric4(const float2* win, int at, const float2* __restrict__ preamble, int pre,
-                                             float pre_energy, int lane, float (&out)[4])
+                                             float pre_energy, float tail_energy, float threshold, int lane,
+                                             float (&out)[4])
 {
-    float cr[4] = {0.f, 0.f, 0.f, 0.f}, ci[4] = {0.f, 0.f, 0.f, 0.f}, eng[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-    for (int i = lane; i < pre; i += 32) {
+    float cr[4] = {0.f, 0.f, 0.f, 0.f}, ci[4] = {0.f, 0.f, 0.f, 0.f}, e1 = 0.f, e2 = 0.f;
+    const float2* y0 = win + at;
+    auto correlate = [&](int i) {
         const float2 q = __ldg(preamble + i);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float2 y = win[at + i + k];
+            const float2 y = y0[i + k];
             cr[k] = fmaf(y.x, q.x, fmaf(y.y, q.y, cr[k]));
             ci[k] = fmaf(y.y, q.x, fmaf(-y.x, q.y, ci[k]));
-            eng[k] = fmaf(y.x, y.x, fmaf(y.y, y.y, eng[k]));
         }
+    };
+    auto energy = [&](int i, float e) { return fmaf(y0[i].x, y0[i].x, fmaf(y0[i].y, y0[i].y, e)); };
+    const int half = fine_half(pre);
+    int i = lane;
+#pragma unroll 2
+    for (; i < half; i += 32) {
+        correlate(i);
+        if (i > 2) e1 = energy(i, e1);
     }
+#pragma unroll 4
+    for (int t = i; t < pre; t += 32)
+        if (t > 2) e2 = energy(t, e2);
+    e2 = warp_sum(e2);
+    const float common = warp_sum(e1) + e2;
+    float eng[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float r = warp_sum(cr[k]), j = warp_sum(ci[k]), e = warp_sum(eng[k]);
-        out[k] = (r * r + j * j) / fmaxf(e * pre_energy, 1e-18f);
+        eng[k] = common;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) eng[k] = energy(j >= k ? j : pre + j, eng[k]);
+    }
+    float over = e2;  // at least each position's energy against the preamble's other half
+#pragma unroll
+    for (int j = 0; j < 3; ++j) over = energy(pre + j, over);
+    const float rest = sqrtf(over * tail_energy);
+    bool below = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float r = warp_sum(cr[k]), j = warp_sum(ci[k]), full = eng[k] * pre_energy;
+        const float most = sqrtf(r * r + j * j) + rest + 1e-5f * sqrtf(full);
+        below = below && most * most < threshold * fmaxf(full, 1e-18f);
+    }
+    if (__all_sync(0xffffffffu, below)) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) out[k] = -1.0f;
+        return;
+    }
+#pragma unroll 2
+    for (; i < pre; i += 32) correlate(i);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float r = warp_sum(cr[k]), j = warp_sum(ci[k]);
+        out[k] = (r * r + j * j) / fmaxf(eng[k] * pre_energy, 1e-18f);
     }
 }
 
@@ -146,6 +194,7 @@ struct SyncShared {
     float* red;       // [4][kSyncOwners / 32] reductions
     float* rmetric;   // [kMaxRefine] mode-1 refinement
     int* s_key;       // [kSyncThreads / 32 + 2]
+    float* s_tail;    // energy of the preamble's other half (fine_metric4)
     PassResult* s_res;
 };
 
@@ -163,7 +212,7 @@ __host__ __device__ inline size_t sync_smem(int pre_len, int radius)
 }
 
 __device__ __forceinline__ SyncShared sync_shared(unsigned char* smem_raw, int pre_len, int radius, float* red,
-                                                  float* rmetric, int* s_key, PassResult* s_res)
+                                                  float* rmetric, int* s_key, float* s_tail, PassResult* s_res)
 {
     SyncShared sh;
     sh.win = reinterpret_cast<float2*>(smem_raw);
@@ -174,6 +223,7 @@ __device__ __forceinline__ SyncShared sync_shared(unsigned char* smem_raw, int p
     sh.red = red;
     sh.rmetric = rmetric;
     sh.s_key = s_key;
+    sh.s_tail = s_tail;
     sh.s_res = s_res;
     return sh;
 }
@@ -209,6 +259,15 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
     __syncthreads();
     if (tid >= kSyncOwners) {
         // the other threads share in the loads, the block sums and the fine metric
+        if (warp == kSyncOwners / 32) {
+            float e = 0.f;
+            for (int i = fine_half(pre) + lane; i < pre; i += 32) {
+                const float2 q = __ldg(preamble + i);
+                e = fmaf(q.x, q.x, fmaf(q.y, q.y, e));
+            }
+            e = warp_sum(e);
+            if (lane == 0) *sh.s_tail = e;
+        }
     } else if (tid >= nchunks) {
         for (int c = 0; c < kSyncChunk; ++c) sh.metric[tid * kSyncChunk + c] = -1.0f;
     } else {
@@ -326,8 +385,8 @@ __device__ void sync_scan_pass(const float2* __restrict__ x, int avail, int limi
             if (b + warp < total) {
                 const int i0 = 4 * sh.list[b + warp], x0 = base - R + i0;
                 float m[4];
-                if (x0 >= base && x0 + 3 + pre <= base + span) {
-                    fine_metric4(sh.win, x0 - base, preamble, pre, p.pre_energy, lane, m);
+                if (pre >= 4 && x0 >= base && x0 + 3 + pre <= base + span) {
+                    fine_metric4(sh.win, x0 - base, preamble, pre, p.pre_energy, *sh.s_tail, p.threshold, lane, m);
                 } else {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
@@ -477,9 +536,10 @@ sync_kernel(const float2* __restrict__ samples, long long stride, const long lon
     __shared__ float red[4 * (kSyncOwners / 32)];
     __shared__ float rmetric[kMaxRefine];
     __shared__ int s_key[kSyncThreads / 32 + 2];
+    __shared__ float s_tail;
     __shared__ PassResult s_res;
     __shared__ int s_flag;
-    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_res);
+    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_tail, &s_res);
 
     // pass-major order: the first passes of all frames run first, so later
     // passes of a frame found early skip their scans
@@ -559,10 +619,11 @@ ingest_extract_kernel(const float2* __restrict__ window, int n, const float2* __
     __shared__ float red[4 * (kSyncOwners / 32)];
     __shared__ float rmetric[kMaxRefine];
     __shared__ int s_key[kSyncThreads / 32 + 2];
+    __shared__ float s_tail;
     __shared__ PassResult s_res;
     __shared__ SyncOut s_out;
     __shared__ IngestState s_st;
-    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_res);
+    const SyncShared sh = sync_shared(smem_raw, p.pre_len, p.radius, red, rmetric, s_key, &s_tail, &s_res);
     const int tid = threadIdx.x;
     if (tid == 0) {
         s_st = *state;

@@ -274,3 +274,28 @@ def test_mixed_shapes(cuda, oracle, more):
         o = ocs[ci].layered(x, 8, 0.8, 0.1)
         assert gok[i] == o[0] and git[i] == o[4], (ci, i)
         assert np.array_equal(got[io[i]:io[i] + cs[ci].k], o[1][: cs[ci].k]), (ci, i)
+
+
+@pytest.mark.parametrize("threshold", [0.02, 0.2, 0.7, 0.93])
+def test_search_thresholds(cuda, oracle, threshold):
+    """Early stop of the fine metric: low and high thresholds, bursts of strong samples around the frame."""
+    from sicc_gb300.pipeline import SYNC_RECORD, RxPipeline
+    torch = cuda
+    t, code = ofdm.reference_tables(ofdm.PhyConfig(nfft=64, cp=8, num_symbols=6, active_sc=32, pilot_period=3, pre_half_len=97,
+                                                   modulation="qpsk", sync_threshold=threshold)), codes.short_code()
+    b = ofdm.FrameGenerator(t, code, seed=23).batch(12, snr_db=20.0, cfo_subcarriers=0.05, max_offset=400, rayleigh_taps=0)
+    rng = np.random.default_rng(5)
+    for f in range(0, 12, 3):
+        at = rng.integers(0, b.iq.shape[1], 20)
+        b.iq[f, at] *= np.float32(50.0)
+    p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, float(b.noise_var[0]), max_batch_frames=12)
+    llr = torch.zeros((12, p.coded_bits), dtype=torch.float32, device="cuda")
+    rec = torch.zeros(12 * SYNC_RECORD.itemsize, dtype=torch.uint8, device="cuda")
+    p.demod_batch(torch.from_numpy(b.iq).cuda(), b.iq.shape[1], b.iq.shape[1], 12, llr, rec, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    sync, ph = rec.cpu().numpy().view(SYNC_RECORD), oracle.phy(t)
+    for f in range(12):
+        r = oracle.sync_earliest(ph, b.iq[f])
+        assert sync[f]["found"] == r[0], f
+        if r[0]:
+            assert sync[f]["start"] == r[1], f
