@@ -153,23 +153,27 @@ struct WideRow {
 };
 
 // Threads: as many as the rows' registers allow without spills in the row loop (they hide the L2
-// latency of tables and messages).  608 codewords of (64800,32400), D = 7: 768 threads 6.41 ms,
-// 1,024 (64 registers, spilling) 6.83; 600 of (16200,3240), D = 4: 2.58 and 2.35.
+// latency of tables and messages).  608 codewords of (64800,32400), D = 7: 768 threads 5.28 ms, 896
+// 5.09, 1,024 5.15; 600 of (16200,13320), D = 18: 512 threads 0.38 ms, 576 (spilling) 0.41.
 template <int D>
 constexpr int wide_threads() { return D <= 4 ? 1024 : D <= 7 ? 896 : D <= 10 ? 768 : 512; }
 
 }  // namespace
 
 // The next row's offsets and messages are loaded while the current one is updated, across the
-// layer barriers too: they do not depend on posteriors.  Slots below cv.wide_smem_slots hold
-// shared-memory posteriors in every row (columns ascend within a row, so for the accumulator
-// codes only the parity slots can lie beyond the split): only the others test.  Without
+// layer barriers too: they do not depend on posteriors.  Slots below D - kFar hold shared-memory
+// posteriors in every row (columns ascend within a row, so for the accumulator codes only the
+// two parity slots can lie beyond the split): only the last kFar (0, 2 or D) test.  A run-time
+// bound put a branch before every access and cost 6.42 against 5.28 ms on the code below.
+// Up to 4 slots a row keeps its messages as they are, in the 16 bytes that the compressed form
+// takes ((16200,3240): 1.99 against 1.76 ms); for 7 slots that form outgrows L2 (7.4 ms).  Without
 // best-syndrome tracking only "zero syndrome or not" matters, so the check stops at the first
 // layer with an unsatisfied row.
 //
 // Measured on GB300, 608 codewords of (64800,32400) at 2 dB: 12.1 ms before (512 threads, a
 // branch per posterior access, variable indices slot by slot, (min1, min2, argmin) row
-// arithmetic, full syndrome: 78 instructions per edge and iteration), 6.41 ms now.
+// arithmetic, full syndrome: 78 instructions per edge and iteration), 5.10 ms now (31); the last
+// SM runs 76 iterations, the average one 55.
 template <int D, int kFar>
 __global__ void __launch_bounds__(wide_threads<D>(), 1)
 bp_layered_wide_kernel(LayeredView cv, BpParams p, BpIO io, float* scratch, long long slice, int split, int track_best)

@@ -14,13 +14,15 @@
 //     thread slides it over its 17 candidates (30 block sums instead of 512
 //     products per chunk at L = 512);
 //   * the fine metric is computed for four neighbouring positions at a time (one
-//     read of the preamble for four), in increasing order, and only as far as
-//     the earliest position over the threshold decides the search.
+//     read of the preamble and one energy sum for four), in increasing order, only
+//     as far as the earliest position over the threshold decides the search, and
+//     over half the preamble where the other half cannot reach the threshold.
 // Every pass publishes its result to global scratch and the last pass of a
 // frame to finish resolves the frame.  Measured on GB300, 256 frames of 16,888
 // samples (1,024-sample preamble, 6-tap fading): 243 us with a product per
-// sample and chunk and every position's fine metric, 77 us now; it stays
-// bound by instruction issue (the fine correlations).
+// sample and chunk and every position's fine metric, 57 us now (77 with the whole
+// preamble everywhere on 256 threads); a frame's pass is one CTA, so it is bound by
+// issue (57%) and by the barriers between its phases.
 //
 // demod_kernel (grid = frames x data-symbol groups) fuses the demodulator of
 // gpu_ofdm_pipeline.cu:566-672 / uhd_ldpc_ofdm_link.cpp:5350-5521: CFO
