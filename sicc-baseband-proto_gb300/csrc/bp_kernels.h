@@ -67,7 +67,7 @@ struct OsdHBounds {
     bool empty() const { return nmax == 0; }
 };
 // The large-code OSD runs in classes by m, each with the shared memory its longest code needs, so that
-// up to m = 640 two CTAs of 256 threads share an SM (a round's serial pivot choice leaves issue slots
+// up to m = 640 two CTAs of 320 threads share an SM (a round's serial pivot choice leaves issue slots
 // that only another CTA fills); above, T fills the SM's shared memory and a CTA has 512 threads.
 constexpr int kOsdHClasses = 4;
 constexpr int kOsdHClassMaxM[kOsdHClasses] = {256, 512, 640, 1024};

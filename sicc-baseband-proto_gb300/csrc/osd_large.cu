@@ -37,9 +37,12 @@ namespace sicc {
 
 namespace {
 
-// CTA size by class.  128 threads for m <= 256 was no better: 500 codewords of 27 mixed codes 520 us
-// against 510, 20,000 the same within the runs.
-constexpr int kOsdHClassThreads[kOsdHClasses] = {256, 256, 256, 512};
+// CTA size by class: with at least nine warps each worker reduces one of a round's eight candidates.
+// 500 and 20,000 codewords of 15 mixed codes, narrow / wide: 256 / 512 497 us and 4.18 ms, 288 / 512
+// 465 and 4.14, 320 / 512 454 and 4.16, 384 / 640 467 and 4.33, 320 / 640 452 and 4.26.
+constexpr int kOsdHNarrow = 320, kOsdHWide = 512;
+constexpr int kOsdHClassThreads[kOsdHClasses] = {kOsdHNarrow, kOsdHNarrow, kOsdHNarrow, kOsdHWide};
+constexpr int kOsdHMaxWarps = kOsdHWide / 32;
 constexpr int kOsdHMaxPool = 128;
 constexpr int kRound = 8;  // columns of H per elimination round
 constexpr int kTabStride = 33;  // words per table entry: lanes reading different entries hit different banks
@@ -94,7 +97,7 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
     OsdHSmem t{};
     {  // the sort keys, then T (the keys are dead once the sorted order is extracted)
         const size_t bt = (rows + 2 * kRound) * l.ts * 4, bk = static_cast<size_t>(l.np) * 8;
-        const size_t bc = (l.mw * 128 + 16 * osd_h_terms(l.mw)) * sizeof(float);  // nibble sums, 16 warps' terms
+        const size_t bc = (l.mw * 128 + kOsdHMaxWarps * osd_h_terms(l.mw)) * sizeof(float);  // nibble sums, the warps' terms
         const size_t most = bt > bk ? bt : bk;
         unsigned char* g = take(most > bc ? most : bc);
         t.T = reinterpret_cast<uint32_t*>(g);
@@ -132,7 +135,7 @@ __host__ __device__ inline size_t carve(const OsdHLayout& l, unsigned char* base
 __device__ __forceinline__ unsigned tbit(const uint32_t* row, int q) { return (row[q >> 5] >> (q & 31)) & 1u; }
 
 // CTAs per SM the registers are bounded for (shared memory sets the same or less).
-constexpr int osd_h_ctas(int threads) { return threads == 256 ? 2 : 1; }
+constexpr int osd_h_ctas(int threads) { return threads < 512 ? 2 : 1; }
 
 }  // namespace
 
@@ -261,7 +264,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
         //      rows (e_p + U_p), meet on a named barrier and reduce round k+1's candidates against T,
         //      whose rows they fetched from H during round k-1.
         // Warp 0's chain takes about 2,000 cycles of a round, the step before it 700-1,000; with the
-        // rows fetched at the reduction instead, staged in shared memory, 500 codewords of 27 mixed
+        // rows fetched at the reduction instead, staged in shared memory, 500 codewords of 15 mixed
         // codes took 533 us (500 now; 20,000 took the same 4.2 ms).  Tables and indices built by the
         // other warps in 2 instead of by all in 1: 512 us and 4.25 ms.  Windows of 16 candidates to
         // fill each round with 8 pivots: 538 us and 4.8 ms.
@@ -449,10 +452,12 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                     }
                 }
                 if (pending && pnp > 0) {
-                    // a warp takes 32 columns, and above 16 words a half of their words: smaller pieces
+                    // a warp takes 32 columns, and above 24 words a half of their words: smaller pieces
                     // share out better (three loads and a store per word: shared-memory bandwidth
-                    // bounds this at m = 1024)
-                    const int halves = MW > 16 ? 2 : 1, per = ((MW + halves - 1) / halves + 3) & ~3;
+                    // bounds this at m = 1024; pieces of 8 words cost more than they spread: 4.50 ms
+                    // and 499 us on the mixes above, against 4.14 and 448; halves from 17 words on 4.15
+                    // and 455)
+                    const int halves = MW > 24 ? 2 : 1, per = ((MW + halves - 1) / halves + 3) & ~3;
                     for (int piece = warp - 1; piece < ((pt + 31) >> 5) * halves; piece += kWarps - 1) {
                         const int at = (halves == 2 ? piece >> 1 : piece) * 32 + lane;
                         const int w0 = halves == 2 ? (piece & 1) * per : 0, w1 = min(MW, w0 + per);
@@ -788,7 +793,7 @@ void launch_osd_h_class(const OsdHBounds& bd, int mlo, int mhi, const OsdIO& io_
     OsdHLayout l = osd_h_layout(bd, mlo, mhi);
     const size_t smem = carve(l, nullptr, nullptr);
     if (smem > 227 * 1024) throw InvalidArgument("large-code OSD tables exceed shared memory (m <= 1024, n <= 4096)");
-    // the 256-thread classes share this kernel with different sizes: the limit only grows
+    // the narrow classes share this kernel with different sizes: the limit only grows
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(osd_h_kernel<kThreads>), smem),
                "cudaFuncSetAttribute(osd_h)");
     int per_sm = 0;
@@ -844,8 +849,8 @@ void launch_osd_h(const OsdHBounds* cls, const OsdIO& io, int max_items, cudaStr
             check_cuda(cudaStreamWaitEvent(cs, fork, 0), "cudaStreamWaitEvent(osd fork)");
         }
         const int mlo = c == 0 ? 0 : kOsdHClassMaxM[c - 1];
-        if (kOsdHClassThreads[c] == 256) launch_osd_h_class<256>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
-        else launch_osd_h_class<512>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
+        if (kOsdHClassThreads[c] == kOsdHNarrow) launch_osd_h_class<kOsdHNarrow>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
+        else launch_osd_h_class<kOsdHWide>(cls[c], mlo, kOsdHClassMaxM[c], io, max_items, cs, c);
         if (fan && used > 0) {
             check_cuda(cudaEventRecord(join[used - 1], cs), "cudaEventRecord(osd join)");
             check_cuda(cudaStreamWaitEvent(st, join[used - 1], 0), "cudaStreamWaitEvent(osd join)");
