@@ -452,23 +452,18 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                     }
                 }
                 if (pending && pnp > 0) {
-                    // a warp takes 32 columns, and above 24 words a half of their words: smaller pieces
-                    // share out better (three loads and a store per word: shared-memory bandwidth
-                    // bounds this at m = 1024; pieces of 8 words cost more than they spread: 4.50 ms
-                    // and 499 us on the mixes above, against 4.14 and 448; halves from 17 words on 4.15
-                    // and 455)
-                    const int halves = MW > 24 ? 2 : 1, per = ((MW + halves - 1) / halves + 3) & ~3;
-                    for (int piece = warp - 1; piece < ((pt + 31) >> 5) * halves; piece += kWarps - 1) {
-                        const int at = (halves == 2 ? piece >> 1 : piece) * 32 + lane;
-                        const int w0 = halves == 2 ? (piece & 1) * per : 0, w1 = min(MW, w0 + per);
-                        if (at >= pt) continue;
+                    // a thread takes a whole column (three loads and a store per word).  Splitting a
+                    // column's words over threads does not pay: pieces of 8 words took 4.50 ms and
+                    // 499 us on the mixes above, halves from 25 words on 4.14 and 447, whole columns 4.07
+                    // and 432.
+                    for (int at = tid - 32; at < pt; at += kThreads - 32) {
                         uint32_t* c = s.T + at * TS;
                         const unsigned idx = s.tidx[at];
                         if (idx == 0u) continue;
                         const uint32_t* lo = s.tab + (idx & 15u) * kTabStride;
                         const uint32_t* hi = s.tab + (16u + (idx >> 4)) * kTabStride;
-                        int w = w0;
-                        for (; w + 4 <= w1; w += 4) {
+                        int w = 0;
+                        for (; w + 4 <= MW; w += 4) {
                             const unsigned a0 = c[w] ^ lo[w] ^ hi[w];
                             const unsigned a1 = c[w + 1] ^ lo[w + 1] ^ hi[w + 1];
                             const unsigned a2 = c[w + 2] ^ lo[w + 2] ^ hi[w + 2];
@@ -478,7 +473,7 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
                             c[w + 2] = a2;
                             c[w + 3] = a3;
                         }
-                        for (; w < w1; ++w) c[w] ^= lo[w] ^ hi[w];
+                        for (; w < MW; ++w) c[w] ^= lo[w] ^ hi[w];
                     }
                     for (int r = warp - 1; r < kRound; r += kWarps - 1) {  // the pivot rows' columns: e_p + U_p
                         const int p = s_rp[pb][r];
