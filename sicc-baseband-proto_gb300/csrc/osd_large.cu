@@ -38,8 +38,9 @@ namespace sicc {
 namespace {
 
 // CTA size by class: with at least nine warps each worker reduces one of a round's eight candidates.
-// 500 and 20,000 codewords of 15 mixed codes, narrow / wide: 256 / 512 497 us and 4.18 ms, 288 / 512
-// 465 and 4.14, 320 / 512 454 and 4.16, 384 / 640 467 and 4.33, 320 / 640 452 and 4.26.
+// 500 and 20,000 codewords of 15 mixed codes, narrow / wide: 288 / 512 446 us and 4.03 ms, 320 / 512
+// 433 and 4.04, 320 / 384 433 and 4.11, 320 / 448 432 and 4.18, 352 / 576 450 and 4.17 (256 / 512 was
+// 32 us and 0.04 ms slower than 288 / 512).
 constexpr int kOsdHNarrow = 320, kOsdHWide = 512;
 constexpr int kOsdHClassThreads[kOsdHClasses] = {kOsdHNarrow, kOsdHNarrow, kOsdHNarrow, kOsdHWide};
 constexpr int kOsdHMaxWarps = kOsdHWide / 32;
