@@ -314,11 +314,12 @@ struct Group {
     }
 };
 
-// Channel values of codeword c into app (canonical) and, when given, a plain copy.
+// Channel values of codeword c into app (canonical) and, when given, a plain copy.  The caller's array
+// may start at any float (the rows then all start equally far from a 16-byte boundary).
 __device__ __forceinline__ void load_llr(const BpIO& io, int c, int n, int gl, int G, float* app, float* plain)
 {
     const float* src = io.llr + static_cast<size_t>(c) * n;
-    if ((n & 3) == 0) {
+    if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
         const float4* s4 = reinterpret_cast<const float4*>(src);
         for (int i = gl; i < (n >> 2); i += G) {
             const float4 v = __ldcs(s4 + i);

@@ -1,0 +1,63 @@
+"""Calls that the entry points accept, at the edges of what the fast paths take.
+
+Each of them is a form that a general path answered before a faster kernel took over its sizes: arrays
+that start away from a 16-byte boundary.  Results are compared with the same call in its ordinary form.
+"""
+import numpy as np
+import pytest
+
+from sicc_gb300 import channel, codes, fec
+
+pytestmark = pytest.mark.gpu
+
+
+# --- soft values away from a 16-byte boundary ---------------------------------------------------------
+
+def _decode(torch, dec, d_llr, n):
+    b = d_llr.shape[0]
+    out = [torch.zeros((b, n), dtype=torch.uint8, device="cuda"), torch.zeros(b, dtype=torch.uint8, device="cuda"),
+           torch.zeros((b, n), dtype=torch.float32, device="cuda"), torch.zeros(b, dtype=torch.uint8, device="cuda")]
+    dec.decode_device_batch(d_llr, *out, stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    return [x.cpu().numpy() for x in out]
+
+
+def _offset(torch, llr, floats):
+    """The rows as a view that starts `floats` floats into a buffer."""
+    buf = torch.zeros(llr.size + 4, dtype=torch.float32, device="cuda")
+    view = buf[floats:floats + llr.size].view(llr.shape)
+    view.copy_(torch.from_numpy(llr))
+    assert view.data_ptr() % 16 == 4 * floats
+    return view
+
+
+@pytest.mark.parametrize("floats", [1, 2, 3])
+@pytest.mark.parametrize("schedule", [fec.FLOODING, fec.NODE_PARALLEL, fec.COLORED_LAYERED, fec.FLAT_LAYERED])
+@pytest.mark.parametrize("base", [(4, 8, 16), (8, 16, 64), (8, 16, 128), (4, 8, 33)])
+def test_unaligned_soft_values_register_kernels(cuda, base, schedule, floats):
+    code = codes.qc_code(*base, seed=41)
+    llr = channel.awgn_llrs(code, 37, 2.0, 3)[2].astype(np.float32)
+    dec = fec.CsrBpDecoder.for_code(code, max_batch=37, max_iter=10, normalization=0.8, schedule=schedule)
+    want = _decode(cuda, dec, cuda.from_numpy(llr).cuda(), code.n)
+    for a, b in zip(want, _decode(cuda, dec, _offset(cuda, llr, floats), code.n)):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("schedule", [fec.NODE_PARALLEL, fec.FLAT_LAYERED])
+def test_unaligned_soft_values_stream_decoder(cuda, schedule):
+    """BP with its best posteriors kept for OSD."""
+    torch, code = cuda, codes.short_code()
+    llr = channel.awgn_llrs(code, 500, 2.0, 4)[2].astype(np.float32)
+    dec = fec.StreamBpOsdDecoder(code, max_batch=500, max_iter=20, schedule=schedule)
+
+    def run(d_llr):
+        out = [torch.zeros((500, code.k), dtype=torch.uint8, device="cuda")] + \
+              [torch.zeros(500, dtype=torch.uint8, device="cuda") for _ in range(3)]
+        dec.decode_device_batch(d_llr, *out, stream=torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        return [x.cpu().numpy() for x in out]
+
+    want = run(torch.from_numpy(llr).cuda())
+    assert want[2].any()  # some went through OSD
+    for a, b in zip(want, run(_offset(torch, llr, 1))):
+        assert np.array_equal(a, b)
