@@ -103,7 +103,7 @@ bp_layered_kernel(LayeredView cv, BpParams p, BpIO io, int slots_per_cta, int sl
 
     auto init = [&](int cw) {
         const float* src = io.llr + static_cast<size_t>(cw) * n;
-        if ((n & 3) == 0) {
+        if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {  // the caller's array may start at any float
             const float4* s4 = reinterpret_cast<const float4*>(src);
             for (int i = gl; i < (n >> 2); i += G) {
                 const float4 v = __ldcs(s4 + i);

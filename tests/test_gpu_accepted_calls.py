@@ -43,6 +43,18 @@ def test_unaligned_soft_values_register_kernels(cuda, base, schedule, floats):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("floats", [1, 2, 3])
+@pytest.mark.parametrize("base", [(6, 12, 64), (7, 14, 96)])
+def test_unaligned_soft_values_general_layered_kernel(cuda, base, floats):
+    """Codes whose rows fit no register-resident shape."""
+    code = codes.qc_code(*base, seed=41)
+    llr = channel.awgn_llrs(code, 37, 2.0, 3)[2].astype(np.float32)
+    dec = fec.CsrBpDecoder.for_code(code, max_batch=37, max_iter=10, normalization=0.8, schedule=fec.FLAT_LAYERED)
+    want = _decode(cuda, dec, cuda.from_numpy(llr).cuda(), code.n)
+    for a, b in zip(want, _decode(cuda, dec, _offset(cuda, llr, floats), code.n)):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("schedule", [fec.NODE_PARALLEL, fec.FLAT_LAYERED])
 def test_unaligned_soft_values_stream_decoder(cuda, schedule):
     """BP with its best posteriors kept for OSD."""
