@@ -1002,6 +1002,8 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
     unsigned phase = 0u;  // bit b: parity of buffer b's next completion
 
     float* out = llr + (llr_off ? llr_off[f] : static_cast<long long>(f) * llr_stride);
+    // a symbol's LLRs in one store where they align (the caller's array may start at any float)
+    const bool aligned = (bps == 2 || bps == 4) && (reinterpret_cast<uintptr_t>(out) & (sizeof(float) * bps - 1)) == 0;
     for (int i = 0; i < nsym; ++i) {
         const int b = i & 1;
         const int sym = sym_at(i);
@@ -1078,13 +1080,13 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
                     vals[abits + bb] =
                         __fmul_rn(__fsub_rn(__fadd_rn(mi_all, mq1[bb]), __fadd_rn(mi_all, mq0[bb])), inv_sig);
                 }
-                if constexpr (bps == 4) {
+                if (!aligned) {
+#pragma unroll
+                    for (int bb = 0; bb < bps; ++bb) o[bb] = vals[bb];
+                } else if constexpr (bps == 4) {
                     *reinterpret_cast<float4*>(o) = make_float4(vals[0], vals[1], vals[2], vals[3]);
                 } else if constexpr (bps == 2) {
                     *reinterpret_cast<float2*>(o) = make_float2(vals[0], vals[1]);
-                } else {
-#pragma unroll
-                    for (int bb = 0; bb < bps; ++bb) o[bb] = vals[bb];
                 }
             }
         }

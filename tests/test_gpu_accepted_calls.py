@@ -1,12 +1,12 @@
 """Calls that the entry points accept, at the edges of what the fast paths take.
 
 Each of them is a form that a general path answered before a faster kernel took over its sizes: arrays
-that start away from a 16-byte boundary.  Results are compared with the same call in its ordinary form.
+that start away from a 16-byte boundary (soft values in, LLRs out).  Results are compared with the same call in its ordinary form.
 """
 import numpy as np
 import pytest
 
-from sicc_gb300 import channel, codes, fec
+from sicc_gb300 import channel, codes, fec, ofdm
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +73,28 @@ def test_unaligned_soft_values_stream_decoder(cuda, schedule):
     assert want[2].any()  # some went through OSD
     for a, b in zip(want, run(_offset(torch, llr, 1))):
         assert np.array_equal(a, b)
+
+
+# --- OFDM receiver --------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("modulation", ["bpsk", "qpsk", "16qam", "64qam"])
+def test_gather_to_unaligned_llr_rows(cuda, modulation):
+    """demod_gather writes each frame's LLRs wherever the caller says, at any float."""
+    from sicc_gb300.pipeline import SYNC_RECORD, RxPipeline
+    torch = cuda
+    cfg = ofdm.PhyConfig(nfft=128, cp=16, num_symbols=8, active_sc=64, pre_half_len=64, modulation=modulation,
+                         pilot_period=4)
+    t, code = ofdm.reference_tables(cfg), codes.short_code()
+    b = ofdm.FrameGenerator(t, code, seed=5).batch(4, snr_db=25.0, cfo_subcarriers=0.05, max_offset=30, rayleigh_taps=0)
+    p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, float(b.noise_var[0]), max_batch_frames=4)
+    iq, n, st = torch.from_numpy(b.iq).cuda(), b.iq.shape[1], torch.cuda.current_stream()
+    sync = torch.zeros(4 * SYNC_RECORD.itemsize, dtype=torch.uint8, device="cuda")
+    want = torch.zeros((4, p.coded_bits), dtype=torch.float32, device="cuda")
+    p.demod_batch(iq, n, n, 4, want, sync, st)
+    rows = [f * (p.coded_bits + 4) + f for f in range(4)]  # 0 to 3 floats off
+    got = torch.zeros(4 * (p.coded_bits + 5), dtype=torch.float32, device="cuda")
+    p.demod_gather(iq, torch.arange(4, device="cuda") * n, n, 4, got, torch.tensor(rows, device="cuda"), sync, st)
+    torch.cuda.synchronize()
+    assert want.abs().sum() > 0
+    for f in range(4):
+        assert torch.equal(got[rows[f]:rows[f] + p.coded_bits], want[f]), f
