@@ -729,18 +729,18 @@ struct Engine {
         return (w + 3) & ~3;
     }
 
-    // Shared memory of a CTA of the mixed kernel.  The register-resident units hold 16-bit byte
-    // offsets into it, so with a larger CTA (a wide ragged code on one warp) no code runs so.
-    size_t mixed_smem()
+    // Shared memory of a CTA of the mixed kernel.
+    size_t mixed_smem() const { return static_cast<size_t>(kMixedWarps) * warp_floats() * sizeof(float); }
+
+    // Settles which codes run register-resident: every plain one at its default warps, unless the CTA
+    // then passes the 64 KB that the units' 16-bit byte offsets reach (a wide code on one warp); then
+    // none.  Decided anew for all codes from their warps alone, so that a shape tried once and given
+    // up leaves nothing behind.
+    void settle_reg()
     {
-        size_t smem = static_cast<size_t>(kMixedWarps) * warp_floats() * sizeof(float);
-        if (smem > 65536)
-            for (auto& c : codes)
-                if (c.desc.reg) {
-                    set_code_warps(c, c.desc.warps, false);
-                    dirty = true;
-                }
-        return static_cast<size_t>(kMixedWarps) * warp_floats() * sizeof(float);
+        for (auto& c : codes) set_code_warps(c, c.desc.warps);
+        if (mixed_smem() > 65536)
+            for (auto& c : codes) set_code_warps(c, c.desc.warps, false);
     }
 
     // Codewords a warp holds at once with its best posteriors in the global scratch.
@@ -756,7 +756,7 @@ struct Engine {
     void commit()
     {
         if (!dirty) return;
-        mixed_smem();  // settles which codes run register-resident
+        settle_reg();
         const int K = static_cast<int>(codes.size());
         std::vector<CodeDesc> descs(K);
         std::vector<OsdView> views(K);

@@ -6,7 +6,7 @@ that start away from a 16-byte boundary (soft values in, LLRs out).  Results are
 import numpy as np
 import pytest
 
-from sicc_gb300 import channel, codes, fec, ofdm
+from sicc_gb300 import channel, codes, engine, fec, ofdm, tune
 
 pytestmark = pytest.mark.gpu
 
@@ -98,3 +98,58 @@ def test_gather_to_unaligned_llr_rows(cuda, modulation):
     assert want.abs().sum() > 0
     for f in range(4):
         assert torch.equal(got[rows[f]:rows[f] + p.coded_bits], want[f]), f
+
+
+# --- mixed-code engine ------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("how", ["set", "autotune"])
+def test_engine_speed_survives_a_shape_given_up(cuda, how):
+    """One warp for a 2,048-bit code takes the whole batch off the register-resident rows; afterwards the
+    narrow codes, which have no other shape, are as fast as in an engine that never had it."""
+    torch = cuda
+    tune.clear()
+    cs = codes.mixed_codes()
+    narrow = [i for i, c in enumerate(cs) if c.n <= 256]
+    wide = [i for i, c in enumerate(cs) if c.n == 2048]
+    rng = np.random.default_rng(6)
+    code_of = np.sort(rng.choice(narrow, 20000)).astype(np.uint8)
+    rows = np.concatenate([channel.awgn_llrs(cs[c], int((code_of == c).sum()), 2.0, 9 + c)[2].reshape(-1)
+                           for c in sorted(set(code_of.tolist()))]).astype(np.float32)
+    ns, ks = (np.array([getattr(cs[c], a) for c in code_of], np.int64) for a in "nk")
+    off = lambda v: torch.from_numpy(np.concatenate([[0], np.cumsum(v)[:-1]])).cuda()  # noqa: E731
+    d = (torch.from_numpy(code_of).cuda(), torch.from_numpy(rows).cuda(), off(ns))
+    io, b = off(ks), len(code_of)
+
+    def make():
+        eng = engine.Engine(max_codewords=b, max_llr_floats=rows.size)
+        for c in cs:
+            eng.add_code(c, engine.iteration_cap(c.n), osd_order=engine.osd_order_for(c))
+        return eng
+
+    def decode(eng):
+        out = [torch.zeros(int(ks.sum()), dtype=torch.uint8, device="cuda")] + \
+              [torch.zeros(b, dtype=torch.uint8, device="cuda") for _ in range(3)]
+        eng.decode_device(b, *d, out[0], io, *out[1:], stream=torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        return [x.cpu().numpy() for x in out]
+
+    plain, tried = make(), make()
+    want = decode(plain)
+    if how == "set":
+        for i in wide:
+            tried.set_code_warps(i, 1)
+        decode(tried)
+        for i in wide:
+            tried.set_code_warps(i, 4)
+    else:
+        tried.autotune(b, *d, torch.zeros(int(ks.sum()), dtype=torch.uint8, device="cuda"), io, reps=1)
+    for x, y in zip(want, decode(tried)):
+        assert np.array_equal(x, y)
+    ms = {}
+    for _ in range(5):  # in turn; the least of each
+        for name, eng in (("plain", plain), ("tried", tried)):
+            decode(eng)
+            ms[name] = min(ms.get(name, 1e9), eng.last_ms()[1])
+    # off the register-resident rows the mixed kernel takes about twice as long
+    assert ms["tried"] <= 1.25 * ms["plain"], ms
+    tune.clear()
