@@ -935,7 +935,9 @@ __device__ __forceinline__ float sq_dist(float x, float c)
 
 }  // namespace
 
-template <int kBps>
+// kSharedTw: the FFT's twiddles copied to shared memory, else read from global memory (the largest
+// grids, whose pilots leave no room for them).
+template <int kBps, bool kSharedTw>
 __global__ void __launch_bounds__(kDemodThreads)
 demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, const SyncOut* __restrict__ sync,
              float* __restrict__ llr, long long llr_stride, int symbols_per_cta, const long long* __restrict__ frame_off,
@@ -947,8 +949,8 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
     float2* work = reinterpret_cast<float2*>(smem_raw);  // derotated symbol, FFT buffer
     // stage(b) = work + (1 + b) * nfft: staged raw symbols (two buffers), FFT buffer after use
     auto stage = [&](int b) { return work + static_cast<size_t>(1 + b) * v.nfft; };
-    float2* tw = work + 3 * v.nfft;                       // the FFT's twiddles in stage order
-    float2* hp = tw + fft_twiddles(v.nfft);               // [max_pilots_per_cta][active_sc]
+    float2* s_tw = work + 3 * v.nfft;                     // the FFT's twiddles in stage order
+    float2* hp = s_tw + (kSharedTw ? fft_twiddles(v.nfft) : 0);  // [max_pilots_per_cta][active_sc]
     __shared__ __align__(8) uint64_t s_bar[2];
 
     const int f = blockIdx.x;
@@ -990,7 +992,11 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
         mbar_init(&s_bar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < fft_twiddles(v.nfft); i += blockDim.x) tw[i] = __ldg(v.twiddle + i);
+    const float2* tw = v.twiddle;
+    if constexpr (kSharedTw) {
+        for (int i = threadIdx.x; i < fft_twiddles(v.nfft); i += blockDim.x) s_tw[i] = __ldg(v.twiddle + i);
+        tw = s_tw;
+    }
     constexpr int bps = kBps, abits = kBps >> 1, levels = 1 << abits;
     // the constellation's axis levels (at most 8: 64-QAM) in registers
     float lvl[levels];
@@ -1127,10 +1133,15 @@ void launch_demod(const DemodView& v, const float2* samples, long long stride, c
         if (static_cast<long long>(frames) * ((v.num_data + part - 1) / part) > device_sm_count()) break;
         spc = part;
     }
-    const size_t smem = (3 * static_cast<size_t>(v.nfft) + fft_twiddles(v.nfft) +
-                         static_cast<size_t>(v.max_pilots_per_cta) * v.active_sc) *
-                        sizeof(float2);
-    if (smem > 227 * 1024) throw InvalidArgument("nfft and active_sc exceed the demodulator's shared memory");
+    // Accepted: grids that fit the 227 KB with 3/4 nfft further points (a plain twiddle table).  Of
+    // these the largest (4,096 points with four pilots of more than 3,169 subcarriers) do not fit the
+    // stage-ordered twiddles and read them from global memory.
+    constexpr size_t most = 227 * 1024 / sizeof(float2);
+    const size_t points = 3 * static_cast<size_t>(v.nfft) + static_cast<size_t>(v.max_pilots_per_cta) * v.active_sc;
+    if (points + ((3 * static_cast<size_t>(v.nfft) / 4 + 1) & ~size_t(1)) > most)
+        throw InvalidArgument("nfft and active_sc exceed the demodulator's shared memory");
+    const bool shared_tw = points + fft_twiddles(v.nfft) <= most;
+    const size_t smem = (points + (shared_tw ? fft_twiddles(v.nfft) : 0)) * sizeof(float2);
     const dim3 grid(frames, (v.num_data + spc - 1) / spc);
     const auto go = [&](auto kernel) {
         check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(demod)");
@@ -1139,10 +1150,10 @@ void launch_demod(const DemodView& v, const float2* samples, long long stride, c
         check_cuda(cudaGetLastError(), "demod_kernel launch");
     };
     switch (v.bits_per_symbol) {
-        case 1: go(demod_kernel<1>); break;
-        case 2: go(demod_kernel<2>); break;
-        case 4: go(demod_kernel<4>); break;
-        default: go(demod_kernel<6>); break;
+        case 1: shared_tw ? go(demod_kernel<1, true>) : go(demod_kernel<1, false>); break;
+        case 2: shared_tw ? go(demod_kernel<2, true>) : go(demod_kernel<2, false>); break;
+        case 4: shared_tw ? go(demod_kernel<4, true>) : go(demod_kernel<4, false>); break;
+        default: shared_tw ? go(demod_kernel<6, true>) : go(demod_kernel<6, false>); break;
     }
 }
 

@@ -100,6 +100,51 @@ def test_gather_to_unaligned_llr_rows(cuda, modulation):
         assert torch.equal(got[rows[f]:rows[f] + p.coded_bits], want[f]), f
 
 
+def _large_grid(active, modulation):
+    """4,096 points, every second symbol a pilot: a demodulator CTA holds four pilots of `active` subcarriers."""
+    cfg = ofdm.PhyConfig(nfft=4096, cp=288, num_symbols=13, active_sc=active, pre_half_len=200, modulation=modulation,
+                         pilot_period=2)
+    return ofdm.reference_tables(cfg)
+
+
+@pytest.mark.parametrize("frames", [1, 60])
+@pytest.mark.parametrize("active,modulation", [(3168, "qpsk"), (3172, "qpsk"), (3276, "bpsk"), (3276, "16qam"),
+                                               (3276, "64qam"), (3424, "qpsk")])
+def test_demodulator_near_its_shared_memory_limit(cuda, oracle, active, modulation, frames):
+    from sicc_gb300.pipeline import SYNC_RECORD, RxPipeline
+    from test_gpu_ofdm import _llr_close
+    torch = cuda
+    t, code = _large_grid(active, modulation), codes.short_code()
+    b = ofdm.FrameGenerator(t, code, seed=19).batch(2, snr_db=25.0, cfo_subcarriers=0.05, max_offset=60, rayleigh_taps=0)
+    iq = np.tile(b.iq, ((frames + 1) // 2, 1))[:frames]
+    p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, float(b.noise_var[0]), max_batch_frames=frames)
+    llr = torch.zeros((frames, p.coded_bits), dtype=torch.float32, device="cuda")
+    rec = torch.zeros(frames * SYNC_RECORD.itemsize, dtype=torch.uint8, device="cuda")
+    p.demod_batch(torch.from_numpy(iq).cuda(), iq.shape[1], iq.shape[1], frames, llr, rec, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    sync, got, ph = rec.cpu().numpy().view(SYNC_RECORD), llr.cpu().numpy(), oracle.phy(t)
+    for f in range(min(frames, 2)):
+        r = oracle.sync_earliest(ph, iq[f])
+        assert sync[f]["found"] == r[0] == 1 and sync[f]["start"] == r[1]
+        ref = oracle.demod_frame(ph, iq[f][r[1]:r[1] + t.frame_len], float(sync[f]["cfo_hz"]),
+                                 float(np.float32(b.noise_var[0])))
+        _llr_close(got[f], ref[: p.coded_bits])
+    for f in range(2, frames):
+        assert np.array_equal(got[f], got[f % 2]), f
+
+
+def test_demodulator_past_its_shared_memory_limit_is_refused(cuda):
+    from sicc_gb300 import _lib
+    from sicc_gb300.pipeline import RxPipeline
+    torch = cuda
+    t, code = _large_grid(3426, "qpsk"), codes.short_code()
+    p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, 0.1, max_batch_frames=1)
+    iq = torch.zeros((1, t.frame_len), dtype=torch.complex64, device="cuda")
+    llr = torch.zeros((1, p.coded_bits), dtype=torch.float32, device="cuda")
+    with pytest.raises(_lib.SiccError, match="shared memory"):
+        p.demod_batch(iq, t.frame_len, t.frame_len, 1, llr, None, torch.cuda.current_stream())
+
+
 # --- mixed-code engine ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("how", ["set", "autotune"])
