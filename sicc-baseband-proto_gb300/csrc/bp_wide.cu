@@ -321,35 +321,42 @@ struct PlainApp {
 template <int D>
 constexpr int flood_threads() { return D <= 18 ? 1024 : 512; }
 
+// What the flooding kernel keeps in shared memory: nothing, the hard decisions, the messages too.
+enum class Place { kSlice, kHardSmem, kAllSmem };
+
 // One float per edge, input and message of the edge in turn: the check phase replaces a row's
 // inputs by its messages, the variable phase a column's messages by its next inputs.  Edge j of
 // row r sits at cv.wide_stride * j + (r with its low 5 bits XORed by the next 5): rows are read
 // conflict-free and the strided rows of a quasi-cyclic column spread over the banks.  The array
-// lives in shared memory when it fits (kSmem: the N16200 codes), else in the CTA's slice.  The
-// syndrome reads the hard decisions packed 32 to a word; without best-syndrome tracking it stops
-// at the first unsatisfied rows.  kDamp: the inputs are kept beside, in the slice.
+// lives in shared memory when it fits (the N16200 codes), else in the CTA's slice.  The syndrome reads
+// the hard decisions packed 32 to a word, in shared memory too (in the slice for codes of more than
+// 1.8 million bits); without best-syndrome tracking it stops at the first unsatisfied rows.  kDamp:
+// the inputs are kept beside, in the slice.
 //
 // Measured on GB300, 333 codewords of (16200,13320) at 4 dB: 2.8 ms before (per edge of each of
 // two column passes an edge, row and row-pointer lookup and a message rebuild, all from L2),
 // 0.38 ms now.
-template <int D, bool kDamp, bool kSmem>
+template <int D, bool kDamp, Place kPlace>
 __global__ void __launch_bounds__(flood_threads<D>(), 1)
 bp_flooding_wide_kernel(FloodView cv, BpParams p, BpIO io, float* scratch, long long slice, int track_best)
 {
     constexpr int kThreads = flood_threads<D>();
+    constexpr bool kSmem = kPlace == Place::kAllSmem;
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ int s_red[kThreads / 32];
     __shared__ int s_next, s_slot;
     const int tid = threadIdx.x;
     const int n = cv.n, m = cv.m, n_pad = (n + 3) & ~3, stride = cv.wide_stride;
     const int words = (n + 31) / 32 + 1;  // the last one stays 0: missing edges of short rows read it
-    uint32_t* hard = reinterpret_cast<uint32_t*>(s_raw);
     float* g = scratch + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(slice);
     float* app = g;
     float* best = app + n_pad;  // only when track_best
     float* rest = best + (track_best ? n_pad : 0);
     float* msg = kSmem ? reinterpret_cast<float*>(s_raw + ((static_cast<size_t>(words) * 4 + 15) & ~size_t(15))) : rest;
     float* old = rest + (kSmem ? 0 : static_cast<size_t>(cv.maxdeg) * stride);  // only when kDamp
+    uint32_t* hard = reinterpret_cast<uint32_t*>(s_raw);
+    if constexpr (kPlace == Place::kSlice)
+        hard = reinterpret_cast<uint32_t*>(old + (kDamp ? static_cast<size_t>(cv.maxdeg) * stride : 0));
     const float keep = __fsub_rn(1.0f, p.damping);
     const auto slot = [](int r) { return r ^ ((r >> 5) & 31); };
 
@@ -489,17 +496,19 @@ int wide_grid(int count, int per_sm, size_t slice_bytes)
 size_t flood_hard_bytes(const FloodView& cv) { return (static_cast<size_t>((cv.n + 31) / 32 + 1) * 4 + 15) & ~size_t(15); }
 size_t flood_msg_bytes(const FloodView& cv) { return static_cast<size_t>(cv.maxdeg) * cv.wide_stride * sizeof(float); }
 
-template <int D, bool kDamp, bool kSmem>
+template <int D, bool kDamp, Place kPlace>
 void launch_flooding_wide_t(const FloodView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
 {
-    const auto kernel = bp_flooding_wide_kernel<D, kDamp, kSmem>;
-    const size_t smem = flood_hard_bytes(cv) + (kSmem ? flood_msg_bytes(cv) : 0);
+    constexpr bool kSmem = kPlace == Place::kAllSmem;
+    const auto kernel = bp_flooding_wide_kernel<D, kDamp, kPlace>;
+    const size_t smem = (kPlace == Place::kSlice ? 0 : flood_hard_bytes(cv)) + (kSmem ? flood_msg_bytes(cv) : 0);
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp wide)");
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, flood_threads<D>(), smem) != cudaSuccess || per_sm <= 0)
         per_sm = 1;
     const long long n_pad = (cv.n + 3) & ~3, edges = static_cast<long long>(cv.maxdeg) * cv.wide_stride;
-    long long slice = n_pad + (track_best ? n_pad : 0) + (kSmem ? 0 : edges) + (kDamp ? edges : 0);
+    long long slice = n_pad + (track_best ? n_pad : 0) + (kSmem ? 0 : edges) + (kDamp ? edges : 0) +
+                      (kPlace == Place::kSlice ? static_cast<long long>(flood_hard_bytes(cv) / sizeof(float)) : 0);
     slice = (slice + 31) & ~31LL;
     const size_t slice_bytes = static_cast<size_t>(slice) * sizeof(float);
     const int ctas = wide_grid(io.count, per_sm, slice_bytes);
@@ -515,18 +524,20 @@ void launch_flooding_wide_t(const FloodView& cv, const BpParams& p, const BpIO& 
     check_cuda(ferr, "cudaFreeAsync(bp wide)");
 }
 
-template <int D>
+template <int D, bool kDamp>
 void launch_flooding_wide_d(const FloodView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
 {
-    // 1 KB of the 227 KB stays for the kernel's static arrays
-    const bool fits = flood_hard_bytes(cv) + flood_msg_bytes(cv) <= 226 * 1024;
-    if (p.damping == 0.0f) {
-        if (fits) launch_flooding_wide_t<D, false, true>(cv, p, io, track_best, st);
-        else launch_flooding_wide_t<D, false, false>(cv, p, io, track_best, st);
-    } else {
-        if (fits) launch_flooding_wide_t<D, true, true>(cv, p, io, track_best, st);
-        else launch_flooding_wide_t<D, true, false>(cv, p, io, track_best, st);
-    }
+    constexpr size_t most = 226 * 1024;  // 1 KB of the 227 KB stays for the kernel's static arrays
+    if (flood_hard_bytes(cv) + flood_msg_bytes(cv) <= most) launch_flooding_wide_t<D, kDamp, Place::kAllSmem>(cv, p, io, track_best, st);
+    else if (flood_hard_bytes(cv) <= most) launch_flooding_wide_t<D, kDamp, Place::kHardSmem>(cv, p, io, track_best, st);
+    else launch_flooding_wide_t<27, kDamp, Place::kSlice>(cv, p, io, track_best, st);  // one instance for any degree
+}
+
+template <int D>
+void launch_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO& io, bool track_best, cudaStream_t st)
+{
+    if (p.damping == 0.0f) launch_flooding_wide_d<D, false>(cv, p, io, track_best, st);
+    else launch_flooding_wide_d<D, true>(cv, p, io, track_best, st);
 }
 
 template <int D, int kFar>
@@ -614,10 +625,10 @@ void launch_bp_flooding_wide(const FloodView& cv, const BpParams& p, const BpIO&
     if (cv.maxdeg > 27) throw InvalidArgument("flooding schedule supports row degree <= 27");
     const bool track_best = p.route_failures_to_osd && io.osd_llr != nullptr;
     if (!io.work_zeroed) check_cuda(cudaMemsetAsync(io.work_counter, 0, sizeof(int), st), "reset work counter");
-    if (cv.maxdeg <= 6) launch_flooding_wide_d<6>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 10) launch_flooding_wide_d<10>(cv, p, io, track_best, st);
-    else if (cv.maxdeg <= 18) launch_flooding_wide_d<18>(cv, p, io, track_best, st);
-    else launch_flooding_wide_d<27>(cv, p, io, track_best, st);
+    if (cv.maxdeg <= 6) launch_flooding_wide<6>(cv, p, io, track_best, st);
+    else if (cv.maxdeg <= 10) launch_flooding_wide<10>(cv, p, io, track_best, st);
+    else if (cv.maxdeg <= 18) launch_flooding_wide<18>(cv, p, io, track_best, st);
+    else launch_flooding_wide<27>(cv, p, io, track_best, st);
 }
 
 }  // namespace sicc

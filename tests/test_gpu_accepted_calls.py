@@ -75,6 +75,30 @@ def test_unaligned_soft_values_stream_decoder(cuda, schedule):
         assert np.array_equal(a, b)
 
 
+# --- codes of millions of bits ------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("damping", [0.0, 0.2])
+@pytest.mark.parametrize("n", [1851360, 1851362, 2000000])  # the packed hard decisions in and past shared memory
+def test_flooding_of_a_huge_code(cuda, oracle, n, damping):
+    m = n // 2
+    k, r = n - m, np.arange(m, dtype=np.int64)
+    cols = np.stack([(3 * r) % k, (3 * r + 1 + r % 1001) % k, k + np.maximum(r - 1, 0), k + r], axis=1)
+    cols.sort(axis=1)
+    keep = np.ones((m, 4), bool)
+    keep[0, 3] = False  # the first row has no previous parity
+    row_ptr = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int32)
+    col_ind = cols[keep].astype(np.int32)
+    llr = (2.0 / 0.4 * (1.0 + np.sqrt(0.4) * np.random.default_rng(n).standard_normal((2, n)))).astype(np.float32)
+    dec = fec.CsrBpDecoder(n, m, row_ptr, col_ind, max_batch=2, max_iter=3, normalization=0.8, damping=damping,
+                           schedule=fec.FLOODING)
+    got = _decode(cuda, dec, cuda.from_numpy(llr).cuda(), n)
+    oc = oracle.code(n, m, row_ptr, col_ind)
+    for i, x in enumerate(llr):
+        o = oc.flooding(x, 3, 0.8, 0.0, damping)
+        assert got[1][i] == o[0] and got[3][i] == o[4]
+        assert np.array_equal(got[0][i], o[1]) and np.array_equal(got[2][i], o[2])
+
+
 # --- OFDM receiver --------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("modulation", ["bpsk", "qpsk", "16qam", "64qam"])
