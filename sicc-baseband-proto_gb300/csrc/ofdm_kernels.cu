@@ -119,9 +119,10 @@ __device__ __forceinline__ int fine_half(int pre) { return (pre >> 6) << 5; }
 // with one read of the preamble for the four and one energy sum: the samples common to the four,
 // then each position's own ones (sums of non-negative terms only).  After the first half of the
 // preamble |c| <= |c1| + sqrt(e2 E2) (e2, E2: energies of the other half of the samples and of the
-// preamble), widened by 1e-5 of sqrt(e E) for the rounding of the sums (at most 40 of 6e-8 each for
-// the lengths that fit); when that puts all four below the threshold they are reported as -1 and the
-// other half is not correlated.  Away from the preamble c1 is small and the bound about 1/4: most
+// preamble), widened for the rounding of the sums: a lane adds pre / 32 times in each half, so c1, c,
+// e2 and E2 together are off by less than 0.17 pre + 33 rounding units of sqrt(e E) (2^-24 each;
+// pre / 4 + 64 are taken).  When that puts all four below the threshold they are reported as -1 and the
+// other half is not correlated.  Preambles under 64 samples have no first half and no early stop.  Away from the preamble c1 is small and the bound about 1/4: most
 // groups stop there (256 frames at threshold 0.45, search
 // and demodulation: 120 us without the early stop and the shared energy, 106 with them).
 __device__ __forceinline__ void fine_metric4(const float2* win, int at, const float2* __restrict__ preamble, int pre,
@@ -162,12 +163,12 @@ __device__ __forceinline__ void fine_metric4(const float2* win, int at, const fl
     float over = e2;  // at least each position's energy against the preamble's other half
 #pragma unroll
     for (int j = 0; j < 3; ++j) over = energy(pre + j, over);
-    const float rest = sqrtf(over * tail_energy);
-    bool below = true;
+    const float rest = sqrtf(over * tail_energy), widen = (0.25f * static_cast<float>(pre) + 64.0f) * 5.9604645e-08f;
+    bool below = half > 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const float r = warp_sum(cr[k]), j = warp_sum(ci[k]), full = eng[k] * pre_energy;
-        const float most = sqrtf(r * r + j * j) + rest + 1e-5f * sqrtf(full);
+        const float most = sqrtf(r * r + j * j) + rest + widen * sqrtf(full);
         below = below && most * most < threshold * fmaxf(full, 1e-18f);
     }
     if (__all_sync(0xffffffffu, below)) {

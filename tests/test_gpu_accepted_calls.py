@@ -169,6 +169,39 @@ def test_demodulator_past_its_shared_memory_limit_is_refused(cuda):
         p.demod_batch(iq, t.frame_len, t.frame_len, 1, llr, None, torch.cuda.current_stream())
 
 
+@pytest.mark.parametrize("value", [0.8349244594573975 + 0.571209192276001j, 0.6395646333694458 + 0.7616397142410278j,
+                                   0.5345859527587891 + 0.8649413585662842j])
+@pytest.mark.parametrize("half", [24, 3968, 7936])  # no first half to stop after; long sums
+def test_search_at_a_threshold_equal_to_the_metric(cuda, half, value):
+    """A frame whose fine metric is exactly the threshold is found.  The preamble repeats one value whose
+    square rounds the same way in every step of a sum, so long sums are off by more than 1e-5; each half
+    begins and ends with three zeros, so the neighbouring positions have the same energy."""
+    import dataclasses
+    from sicc_gb300.pipeline import SYNC_RECORD, RxPipeline
+    torch, code, at = cuda, codes.short_code(), 303
+
+    def search(threshold):
+        cfg = ofdm.PhyConfig(nfft=64, cp=16, num_symbols=6, active_sc=32, pre_half_len=half, modulation="qpsk",
+                             pilot_period=3, sync_threshold=float(threshold))
+        pre = np.full((2, half), value, np.complex64)
+        pre[:, :3] = pre[:, -3:] = 0
+        t = dataclasses.replace(ofdm.reference_tables(cfg), preamble=pre.reshape(-1))
+        iq = np.zeros((1, at + t.frame_len + 50), np.complex64)
+        iq[0, at:at + 2 * half] = t.preamble
+        p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, 0.1, max_batch_frames=1)
+        llr = torch.zeros((1, p.coded_bits), dtype=torch.float32, device="cuda")
+        rec = torch.zeros(SYNC_RECORD.itemsize, dtype=torch.uint8, device="cuda")
+        p.demod_batch(torch.from_numpy(iq).cuda(), iq.shape[1], iq.shape[1], 1, llr, rec, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        return rec.cpu().numpy().view(SYNC_RECORD)[0]
+
+    first = search(1.0 - 0.9 / half)
+    assert first["found"] == 1 and first["start"] == at
+    again = search(min(first["coarse"], first["fine"], 1.0))
+    assert again["found"] == 1 and again["start"] == at
+    assert again["fine"] == first["fine"]
+
+
 # --- mixed-code engine ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("how", ["set", "autotune"])
