@@ -26,8 +26,9 @@
  * The autotuner times candidate shapes on the caller's own batch (CUDA events
  * on the decoder's stream, median of `reps` decodes after one warm-up),
  * applies the fastest to the handle and records it in a process-wide cache
- * keyed by the code (parity-check matrix and schedule), its decode settings
- * and the device (name and SM count).  Decoders and engine codes created
+ * keyed by the code (parity-check matrix and schedule), its decode settings,
+ * the device (name and SM count) and the generation of the library's kernels
+ * (shapes saved by a library with other kernels are not applied).  Decoders and engine codes created
  * later with the same key start from the cached shape; sicc_tune_save /
  * sicc_tune_load carry the cache across processes as a text file.
  * Status codes and the last-error string are those of sicc_fec.h.

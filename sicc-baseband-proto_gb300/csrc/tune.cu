@@ -1,7 +1,8 @@
 // Process-wide cache of tuned launch shapes (include/sicc_tune.h).
 //
 // Keys name the code (a fingerprint of its parity-check matrix, schedule and
-// decode settings) and the device (name and SM count); values are the shape
+// decode settings), the device (name and SM count) and the generation of the
+// kernels that were timed; values are the shape
 // fields of the owner (a stream / CSR decoder, or an engine code).  The cache
 // is a plain text file on disk: one "key v1 v2 ..." line per entry.
 #include "../../include/sicc_tune.h"
@@ -21,6 +22,12 @@ namespace {
 std::mutex g_tune_mu;
 std::map<std::string, std::vector<int>> g_tune;
 
+// Counted up when kernels change what a shape means or which one is fastest: a shape saved for others
+// stays in the table and the file but is not applied.  1 (keys without a number): row messages in
+// compressed form.  2: messages in registers, where fixed lanes per codeword or other warps than a
+// code's default take it off them.
+constexpr int kKernelGeneration = 2;
+
 }  // namespace
 
 std::string tune_key(const char* kind, uint64_t fingerprint)
@@ -33,7 +40,8 @@ std::string tune_key(const char* kind, uint64_t fingerprint)
     std::replace(name.begin(), name.end(), ' ', '_');
     char buf[64];
     std::snprintf(buf, sizeof buf, "%016llx", static_cast<unsigned long long>(fingerprint));
-    return std::string(kind) + ":" + buf + "@" + name + "/" + std::to_string(prop.multiProcessorCount);
+    return std::string(kind) + ":" + buf + "@" + name + "/" + std::to_string(prop.multiProcessorCount) + "/k" +
+           std::to_string(kKernelGeneration);
 }
 
 bool tune_cache_get(const std::string& key, std::vector<int>& values)

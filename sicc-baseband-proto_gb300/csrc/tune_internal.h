@@ -31,7 +31,7 @@ struct Fingerprint {
     }
 };
 
-// "<kind>:<fingerprint hex>@<device name>/<SMs>" for the current device.
+// "<kind>:<fingerprint hex>@<device name>/<SMs>/k<kernel generation>" for the current device.
 std::string tune_key(const char* kind, uint64_t fingerprint);
 bool tune_cache_get(const std::string& key, std::vector<int>& values);
 void tune_cache_put(const std::string& key, const std::vector<int>& values);

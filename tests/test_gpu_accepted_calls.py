@@ -255,3 +255,40 @@ def test_engine_speed_survives_a_shape_given_up(cuda, how):
     # off the register-resident rows the mixed kernel takes about twice as long
     assert ms["tried"] <= 1.25 * ms["plain"], ms
     tune.clear()
+
+
+# --- saved shapes -----------------------------------------------------------------------------------------
+
+def test_shapes_saved_for_other_kernels_are_not_applied(cuda, tmp_path):
+    """Keys of the first kernels carry no generation; the same shapes under today's keys are applied."""
+    import re
+    torch, code, wide = cuda, codes.short_code(), codes.qc_code(8, 16, 128, seed=3)
+    tune.clear()
+    d_llr = torch.from_numpy(channel.awgn_llrs(wide, 64, 2.0, 1)[2].astype(np.float32)).cuda()
+
+    def decoder():
+        return fec.CsrBpDecoder.for_code(code, max_batch=64, max_iter=5)
+
+    def eng():
+        e = engine.Engine(max_codewords=64, max_llr_floats=64 * wide.n)
+        e.add_code(wide, 5)
+        return e
+
+    decoder().autotune(torch.from_numpy(channel.awgn_llrs(code, 64, 2.0, 1)[2].astype(np.float32)).cuda(), reps=1)
+    off = torch.arange(64, device="cuda")
+    eng().autotune(64, torch.zeros(64, dtype=torch.uint8, device="cuda"), d_llr, off * wide.n,
+                   torch.zeros(64 * wide.k, dtype=torch.uint8, device="cuda"), off * wide.k, reps=1)
+    path = tmp_path / "shapes.txt"
+    tune.save(str(path))
+    keys = {line.split()[0].split(":")[0]: line.split()[0] for line in path.read_text().splitlines()}
+    shapes = {"fec": "8 16 0 0 0", "engine-code": "1"}
+    for strip in (True, False):
+        tune.clear()
+        path.write_text("".join("%s %s\n" % (re.sub(r"/k\d+$", "", k) if strip else k, shapes[kind])
+                                for kind, k in keys.items()))
+        tune.load(str(path))
+        assert tune.entries() == 2
+        shape = decoder().shape()
+        assert (shape["lanes_per_codeword"], shape["slots_per_cta"]) == ((0, 0) if strip else (8, 16))
+        assert eng().code_warps(0) == (4 if strip else 1)
+    tune.clear()
