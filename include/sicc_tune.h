@@ -13,8 +13,8 @@
  *     slots_per_cta       codewords resident per CTA of the persistent kernel;
  *     ctas                persistent grid size;
  *   OSD (warp-per-codeword kernel):
- *     osd_share_rounds    0..64, kept for saved shapes: the kernel exchanges its
- *                         best metric whenever it changes;
+ *     osd_share_rounds    candidates each warp tests between exchanges of its
+ *                         best metric, in rounds of 32 (one per lane), 0..64;
  *     osd_ctas            grid size;
  *   mixed-code engine (include/sicc_engine.h):
  *     warps per codeword of each registered code (1, 2 or 4: the check-node

@@ -22,7 +22,7 @@ inline int pad_slot_stride(int floats, int group)
 struct BpLaunch {
     int slots_per_cta = 0;    // codewords resident per CTA (multiple of 32/group)
     int ctas = 0;             // grid size (persistent CTAs)
-    int osd_share_rounds = 0; // kept for saved shapes: the warp OSD exchanges its best metric whenever it changes
+    int osd_share_rounds = 0; // warp OSD: candidate passes between best-metric exchanges (0 = 1)
     int osd_ctas = 0;         // warp OSD grid size (0 = occupancy x SMs)
 };
 

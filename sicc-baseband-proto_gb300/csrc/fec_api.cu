@@ -193,6 +193,7 @@ void run_bp_osd(const DeviceCode& code, const BpParams& bp, const BpLaunch& shap
         oio.out_info = d_bits;
         oio.info_stride = out_stride;
         oio.used_osd = d_used_osd;
+        oio.share_rounds = shape.osd_share_rounds;
         oio.work = s.counters.p + 2;
         oio.work_zeroed = true;
         launch_osd(code.osd_view(), oio, count, st, 0, shape.osd_ctas);
@@ -843,6 +844,7 @@ int decode_with_caller_scratch(unsigned long long handle, const float* d_llr, in
         oio.out_info = d_info;
         oio.info_stride = d->k;
         oio.used_osd = d_used_osd;
+        oio.share_rounds = d->shape.osd_share_rounds;
         oio.work = counters + 2;  // inside the counters' 256 bytes
         oio.work_zeroed = true;
         launch_osd(d->code->osd_view(), oio, count, st, 0, d->shape.osd_ctas);
@@ -1026,6 +1028,7 @@ int cuda_osd_decode_osd_batch(unsigned long long handle, const float* llrs, int 
             io.out_info = d->info.p;
             io.info_stride = d->k;
             io.out_metric = d->dist.p;
+            io.share_rounds = d->shape.osd_share_rounds;
             launch_osd(d->code->osd_view(), io, cnt, d->stream, 0, d->shape.osd_ctas);
             check_cuda(cudaMemcpyAsync(out_info_bits + static_cast<size_t>(off) * d->k, d->info.p,
                                        static_cast<size_t>(cnt) * d->k, cudaMemcpyDeviceToHost, d->stream),
@@ -1311,6 +1314,12 @@ int sicc_fec_autotune(unsigned long long handle, const float* device_llrs, int c
             }
         }
         if (with_osd && d->code->has_osd()) {
+            const sicc_fec_shape_t bp_best = best;
+            for (int share : {2, 4, 8}) {
+                sicc_fec_shape_t sh = bp_best;
+                sh.osd_share_rounds = share;
+                consider(sh);
+            }
             const sicc_fec_shape_t osd_best = best;
             for (int per_sm : {1, 2}) {
                 sicc_fec_shape_t sh = osd_best;
@@ -1420,6 +1429,7 @@ int sicc_osd_decode_device(unsigned long long handle, const float* device_llrs, 
         io.info_stride = d->k;
         io.out_code = device_code_bits;
         io.out_metric = device_distances;
+        io.share_rounds = d->shape.osd_share_rounds;
         launch_osd(d->code->osd_view(), io, codewords, static_cast<cudaStream_t>(cuda_stream), 0,
                    d->shape.osd_ctas);
         return CUDA_OSD_STATUS_OK;

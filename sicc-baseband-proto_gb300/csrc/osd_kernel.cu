@@ -87,7 +87,11 @@ __device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v,
 
 }  // namespace
 
-template <int NW, int KR>
+// kRounds: the best metric is exchanged at a given interval (a launch shape's choice), an instance of its
+// own: a test of the interval in the default loop cost 1-4% of the whole (128,64) decode.  16,384 frames:
+// order 2 at 2 dB 221 us with an exchange after each pass, 228 every 8, 233 every 64; order 3 at 1 dB
+// 491, 536, 592.
+template <int NW, int KR, bool kRounds>
 __global__ void __launch_bounds__(kOsdWarps * 32)
 osd_kernel(OsdView ov0, OsdIO io)
 {
@@ -517,8 +521,10 @@ osd_kernel(OsdView ov0, OsdIO io)
             __syncwarp();
             return __shfl_sync(0xffffffffu, incl, 31);
         };
-        // 32 tests per pass (one site for the bound and the sum keeps the code small): first the base
-        // test alone, then the tests from 1 on, and for complete order 2 the single flips, then the pairs.
+        // 32 tests per pass (one site for the bound, the sum and the exchange keeps the code small): first
+        // the base test alone, then the tests from 1 on, and for complete order 2 the single flips, then
+        // the pairs.  The best metric is exchanged after every pass that summed a test, or (kRounds) after
+        // every io.share_rounds passes and at the end of a stage.
         int stage = 0, i0 = 0, end = 1, row = 0;
 #pragma unroll 1
         while (true) {
@@ -556,8 +562,9 @@ osd_kernel(OsdView ov0, OsdIO io)
                 go = !(bound(f0, f1, f2) > thr * kSlack);
             }
             i0 += 32;
-            if (!__any_sync(0xffffffffu, go)) continue;
+            if (!__any_sync(0xffffffffu, go) && (!kRounds || i0 < end)) continue;
             if (go) evaluate(q, f0, f1, f2);
+            if (kRounds && i0 < end && (i0 >> 5) % io.share_rounds != 0) continue;
             share_best();
         }
         // ---- 7. winner -> original positions ----
@@ -593,19 +600,19 @@ osd_kernel(OsdView ov0, OsdIO io)
     }
 }
 
-template <int NW, int KR>
+template <int NW, int KR, bool kRounds>
 static void launch_osd_t(const OsdView& ov, const OsdIO& io, int max_items, cudaStream_t st, int ctas)
 {
     if (ctas <= 0) {
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, osd_kernel<NW, KR>, kOsdWarps * 32, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, osd_kernel<NW, KR, kRounds>, kOsdWarps * 32, 0) !=
                 cudaSuccess ||
             per_sm <= 0)
             per_sm = 1;
         ctas = per_sm * device_sm_count();
         ctas = std::max(1, std::min(ctas, (max_items + kOsdWarps - 1) / kOsdWarps));
     }
-    osd_kernel<NW, KR><<<ctas, kOsdWarps * 32, 0, st>>>(ov, io);
+    osd_kernel<NW, KR, kRounds><<<ctas, kOsdWarps * 32, 0, st>>>(ov, io);
     check_cuda(cudaGetLastError(), "osd_kernel launch");
 }
 
@@ -621,7 +628,11 @@ void launch_osd(const OsdView& ov, const OsdIO& io, int max_items, cudaStream_t 
     const int KR = kr <= 1 ? 1 : (kr <= 2 ? 2 : 4);
     if (nw > 4 || kr > 4) throw InvalidArgument("OSD kernel supports n <= 256 and k <= 128");
 #define SICC_OSD_CASE(A, B) \
-    if (NW == A && KR == B) { launch_osd_t<A, B>(ov, io, max_items, st, ctas); return; }
+    if (NW == A && KR == B) { \
+        if (io.share_rounds > 1) launch_osd_t<A, B, true>(ov, io, max_items, st, ctas); \
+        else launch_osd_t<A, B, false>(ov, io, max_items, st, ctas); \
+        return; \
+    }
     SICC_OSD_CASE(1, 1) SICC_OSD_CASE(1, 2) SICC_OSD_CASE(2, 1) SICC_OSD_CASE(2, 2)
     SICC_OSD_CASE(2, 4) SICC_OSD_CASE(4, 2) SICC_OSD_CASE(4, 4) SICC_OSD_CASE(4, 1) SICC_OSD_CASE(1, 4)
 #undef SICC_OSD_CASE

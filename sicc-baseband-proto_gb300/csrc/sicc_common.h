@@ -157,6 +157,9 @@ struct OsdIO {
     const long long* llr_off;
     const long long* info_off;
     const long long* row_off;
+    // warp OSD: passes of 32 candidates (one per lane) between exchanges of the warp's best metric,
+    // which tightens every lane's pruning bound (0, 1: every pass); the winner does not depend on it
+    int share_rounds;
     // Work counters (device ints the launcher zeroes on the stream unless work_zeroed): each warp (warp kernel) or
     // CTA (large-code kernel, one counter per class) takes its next item from them, so a few
     // expensive codewords do not hold up one warp's share.  Null: items by static striding.

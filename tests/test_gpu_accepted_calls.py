@@ -292,3 +292,34 @@ def test_shapes_saved_for_other_kernels_are_not_applied(cuda, tmp_path):
         assert (shape["lanes_per_codeword"], shape["slots_per_cta"]) == ((0, 0) if strip else (8, 16))
         assert eng().code_warps(0) == (4 if strip else 1)
     tune.clear()
+
+
+# --- launch shapes ----------------------------------------------------------------------------------------
+
+def test_osd_exchange_interval_takes_effect(cuda):
+    """The warp OSD's candidate rounds between exchanges of the best metric: the same results at any interval, more
+    sums (so more time, about 1.15 of the whole decode) at a long one, and an axis of the tuner's search."""
+    torch, code = cuda, codes.short_code()
+    llr = torch.from_numpy(channel.awgn_llrs(code, 8192, 1.0, 5)[2].astype(np.float32)).cuda()
+    dec = fec.StreamBpOsdDecoder(code, max_batch=8192, max_iter=20, osd_order=3)
+    out = [torch.zeros((8192, code.k), dtype=torch.uint8, device="cuda")] + \
+          [torch.zeros(8192, dtype=torch.uint8, device="cuda") for _ in range(3)]
+    ms, results = {}, {}
+    for _ in range(6):
+        for share in (0, 3, 64):
+            dec.set_shape(osd_share_rounds=share)
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            dec.decode_device_batch(llr, *out, stream=torch.cuda.current_stream())
+            ev[1].record()
+            torch.cuda.synchronize()
+            ms[share] = min(ms.get(share, 1e9), ev[0].elapsed_time(ev[1]))
+            results[share] = [x.cpu().numpy() for x in out]
+    for share in (3, 64):
+        for a, b in zip(results[0], results[share]):
+            assert np.array_equal(a, b), share
+    assert ms[64] > 1.05 * ms[0], ms
+    tune.clear()
+    res = dec.autotune(llr, reps=1)
+    assert len({shape["osd_share_rounds"] for shape, _ in res.trials}) > 2
+    tune.clear()
