@@ -10,7 +10,8 @@
  *     lanes_per_codeword  lanes of a warp that update one codeword's rows of a
  *                         check-node layer together (a power of two <= 32;
  *                         each lane owns ceil(layer width / lanes) rows);
- *     slots_per_cta       codewords resident per CTA of the persistent kernel;
+ *     slots_per_cta       codewords resident per CTA of the persistent kernel
+ *                         (more than a code's kernel holds run as its most);
  *     ctas                persistent grid size;
  *   OSD (warp-per-codeword kernel):
  *     osd_share_rounds    candidates each warp tests between exchanges of its

@@ -39,6 +39,7 @@ void launch_bp_flooding(const FloodView& cv, const BpParams& p, const BpIO& io, 
 void reg_plan(LayeredView& cv, int widest, int narrowest, int group);
 void launch_bp_layered_reg(const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape,
                            bool track_best, cudaStream_t st);
+int layered_reg_default_slots(const LayeredView& cv, bool track_best);  // codewords per CTA, the most it runs
 void launch_bp_flooding_reg(const LayeredView& cv, const BpParams& p, const BpIO& io, cudaStream_t st);
 size_t layered_smem_bytes(const LayeredView& cv, int slots, bool track_best, int* slot_floats_out);
 int layered_default_slots(const LayeredView& cv, bool track_best);

@@ -391,18 +391,28 @@ inline size_t reg_smem(const LayeredView& cv, int slots, int arrays, int* slot_f
     return static_cast<size_t>(slots) * arrays * *slot_floats * sizeof(float);
 }
 
+// Codewords per CTA: `wanted` (0: as many as run) within the shape's threads, three CTAs per SM, and the
+// posteriors (the first of the arrays) below 64 KB: the large shapes hold their offsets in 16 bits
+// (reg_plan has checked that one warp's codewords do).
+template <int D, int NL>
+int reg_slots(const LayeredView& cv, int wanted, int arrays, int* slot_floats, size_t* smem)
+{
+    const int step = std::max(1, 32 / cv.reg_group), most = reg_threads<D, NL>() / cv.reg_group;
+    int slots = wanted > 0 ? std::min(wanted, most) : most;
+    slots = std::max(step, slots - slots % step);
+    *smem = reg_smem(cv, slots, arrays, slot_floats);
+    while (slots > step && (*smem > 72 * 1024 || *smem / arrays > 65536)) *smem = reg_smem(cv, slots -= step, arrays, slot_floats);
+    return slots;
+}
+
 template <int D, int NL, class Kernel>
 void launch_reg(Kernel kernel, const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape,
                 int arrays, bool track_best, cudaStream_t st)
 {
-    const int G = cv.reg_group, step = std::max(1, 32 / G), most = reg_threads<D, NL>() / G;
-    int slots = shape.slots_per_cta > 0 ? std::min(shape.slots_per_cta, most) : most;
-    slots = std::max(step, slots - slots % step);
+    const int G = cv.reg_group;
     int slot_floats = 0;
-    size_t smem = reg_smem(cv, slots, arrays, &slot_floats);
-    // three CTAs per SM, and the posteriors (the first of the arrays) below 64 KB: the large shapes
-    // hold their offsets in 16 bits (reg_plan has checked that one warp's codewords do)
-    while (slots > step && (smem > 72 * 1024 || smem / arrays > 65536)) smem = reg_smem(cv, slots -= step, arrays, &slot_floats);
+    size_t smem = 0;
+    const int slots = reg_slots<D, NL>(cv, shape.slots_per_cta, arrays, &slot_floats, &smem);
     check_cuda(grant_dynamic_smem(reinterpret_cast<const void*>(kernel), smem), "cudaFuncSetAttribute(bp reg)");
     int ctas = shape.ctas;
     if (ctas <= 0) {

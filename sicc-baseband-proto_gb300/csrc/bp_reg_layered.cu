@@ -90,7 +90,7 @@ bp_layered_reg_kernel(LayeredView cv, BpParams p, BpIO io, int slots_per_cta, in
     }
 }
 
-template <int D, int NL, bool kPlain = true>
+template <int D, int NL, bool kPlain>
 void launch_shape(const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape, bool track_best,
                   cudaStream_t st)
 {
@@ -108,27 +108,45 @@ void launch_shape(const LayeredView& cv, const BpParams& p, const BpIO& io, cons
     launch_reg<D, NL>(bp_layered_reg_kernel<D, NL, 1, kPlain>, cv, p, io, shape, arrays, track_best, st);
 }
 
-}  // namespace
-
 // The shapes compiled: for plain codes the row counts and degrees of the 4-, 5- and 8-layer
 // quasi-cyclic codes, rounded up to (6,4), (14,4), (14,5), (10,8); for ragged ones (layers of
 // different widths, or several rows of a layer per lane) the closest of three with row tests.
+// f(D, NL, plain) as integral constants for the code's shape.
+template <class F>
+void with_shape(const LayeredView& cv, F&& f)
+{
+    const auto call = [&](auto d, auto nl) {
+        if (cv.reg_plain) f(d, nl, std::true_type());
+        else f(d, nl, std::false_type());
+    };
+    const int rows = cv.num_layers * cv.reg_rpl;
+    using std::integral_constant;
+    const bool small = cv.maxdeg <= 6 && (cv.reg_plain ? rows == 4 : rows <= 4);
+    if (small) call(integral_constant<int, 6>(), integral_constant<int, 4>());
+    else if (cv.reg_plain && rows == 4) f(integral_constant<int, 14>(), integral_constant<int, 4>(), std::true_type());
+    else if (cv.reg_plain ? rows == 5 : cv.maxdeg > 10) call(integral_constant<int, 14>(), integral_constant<int, 5>());
+    else call(integral_constant<int, 10>(), integral_constant<int, 8>());
+}
+
+}  // namespace
+
 void launch_bp_layered_reg(const LayeredView& cv, const BpParams& p, const BpIO& io, const BpLaunch& shape,
                            bool track_best, cudaStream_t st)
 {
-    const int rows = cv.num_layers * cv.reg_rpl;
-    if (cv.reg_plain) {
-        if (rows == 4 && cv.maxdeg <= 6) launch_shape<6, 4>(cv, p, io, shape, track_best, st);
-        else if (rows == 4) launch_shape<14, 4>(cv, p, io, shape, track_best, st);
-        else if (rows == 5) launch_shape<14, 5>(cv, p, io, shape, track_best, st);
-        else launch_shape<10, 8>(cv, p, io, shape, track_best, st);
-    } else if (cv.maxdeg <= 6 && rows <= 4) {
-        launch_shape<6, 4, false>(cv, p, io, shape, track_best, st);
-    } else if (cv.maxdeg <= 10) {
-        launch_shape<10, 8, false>(cv, p, io, shape, track_best, st);
-    } else {
-        launch_shape<14, 5, false>(cv, p, io, shape, track_best, st);
-    }
+    with_shape(cv, [&](auto d, auto nl, auto plain) {
+        launch_shape<decltype(d)::value, decltype(nl)::value, decltype(plain)::value>(cv, p, io, shape, track_best, st);
+    });
+}
+
+int layered_reg_default_slots(const LayeredView& cv, bool track_best)
+{
+    int slots = 0;
+    with_shape(cv, [&](auto d, auto nl, auto) {
+        int slot_floats = 0;
+        size_t smem = 0;
+        slots = reg_slots<decltype(d)::value, decltype(nl)::value>(cv, 0, track_best ? 2 : 1, &slot_floats, &smem);
+    });
+    return slots;
 }
 
 void reg_plan(LayeredView& cv, int widest, int narrowest, int group)

@@ -1292,7 +1292,11 @@ int sicc_fec_autotune(unsigned long long handle, const float* device_llrs, int c
                         best_ms = g_ms;
                         best = base;
                     }
-                    for (int slots = step; slots * g <= kBpThreads; slots *= 2) {
+                    // the register-resident kernels run fewer codewords per CTA than the general one: no
+                    // trials of shapes that they would cut down to their default
+                    const LayeredView& v = d->code->layered_view();  // of this group: a trial has set it
+                    const int most = v.reg_group > 0 ? layered_reg_default_slots(v, with_osd) - 1 : kBpThreads / g;
+                    for (int slots = step; slots <= most; slots *= 2) {
                         sicc_fec_shape_t sh = base;
                         sh.slots_per_cta = slots;
                         const float t = time_shape(sh);

@@ -323,3 +323,18 @@ def test_osd_exchange_interval_takes_effect(cuda):
     res = dec.autotune(llr, reps=1)
     assert len({shape["osd_share_rounds"] for shape, _ in res.trials}) > 2
     tune.clear()
+
+
+@pytest.mark.parametrize("base,threads", [((4, 8, 16), 256), ((8, 16, 64), 128), ((8, 16, 128), 128), ((6, 12, 64), 256)])
+def test_tuner_times_no_two_equal_shapes(cuda, base, threads):
+    """Codewords per CTA beyond what the code's kernel runs are cut to its default: no trials of their own."""
+    code = codes.qc_code(*base, seed=8)
+    tune.clear()
+    dec = fec.CsrBpDecoder.for_code(code, max_batch=512, max_iter=5)
+    d_llr = cuda.from_numpy(channel.awgn_llrs(code, 512, 2.0, 3)[2].astype(np.float32)).cuda()
+    shapes = [shape for shape, _ in dec.autotune(d_llr, reps=1).trials]
+    tune.clear()
+    lanes = min(base[2], 128 if threads == 128 else 32)  # of the default; the general kernel has 32 at most
+    slots = [s["slots_per_cta"] for s in shapes if s["lanes_per_codeword"] == 0]
+    assert all(n * lanes < threads or (base == (6, 12, 64) and n * lanes == threads) for n in slots), slots
+    assert len({tuple(sorted(s.items())) for s in shapes}) == len(shapes)
