@@ -358,8 +358,7 @@ void DeviceCode::set_osd(const OsdSettings& s)
     }
     if (!combos.empty()) {
         check_cuda(cudaMalloc(&combos_buf_, combos.size() * sizeof(uint32_t)), "cudaMalloc(osd combos)");
-        check_cuda(cudaMemcpy(combos_buf_, combos.data(), combos.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
-                   "upload osd combos");
+        copy_to_device(combos_buf_, combos.data(), combos.size() * sizeof(uint32_t), "upload osd combos");
     }
     osd_.n = n_;
     osd_.k = k_;
@@ -397,8 +396,7 @@ void DeviceCode::set_osd_h(const OsdSettings& s)
     }
     if (!combos.empty()) {
         check_cuda(cudaMalloc(&combos_h_buf_, combos.size() * sizeof(uint32_t)), "cudaMalloc(osd combos)");
-        check_cuda(cudaMemcpy(combos_h_buf_, combos.data(), combos.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
-                   "upload osd combos");
+        copy_to_device(combos_h_buf_, combos.data(), combos.size() * sizeof(uint32_t), "upload osd combos");
     }
     osd_h_.n = n_;
     osd_h_.m = m_;

@@ -103,7 +103,7 @@ T* device_upload(const std::vector<T>& v, std::vector<void*>& owned)
     if (v.empty()) return nullptr;
     void* p = nullptr;
     check_cuda(cudaMalloc(&p, v.size() * sizeof(T)), "cudaMalloc(code table)");
-    check_cuda(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "upload code table");
+    copy_to_device(p, v.data(), v.size() * sizeof(T), "upload code table");
     owned.push_back(p);
     return static_cast<T*>(p);
 }

@@ -787,6 +787,7 @@ struct Engine {
         up(d_per_warp, per);
         up(d_q_warps, qwarps);
         up(d_q_code, qcode);
+        finish_copies("upload(engine)");
         dirty = false;
     }
 };

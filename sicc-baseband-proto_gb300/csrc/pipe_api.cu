@@ -45,7 +45,7 @@ template <class T>
 void upload(Buf<T>& b, const T* src, size_t n)
 {
     b.alloc(n);
-    if (n) check_cuda(cudaMemcpy(b.p, src, n * sizeof(T), cudaMemcpyHostToDevice), "upload pipeline table");
+    if (n) copy_to_device(b.p, src, n * sizeof(T), "upload pipeline table");
 }
 
 struct Slot {
