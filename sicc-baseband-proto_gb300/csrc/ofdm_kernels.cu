@@ -902,10 +902,24 @@ __device__ __forceinline__ void stage_symbol(const SymbolStage& g, float2* stage
                  : "memory");
 }
 
-__device__ __forceinline__ float2 rotation(float cfo_norm, int n)  // exp(-j 2 pi cfo n / fs), cfo_norm = cfo / fs
+// Carrier offset in turns per sample, cfo / fs as an unevaluated sum of two floats.
+struct TurnRate {
+    float hi, lo;
+};
+__device__ __forceinline__ TurnRate turn_rate(float cfo_hz, float sample_rate)
 {
+    const float hi = __fdiv_rn(cfo_hz, sample_rate);
+    return {hi, __fdiv_rn(__fmaf_rn(-hi, sample_rate, cfo_hz), sample_rate)};
+}
+
+// exp(-j 2 pi cfo n / fs).  The angle is reduced to half a turn before it is rounded, so its error does not
+// grow with n.
+__device__ __forceinline__ float2 rotation(TurnRate c, int n)
+{
+    const float x = static_cast<float>(n), p = __fmul_rn(c.hi, x);
+    const float rest = __fmaf_rn(c.lo, x, __fmaf_rn(c.hi, x, -p));  // what the product dropped
     float sn, cs;
-    sincospif(-2.0f * cfo_norm * static_cast<float>(n), &sn, &cs);
+    sincospif(-2.0f * __fadd_rn(__fsub_rn(p, rintf(p)), rest), &sn, &cs);
     return make_float2(cs, sn);
 }
 
@@ -913,17 +927,21 @@ __device__ __forceinline__ float2 rotation(float cfo_norm, int n)  // exp(-j 2 p
 // exp(-j 2 pi cfo n / fs), n its index from the frame start; the samples come from
 // the staged copy, the edge samples (and every sample if the copy did not land)
 // from global memory.  A thread's samples lie kDemodThreads apart: every fourth gets its
-// rotation from sincospi, the three between by turns of `step` = rotation(kDemodThreads).
+// rotation from sincospi, the three after it by one turn each of it by step[k - 1] =
+// rotation(k kDemodThreads).
 __device__ __forceinline__ void derotate_symbol(const DemodView& v, const SymbolStage& g, const float2* stage,
-                                                float2* work, float cfo_norm, float2 step, int sym, bool staged)
+                                                float2* work, TurnRate cfo, const float2 (&step)[3], int sym, bool staged)
 {
     const int off = v.pre_len + sym * (v.nfft + v.cp) + v.cp;
-    float2 rot = make_float2(1.0f, 0.0f);
-    int turn = 0;
-    for (int i = threadIdx.x; i < v.nfft; i += kDemodThreads, turn = (turn + 1) & 3) {
-        const float2 smp = (!staged || i < g.s || i >= g.s + g.len) ? g.src[i] : stage[i - g.s];
-        rot = turn == 0 ? rotation(cfo_norm, off + i) : cmul(rot, step);
-        work[swz(i)] = cmul(smp, rot);
+    for (int i0 = threadIdx.x; i0 < v.nfft; i0 += 4 * kDemodThreads) {
+        const float2 base = rotation(cfo, off + i0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = i0 + k * kDemodThreads;
+            if (i >= v.nfft) break;
+            const float2 smp = (!staged || i < g.s || i >= g.s + g.len) ? g.src[i] : stage[i - g.s];
+            work[swz(i)] = cmul(smp, k == 0 ? base : cmul(base, step[k > 0 ? k - 1 : 0]));
+        }
     }
     __syncthreads();
 }
@@ -973,7 +991,7 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
         cfo = so.cfo_hz;
     }
     const float2* x = samples + (frame_off ? frame_off[f] : static_cast<long long>(f) * stride) + start;
-    const float cfo_norm = cfo / v.sample_rate;
+    const TurnRate rate = turn_rate(cfo, v.sample_rate);
 
     // pilots referenced by this CTA's data symbols
     int pmin = 0x7fffffff, pmax = -1;
@@ -1003,7 +1021,7 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
     float lvl[levels];
 #pragma unroll
     for (int g = 0; g < levels; ++g) lvl[g] = bps >= 2 ? __ldg(v.axis_levels + g) : 0.0f;
-    const float2 step = rotation(cfo_norm, kDemodThreads);
+    const float2 step[3] = {rotation(rate, kDemodThreads), rotation(rate, 2 * kDemodThreads), rotation(rate, 3 * kDemodThreads)};
     __syncthreads();
     if (threadIdx.x == 0) stage_symbol(symbol_stage(v, x, sym_at(0)), stage(0), &s_bar[0]);
     unsigned phase = 0u;  // bit b: parity of buffer b's next completion
@@ -1019,7 +1037,7 @@ demod_kernel(DemodView v, const float2* __restrict__ samples, long long stride, 
         const SymbolStage g = symbol_stage(v, x, sym);
         const bool staged = mbar_wait_bounded(b ? &s_bar[1] : &s_bar[0], (phase >> b) & 1u);
         phase ^= 1u << b;
-        derotate_symbol(v, g, stage(b), work, cfo_norm, step, sym, staged);
+        derotate_symbol(v, g, stage(b), work, rate, step, sym, staged);
         const float2* Y = fft_stockham(work, stage(b), v.nfft, tw);
         if (i < npil) {  // LS estimate at the pilot symbol
             const int p = pmin + i;

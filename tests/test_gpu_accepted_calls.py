@@ -202,6 +202,40 @@ def test_search_at_a_threshold_equal_to_the_metric(cuda, half, value):
     assert again["fine"] == first["fine"]
 
 
+@pytest.mark.parametrize("cfo", [0.05, 0.45, -0.45])
+def test_derotation_error_does_not_grow_along_the_frame(cuda, cfo):
+    """LLRs of a long frame against double precision, for the carrier offset the receiver estimated.  At 0.45
+    subcarriers the frame turns 46 times: an angle rounded before its reduction is off by up to 46 x 2^-24
+    turns, 1.7e-5 rad.  Reduced first, a rotation is off by less than 4e-7 (angle 1e-7, sincospi 1.2e-7, a
+    product 1.7e-7), the FFT by 10 x 6e-8 more, and the LLR's quotient doubles that: 2e-6."""
+    from sicc_gb300.pipeline import SYNC_RECORD, RxPipeline
+    torch, code = cuda, codes.short_code()
+    cfg = ofdm.PhyConfig(nfft=1024, cp=72, num_symbols=96, active_sc=768, pre_half_len=256, modulation="qpsk",
+                         pilot_period=4)
+    t = ofdm.reference_tables(cfg)
+    b = ofdm.FrameGenerator(t, code, seed=4).batch(1, snr_db=25.0, cfo_subcarriers=cfo, max_offset=40, rayleigh_taps=0)
+    p = RxPipeline(t, code.n, code.k, t.coded_bits // code.n, float(b.noise_var[0]), max_batch_frames=1)
+    llr = torch.zeros((1, p.coded_bits), dtype=torch.float32, device="cuda")
+    rec = torch.zeros(SYNC_RECORD.itemsize, dtype=torch.uint8, device="cuda")
+    p.demod_batch(torch.from_numpy(b.iq).cuda(), b.iq.shape[1], b.iq.shape[1], 1, llr, rec, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    sync = rec.cpu().numpy().view(SYNC_RECORD)[0]
+    assert sync["found"] == 1
+    nv, rate = float(np.float32(b.noise_var[0])), float(np.float32(cfg.sample_rate))
+    n = 2 * cfg.pre_half_len + np.arange(cfg.num_symbols)[:, None] * (cfg.nfft + cfg.cp) + cfg.cp + np.arange(cfg.nfft)
+    x = b.iq[0][int(sync["start"]) + n].astype(np.complex128) * np.exp(-2j * np.pi * float(sync["cfo_hz"]) / rate * n)
+    grid = np.fft.fft(x, axis=1)[:, t.used_bins]
+    pilot = t.pilot_grid.astype(np.complex128)
+    hp = grid[t.pilot_symbols] * pilot.conj() / np.abs(pilot) ** 2
+    al = t.interp_alpha.astype(np.float64)[:, None]
+    h = hp[t.interp_p0] * (1 - al) + hp[t.interp_p1] * al
+    eq = grid[t.data_symbols] * h.conj() / (np.abs(h) ** 2 + nv)
+    sig, level = np.maximum(nv / np.abs(h) ** 2, 1e-8), float(t.axis_levels[0])
+    want = np.stack([((v + level) ** 2 - (v - level) ** 2) / sig for v in (eq.real, eq.imag)], axis=-1).reshape(-1)
+    got, want = llr.cpu().numpy()[0].astype(np.float64), want[:p.coded_bits]
+    assert np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2)) < 2e-6
+
+
 # --- mixed-code engine ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("how", ["set", "autotune"])
