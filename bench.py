@@ -964,7 +964,7 @@ def run_mixed(args, rank, world):
         eng.add_code(c, engine.iteration_cap(c.n), ALPHA, 0.0, engine.osd_order_for(c), OSD_FLIP, OSD_TESTS)
 
     tuned = None
-    if not args.no_tune:  # warps per codeword of each code and warps per CTA, on this batch
+    if not args.no_tune:  # warps per codeword of each code, on this batch
         base_ms, tuned_ms = eng.autotune(w.count, d_code, d_llr, d_llr_off, d_info, d_info_off, reps=2)
         tuned = {"bp_default_ms": round(base_ms, 4), "bp_tuned_ms": round(tuned_ms, 4)}
     code_warps = {c.name(): eng.code_warps(i) for i, c in enumerate(w.codes)}

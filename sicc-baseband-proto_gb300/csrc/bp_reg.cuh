@@ -1,5 +1,5 @@
 // Register-resident min-sum rows: the parts shared by the single-code kernels
-// (bp_reg.cu) and the mixed-code kernel (engine.cu).
+// (bp_reg_layered.cu, bp_reg_flooding.cu) and the mixed-code kernel (engine.cu).
 //
 // A group of G lanes owns one codeword; lane g owns row slots g, g + G, ... of
 // every layer, at most NL rows in all.  A lane keeps its rows' messages in
@@ -13,7 +13,7 @@
 // signs) state.  A row's outgoing messages come as exclusive minima -- over the
 // row's other edges, from the minima of groups of two to four edges -- by
 // min.xorsign.abs, which takes the smaller magnitude and multiplies the signs
-// in one ALU operation: about 2.7 per edge for magnitude and sign together,
+// in one ALU operation: 2.7 to 2.9 per edge for magnitude and sign together,
 // against 15 for rebuild, (min1, min2, argmin), compare, select and signs.
 // Scaling and additions run on the FMA pipe, which is otherwise idle.
 #pragma once

@@ -8,8 +8,8 @@
 //
 // Measured on GB300 against bp_flooding_kernel (bp_kernels.cu, which walks the
 // edge lists and stays for codes that do not fit): 8,191 frames of (128,64) at
-// 2 dB with OSD 370 -> 187 us; 2,001 codewords of (1024,768) at 3.5 dB, damped,
-// 1,434 -> 72 us.  The damped form keeps the inputs and recomputes the messages,
+// 2 dB 230 -> 44 us; 2,001 codewords of (1024,768) at 3.5 dB, damped, 1,434 ->
+// 76 us as a call (kernel 55).  The damped form keeps the inputs and recomputes the messages,
 // so the large shapes take two CTAs per SM there: at three they spill (2,000 of
 // (1024,512): 189 us against 151).
 #include "bp_kernels.h"

@@ -5,8 +5,8 @@
 //
 // Measured on GB300 against the kernels before it (compressed row state, in
 // registers for the (128,64) code, else in shared memory): 65,536 frames of
-// (128,64) at 2 dB with OSD 506 -> 390 us, of which BP 235 -> about 120 (ALU
-// pipe 80% busy before); 7,680 codewords of (1024,512) at 2 dB 1,000 -> 245 us;
+// (128,64) at 2 dB 235 -> 120 us (ALU pipe 80% busy before, 46% now; shared-
+// memory pipe 58%); 7,680 codewords of (1024,512) at 2 dB 1,000 -> 245 us;
 // 1,000 of (2048,1024) at 2.5 dB 645 -> 82 us.
 #include "bp_kernels.h"
 #include "bp_reg.cuh"

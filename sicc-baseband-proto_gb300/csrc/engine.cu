@@ -1020,7 +1020,7 @@ int sicc_engine_set_launch_shape(unsigned long long handle, int warps_per_cta, i
         auto e = get(handle);
         std::lock_guard<std::mutex> lock(e->mu);
         if (warps_per_cta < 0 || warps_per_cta > 8 || ctas < 0) throw InvalidArgument("warps_per_cta must be 0..8");
-        // the kernel has one CTA shape (kMixedWarps); the argument is checked and otherwise unused
+        // the kernel has one CTA shape (kMixedWarps): the argument is checked and otherwise unused
         e->ctas = ctas;
         return CUDA_OSD_STATUS_OK;
     });
@@ -1245,8 +1245,9 @@ int sicc_engine_last_ms(unsigned long long handle, float* out_prepare_ms, float*
 }
 
 // Coordinate search on the caller's batch: codes in decreasing BP cost, each tried at every
-// allowed warps per codeword (kept when the mixed BP kernel gets at least 1% faster).  Trials decode with every codeword's protection at BP only, so OSD
-// time stays out of the comparison; each trial is one warm-up and `reps` timed decodes.
+// allowed warps per codeword (kept when the mixed BP kernel gets at least 1% faster).  Trials
+// decode with every codeword's protection at BP only, so OSD time stays out of the comparison;
+// each trial is one warm-up and `reps` timed decodes.
 int sicc_engine_autotune(unsigned long long handle, int codewords, const unsigned char* device_code_ids,
                          const float* device_llr, const long long* device_llr_offsets, unsigned char* device_info,
                          const long long* device_info_offsets, int reps, float* out_default_ms, float* out_tuned_ms)

@@ -36,8 +36,8 @@
 // given the same equalised symbol.  Measured on GB300, 256 frames of 14 x 1,024
 // (16-QAM): 52 us with a plain FFT buffer (half its shared-memory wavefronts
 // were bank conflicts), one twiddle table read at strides and a sincospi per
-// sample; 40 us with swizzled buffers, twiddles in reading order and one
-// sincospi per four samples.  The transmitter shares the FFT: 256 frames,
+// sample; 37 us with swizzled buffers, twiddles in reading order and one
+// sincospi per four samples (taken together: 39 one after another).  The transmitter shares the FFT: 256 frames,
 // encoder 37 -> 17 us (parity words of the tables only), symbols 69 -> 35 us.
 // Both are bound by instruction issue.
 #include "ofdm_kernels.h"
@@ -517,12 +517,13 @@ __device__ SyncOut sync_finish(const float2* __restrict__ x, int avail, int limi
 }
 
 // Frame search, one CTA per (pass, frame): pass q scans candidates
-// [4352 q, 4352 (q + 1)).  Within a pass every threshold crossing is refined
-// at once: the fine metric of each position within +-radius of any crossing is
-// computed once (one warp per position), then each crossing takes the first
-// maximum over its window (starting from 0, strict >) and the earliest
-// crossing whose maximum reaches the threshold wins -- the outcome of the CPU
-// receiver's sequential retry loop.  Mode 0 wants the earliest success, so a
+// [4352 q, 4352 (q + 1)).  Within a pass the positions within +-radius of any
+// threshold crossing are marked, and their fine metrics computed in increasing
+// order, a warp per group of four, until the first one over the threshold and
+// its 2 radius successors are known (groups that half the preamble rules out
+// count as below).  The earliest crossing within +-radius of that position
+// wins and takes the first maximum of its window (starting from 0, strict >)
+// -- the outcome of the CPU receiver's sequential retry loop.  Mode 0 wants the earliest success, so a
 // pass that starts after an earlier pass of its frame succeeded skips its
 // scan (`ticket[frames + f]` holds passes - earliest successful pass, 0 for
 // none).  Each pass stores its result in `pres`, and the CTA that takes the
