@@ -236,6 +236,36 @@ def test_derotation_error_does_not_grow_along_the_frame(cuda, cfo):
     assert np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2)) < 2e-6
 
 
+# --- OFDM transmitter ------------------------------------------------------------------------------------
+
+@pytest.mark.parametrize("aligned", [True, False])  # information bits away from a 16-byte boundary: the general encoder
+@pytest.mark.parametrize("base", [(8, 16, 128), (5, 16, 128), (4, 16, 32), (4, 8, 128)])
+def test_transmit_long_information_blocks(cuda, base, aligned):
+    """Information blocks of one, two and three passes of 512 bits, the last one full or partial; 4 to 32 parity
+    words; bytes whose low bit alone counts."""
+    import tx_oracle
+    from sicc_gb300.pipeline import RxPipeline
+    from test_gpu_tx import _close, _gen, _kw
+    torch, code = cuda, codes.qc_code(*base, seed=12)
+    cfg = ofdm.PhyConfig(nfft=512, cp=36, num_symbols=9, active_sc=384, pre_half_len=64, modulation="16qam",
+                         pilot_period=4)
+    t = ofdm.reference_tables(cfg)
+    blocks = t.coded_bits // code.n
+    p = RxPipeline(t, code.n, code.k, blocks, 1e-3, slots=2)
+    G = _gen(code)
+    p.upload_tx_tables(generator_kn=G)
+    info = np.random.default_rng(3).integers(0, 256, size=(3, blocks * code.k), dtype=np.uint8)
+    buf = torch.zeros(info.size + 16, dtype=torch.uint8, device="cuda")
+    view = buf[0 if aligned else 3:][:info.size].view(info.shape)
+    view.copy_(torch.from_numpy(info))
+    assert (view.data_ptr() % 16 == 0) == aligned
+    out = torch.zeros((3, t.frame_len), dtype=torch.complex64, device="cuda")
+    p.tx_batch(view, 3, out, stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    coded = tx_oracle.encode_generator(info.reshape(-1, code.k), G).reshape(3, -1)
+    _close(out.cpu().numpy(), tx_oracle.tx_frames(coded, **_kw(t)), base)
+
+
 # --- mixed-code engine ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("how", ["set", "autotune"])
