@@ -223,6 +223,7 @@ DeviceCode::DeviceCode(int n, int m, const int* row_ptr, const int* col_ind, int
         if (probe.reg_plain) build_layered();
     }
     if (need_osd) set_osd(osd);
+    else finish_copies("upload code tables");
 }
 
 DeviceCode::~DeviceCode()
@@ -358,8 +359,10 @@ void DeviceCode::set_osd(const OsdSettings& s)
     }
     if (!combos.empty()) {
         check_cuda(cudaMalloc(&combos_buf_, combos.size() * sizeof(uint32_t)), "cudaMalloc(osd combos)");
-        copy_to_device(combos_buf_, combos.data(), combos.size() * sizeof(uint32_t), "upload osd combos");
+        check_cuda(cudaMemcpy(combos_buf_, combos.data(), combos.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+                   "upload osd combos");
     }
+    finish_copies("upload osd tables");
     osd_.n = n_;
     osd_.k = k_;
     osd_.nw = (n_ + 63) / 64;
@@ -396,8 +399,10 @@ void DeviceCode::set_osd_h(const OsdSettings& s)
     }
     if (!combos.empty()) {
         check_cuda(cudaMalloc(&combos_h_buf_, combos.size() * sizeof(uint32_t)), "cudaMalloc(osd combos)");
-        copy_to_device(combos_h_buf_, combos.data(), combos.size() * sizeof(uint32_t), "upload osd combos");
+        check_cuda(cudaMemcpy(combos_h_buf_, combos.data(), combos.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+                   "upload osd combos");
     }
+    finish_copies("upload osd tables");
     osd_h_.n = n_;
     osd_h_.m = m_;
     osd_h_.k = k_;

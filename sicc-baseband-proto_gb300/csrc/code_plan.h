@@ -97,13 +97,14 @@ void consecutive_layers(int n, int m, const int* row_ptr, const int* col_ind, st
 // number of tests including the base is at most max_tests.
 std::vector<uint32_t> osd_combos(int pool, int order, int max_tests);
 
+// The caller finishes its copies (finish_copies) before the table is used.
 template <class T>
 T* device_upload(const std::vector<T>& v, std::vector<void*>& owned)
 {
     if (v.empty()) return nullptr;
     void* p = nullptr;
     check_cuda(cudaMalloc(&p, v.size() * sizeof(T)), "cudaMalloc(code table)");
-    copy_to_device(p, v.data(), v.size() * sizeof(T), "upload code table");
+    check_cuda(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "upload code table");
     owned.push_back(p);
     return static_cast<T*>(p);
 }

@@ -658,7 +658,7 @@ struct Loop {
             int nc = 0;
             if (engine_code_routes(ln.engine, r, 64, &nc) != CUDA_OSD_STATUS_OK) throw std::runtime_error(last_error());
             ln.routes.alloc(64);
-            copy_to_device(ln.routes.p, r, sizeof(r), "upload code routes");
+            check_cuda(cudaMemcpy(ln.routes.p, r, sizeof(r), cudaMemcpyHostToDevice), "upload code routes");
         }
         std::vector<PhyDev> pd;
         for (size_t q = 0; q < phys.size(); ++q) {
@@ -672,7 +672,9 @@ struct Loop {
         }
         ln.d_phys.alloc(std::max<size_t>(pd.size(), 1));
         if (!pd.empty())
-            copy_to_device(ln.d_phys.p, pd.data(), pd.size() * sizeof(PhyDev), "upload profiles");
+            check_cuda(cudaMemcpy(ln.d_phys.p, pd.data(), pd.size() * sizeof(PhyDev), cudaMemcpyHostToDevice),
+                       "upload profiles");
+        finish_copies("upload lane tables");
         cudaStream_t stream = ln.stream;
         check_cuda(cudaGraphCreate(&ln.graph, 0), "cudaGraphCreate");
         // graph: while (loop) { admit; if (admitted) { layout; demod; decode; complete } publish }

@@ -41,11 +41,12 @@ struct Buf {
     ~Buf() { release(); }
 };
 
+// The caller finishes its copies (finish_copies) before the table is used.
 template <class T>
 void upload(Buf<T>& b, const T* src, size_t n)
 {
     b.alloc(n);
-    if (n) copy_to_device(b.p, src, n * sizeof(T), "upload pipeline table");
+    if (n) check_cuda(cudaMemcpy(b.p, src, n * sizeof(T), cudaMemcpyHostToDevice), "upload pipeline table");
 }
 
 struct Slot {
@@ -414,6 +415,7 @@ int sicc_pipe_upload_static_tables(unsigned long long handle, const sicc_pipe_ta
         x.pilot_grid = p->pilot_grid.p;
         x.preamble = p->preamble.p;
         x.twiddle = p->twiddle.p;
+        finish_copies("upload pipeline tables");
         p->tables = true;
         return CUDA_OSD_STATUS_OK;
     });
@@ -730,6 +732,7 @@ int sicc_pipe_upload_tx_tables(unsigned long long handle, const sicc_pipe_tx_tab
                 check_cuda(cudaEventCreateWithFlags(&sl->tx_done, cudaEventDisableTiming), "cudaEventCreate(tx)");
             }
         }
+        finish_copies("upload transmit tables");
         p->tx_tables = true;
         return CUDA_OSD_STATUS_OK;
     });

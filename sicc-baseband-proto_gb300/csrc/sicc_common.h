@@ -27,13 +27,6 @@ inline void check_cuda(cudaError_t st, const char* what)
 // non-blocking streams do not wait for it: called after the copies of host tables.
 inline void finish_copies(const char* what) { check_cuda(cudaStreamSynchronize(cudaStreamLegacy), what); }
 
-// Host table to device, finished on return.
-inline void copy_to_device(void* dst, const void* src, size_t bytes, const char* what)
-{
-    check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
-    finish_copies(what);
-}
-
 void set_last_error(const std::string& msg);
 const char* last_error();
 
