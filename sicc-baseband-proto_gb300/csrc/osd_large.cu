@@ -269,7 +269,8 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
         // codes took 533 us (500 now; 20,000 took the same 4.2 ms).  Tables and indices built by the
         // other warps in 2 instead of by all in 1: 512 us and 4.25 ms.  Windows of 16 candidates to
         // fill each round with 8 pivots: 538 us and 4.8 ms.
-        // The column at position jj: first edge << 8 | weight (0: none), and its row for this lane.
+        // The column at position jj: first edge << 15 | weight (0: none), and its row
+        // for this lane.  (A code has at most 27 m < 2^15 edges, m <= 1,024.)
         struct Column {
             int info, row;
         };
@@ -277,14 +278,14 @@ osd_h_kernel(OsdHView hv0, OsdHLayout lay, OsdIO io)
             Column c{0, 0};
             if (jj >= 0) {
                 const int v = s.perm[jj], e0 = __ldg(hv.col_ptr + v);
-                c.info = (e0 << 8) | (__ldg(hv.col_ptr + v + 1) - e0);
-                if (lane < (c.info & 255)) c.row = __ldg(hv.col_rows + e0 + lane);
+                c.info = (e0 << 15) | (__ldg(hv.col_ptr + v + 1) - e0);
+                if (lane < (c.info & 32767)) c.row = __ldg(hv.col_rows + e0 + lane);
             }
             return c;
         };
         auto reduce_column = [&](const Column& c, uint32_t* dst) {  // T h_c, word `lane`
             unsigned v = 0u;
-            const int e0 = c.info >> 8, cnt = c.info & 255;
+            const int e0 = c.info >> 15, cnt = c.info & 32767;
             // lane e: row of the column's e-th one (none: a row no lane holds), and that row's
             // column's place in T (-1: a unit vector)
             const int mine = lane < cnt ? (c.row << 16) | static_cast<uint16_t>(s.rank[c.row]) : (2047 << 16) | 0xffff;

@@ -3,6 +3,8 @@
 Each of them is a form that a general path answered before a faster kernel took over its sizes: arrays
 that start away from a 16-byte boundary (soft values in, LLRs out).  Results are compared with the same call in its ordinary form.
 """
+import types
+
 import numpy as np
 import pytest
 
@@ -319,6 +321,39 @@ def test_engine_speed_survives_a_shape_given_up(cuda, how):
     # off the register-resident rows the mixed kernel takes about twice as long
     assert ms["tried"] <= 1.25 * ms["plain"], ms
     tune.clear()
+
+
+@pytest.mark.parametrize("weight", [33, 255, 256, 300, 512])
+def test_long_code_osd_with_a_heavy_column(cuda, oracle, weight):
+    """Columns of H of more than 32, and of more than 255, ones."""
+    torch, m, k = cuda, 512, 512
+    rng = np.random.default_rng(weight)
+    rows = []
+    for r in range(m):  # accumulator parity, three random information columns, column 0 in the first `weight` rows
+        info = set(rng.choice(np.arange(1, k), 3, replace=False).tolist()) | ({0} if r < weight else set())
+        rows.append(sorted(info) + ([k + r - 1] if r else []) + [k + r])
+    row_ptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    code = types.SimpleNamespace(n=m + k, m=m, k=k, row_ptr=row_ptr, col_ind=np.concatenate(rows).astype(np.int32))
+    table = oracle.code(code.n, m, code.row_ptr, code.col_ind).systematic_parity()
+    cw = np.zeros((6, code.n), np.int64)
+    cw[:, :k] = rng.integers(0, 2, (6, k))
+    for r in range(m):  # the row's other columns give its own parity bit
+        cw[:, k + r] = cw[:, rows[r][:-1]].sum(axis=1) % 2
+    llr = (4.0 * (1 - 2 * cw) + 3.0 * rng.standard_normal(cw.shape)).astype(np.float32)
+    llr[:4, 0] = 0.01 * (2 * cw[:4, 0] - 1)  # the elimination meets the heavy column first; its bit is wrong
+    eng = engine.Engine(max_codewords=6, max_llr_floats=llr.size)
+    eng.add_code(code, 10, osd_order=1)
+    info = torch.zeros(6 * k, dtype=torch.uint8, device="cuda")
+    used, off = torch.zeros(6, dtype=torch.uint8, device="cuda"), torch.arange(6, device="cuda")
+    metric = torch.zeros(6, dtype=torch.float32, device="cuda")
+    eng.osd_device(6, torch.zeros(6, dtype=torch.uint8, device="cuda"), torch.from_numpy(llr).cuda(), off * code.n, info,
+                   off * k, used, metric, stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    got, gm = info.cpu().numpy().reshape(6, k), metric.cpu().numpy()
+    assert used.cpu().numpy().all()
+    for i in range(6):
+        out, want, _, _ = oracle.osd(table, code.n, k, llr[i], 1, 64, 4096)
+        assert np.array_equal(got[i], out[:k]) and gm[i] == np.float32(want), i
 
 
 # --- saved shapes -----------------------------------------------------------------------------------------
