@@ -1,7 +1,8 @@
 """Calls that the entry points accept, at the edges of what the fast paths take.
 
-Each of them is a form that a general path answered before a faster kernel took over its sizes: arrays
-that start away from a 16-byte boundary (soft values in, LLRs out).  Results are compared with the same call in its ordinary form.
+Arrays that start away from a 16-byte boundary, codes and grids beyond a kernel's shared memory, thresholds
+equal to a metric, shapes that were tried and given up or saved for other kernels, columns and information
+blocks longer than usual.  Results are compared with the same call in its ordinary form or with the oracle.
 """
 import types
 
